@@ -15,6 +15,10 @@ struct Vec16;
 template <>
 struct Vec16<float> {
   static constexpr int E = 4;  // elements per 16 B
+  __device__ __forceinline__ static void unpack(const uint4 v, float (&o)[4]) {
+    o[0] = __uint_as_float(v.x); o[1] = __uint_as_float(v.y);
+    o[2] = __uint_as_float(v.z); o[3] = __uint_as_float(v.w);
+  }
   __device__ __forceinline__ static void load(const float* p, float (&o)[4]) {
     const float4 v = __ldg(reinterpret_cast<const float4*>(p));
     o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;

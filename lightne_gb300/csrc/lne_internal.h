@@ -33,19 +33,25 @@ struct __align__(16) Vertex {
 };
 
 // Work list of one sparse operator for the row-parallel SpMM (built once,
-// cached on the matrix or graph): rows with at most kChunkNnz entries are
-// one work item each; longer rows are cut into kChunkNnz-entry chunks.
+// cached on the matrix or graph).  A row with at most kChunkNnz entries is
+// one item, a longer row is cut into items of kChunkNnz entries (chunks).
+// Items come longest first: [0, n_big) the rows above max(kBigNnz, warp_max)
+// and every chunk, [n_big, n_heavy) the rows above warp_max, then the rest
+// (at most warp_max entries).
 static constexpr int kChunkNnz = 2048;
+static constexpr int kBigNnz = 512;
+static constexpr int kWarpNnzMin = 64;
+struct __align__(16) SpmmItem {
+  int64_t begin;  // first nonzero
+  uint32_t row;
+  uint32_t len;
+};
 struct SpmmPlan {
-  int64_t n_short = 0;              // rows with <= kChunkNnz entries (incl. empty rows)
-  int64_t n_chunks = 0;             // chunks of long rows
-  int64_t n_long = 0;               // long rows
-  uint32_t* short_rows = nullptr;   // [n_short]
-  uint32_t* chunk_row = nullptr;    // [n_chunks]
-  int64_t* chunk_begin = nullptr;   // [n_chunks] first nonzero of each chunk
-  uint32_t* long_rows = nullptr;    // [n_long]
-  int64_t* long_first = nullptr;    // [n_long + 1] first chunk of each long row
-  void* mem = nullptr;              // one allocation backing the arrays
+  int64_t n_items = 0, n_big = 0, n_heavy = 0;
+  int warp_max = kChunkNnz;   // a power of two in [kWarpNnzMin, kChunkNnz]
+  SpmmItem* items = nullptr;  // [n_items]
+  uint2* span = nullptr;      // [n_big] {first item of its row, items of its row}
+  void* mem = nullptr;        // one allocation backing the arrays
 };
 
 }  // namespace lne
@@ -160,8 +166,8 @@ void scan_exclusive_i64(const int64_t* counts, int64_t* out, int64_t n, void* tm
                         cudaStream_t stream);
 
 // SpMM work lists (built on ctx->stream; synchronises once): a count
-// kernel, three exclusive scans of three launches each, a fill kernel.
-static constexpr int kPlanLaunches = 11;
+// kernel, two exclusive scans of three launches each, a fill kernel.
+static constexpr int kPlanLaunches = 8;
 int build_plan_csr(lne_ctx* ctx, lne_csr* c);
 int build_plan_graph(lne_ctx* ctx, lne_graph* g);
 void free_plan(SpmmPlan& p);

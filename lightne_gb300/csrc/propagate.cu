@@ -19,6 +19,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <cmath>
 #include <string>
 #include <type_traits>
@@ -81,103 +82,211 @@ __global__ void k_op_coef(const Vertex* __restrict__ vd, int64_t n, float mu, fl
   coef[i] = make_float4((float)(1.0 - (double)mu - inv), (float)(-inv), dt, (float)inv);
 }
 
-// Loads N elements (N a multiple of 4, e0 a multiple of 4) of row r of a
-// dense operand as floats: 16-byte loads for FP32, 8-byte loads for BF16
-// and FP16 (so an e0 that is 4 mod 8 stays aligned).
-template <typename T, int N>
-__device__ __forceinline__ void load_row(const T* __restrict__ X, int64_t ld, int64_t r, int e0, float (&o)[N]) {
-  const T* p = X + r * ld + e0;
-  if constexpr (sizeof(T) == 4) {
+// W 32-bit words at p (16-, 8- or 4-byte accesses; p aligned to them).
+template <int W>
+__device__ __forceinline__ void load_words(const uint32_t* __restrict__ p, uint32_t (&w)[W]) {
+  if constexpr (W % 4 == 0) {
 #pragma unroll
-    for (int i = 0; i < N; i += 4) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(p + i));
-      o[i] = v.x; o[i + 1] = v.y; o[i + 2] = v.z; o[i + 3] = v.w;
+    for (int i = 0; i < W; i += 4) {
+      const uint4 v = *reinterpret_cast<const uint4*>(p + i);
+      w[i] = v.x; w[i + 1] = v.y; w[i + 2] = v.z; w[i + 3] = v.w;
     }
-  } else if constexpr (std::is_same<T, __half>::value) {
-#pragma unroll
-    for (int i = 0; i < N; i += 4) {
-      const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + i));
-      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x));
-      const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
-      o[i] = a.x; o[i + 1] = a.y; o[i + 2] = b.x; o[i + 3] = b.y;
-    }
+  } else if constexpr (W == 2) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    w[0] = v.x; w[1] = v.y;
   } else {
-#pragma unroll
-    for (int i = 0; i < N; i += 4) {
-      const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + i));
-      o[i] = __uint_as_float(v.x << 16); o[i + 1] = __uint_as_float(v.x & 0xffff0000u);
-      o[i + 2] = __uint_as_float(v.y << 16); o[i + 3] = __uint_as_float(v.y & 0xffff0000u);
-    }
+    static_assert(W == 1, "one, two or a multiple of four words");
+    w[0] = *p;
   }
 }
+template <int W>
+__device__ __forceinline__ void store_words(uint32_t* __restrict__ p, const uint32_t (&w)[W]) {
+  if constexpr (W % 4 == 0) {
+#pragma unroll
+    for (int i = 0; i < W; i += 4) *reinterpret_cast<uint4*>(p + i) = make_uint4(w[i], w[i + 1], w[i + 2], w[i + 3]);
+  } else if constexpr (W == 2) {
+    *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
+  } else {
+    static_assert(W == 1, "one, two or a multiple of four words");
+    *p = w[0];
+  }
+}
+
+// N elements of a dense row as loaded (16-bit types: not yet widened); an
+// epilogue sees 4 or 8 of them, or one 32-bit word's.
+template <typename T, int N>
+struct RawRow {
+  static constexpr int W = N * (int)sizeof(T) / 4;
+  uint32_t w[W];
+  __device__ __forceinline__ void load(const T* __restrict__ X, int64_t ld, int64_t r, int e0) {
+    load_words<W>(reinterpret_cast<const uint32_t*>(X + r * ld + e0), w);
+  }
+  __device__ __forceinline__ float at(int i) const {
+    if constexpr (sizeof(T) == 4) {
+      return __uint_as_float(w[i]);
+    } else if constexpr (std::is_same<T, __half>::value) {
+      const __half2 h = *reinterpret_cast<const __half2*>(&w[i >> 1]);
+      return (i & 1) ? __high2float(h) : __low2float(h);
+    } else {
+      return __uint_as_float((i & 1) ? (w[i >> 1] & 0xffff0000u) : (w[i >> 1] << 16));
+    }
+  }
+};
 template <int N>
 __device__ __forceinline__ void load_f32(const float* __restrict__ X, int64_t ld, int64_t r, int e0, float (&o)[N]) {
-  const float* p = X + r * ld + e0;
+  uint32_t w[N];
+  load_words<N>(reinterpret_cast<const uint32_t*>(X + r * ld + e0), w);
 #pragma unroll
-  for (int i = 0; i < N; i += 4) {
-    const float4 v = *reinterpret_cast<const float4*>(p + i);
-    o[i] = v.x; o[i + 1] = v.y; o[i + 2] = v.z; o[i + 3] = v.w;
-  }
+  for (int i = 0; i < N; ++i) o[i] = __uint_as_float(w[i]);
 }
 template <int N>
 __device__ __forceinline__ void store_f32(float* __restrict__ X, int64_t ld, int64_t r, int e0, const float (&o)[N]) {
-  float* p = X + r * ld + e0;
+  uint32_t w[N];
 #pragma unroll
-  for (int i = 0; i < N; i += 4) *reinterpret_cast<float4*>(p + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+  for (int i = 0; i < N; ++i) w[i] = __float_as_uint(o[i]);
+  store_words<N>(reinterpret_cast<uint32_t*>(X + r * ld + e0), w);
 }
 template <typename HT, int N>
 __device__ __forceinline__ void store_16(HT* __restrict__ X, int64_t ld, int64_t r, int e0, const float (&o)[N]) {
-  HT* p = X + r * ld + e0;
+  if constexpr (N % 2 == 0) {  // (an FP32 form keeps no 16-bit copies)
+    uint32_t w[N / 2];
 #pragma unroll
-  for (int i = 0; i < N; i += 2) *reinterpret_cast<uint32_t*>(p + i) = pack2_16<HT>(o[i], o[i + 1]);
+    for (int i = 0; i < N; i += 2) w[i / 2] = pack2_16<HT>(o[i], o[i + 1]);
+    store_words<N / 2>(reinterpret_cast<uint32_t*>(X + r * ld + e0), w);
+  }
 }
 
+// The coefficients of row r that an epilogue needs: {m_i, o_i}, or d~_i.
+__device__ __forceinline__ float2 coef_mo(const float4* __restrict__ coef, int64_t r) {
+  return __ldg(reinterpret_cast<const float2*>(coef + r));
+}
+__device__ __forceinline__ float coef_dt(const float4* __restrict__ coef, int64_t r) {
+  return __ldg(reinterpret_cast<const float*>(coef + r) + 2);
+}
+
+// <V_k, D~ a> sums of the adjoint's parameter gradients, taken in the
+// epilogues of the recursion: per lane in FP32 over the rows of its warp (or
+// one long row), then in FP64, each warp and each long row (which any block
+// may take) into a place of its own; k_dot_sum adds the places in order.
+struct DotOut {
+  const float* __restrict__ a = nullptr;  // the input embedding (n x ld)
+  int64_t ld = 0;
+  double* pv = nullptr;                   // <V_k, D~ a> by place
+  double* pw = nullptr;                   // <M V_k, D~ a>, or null
+};
+struct DotState {
+  static constexpr bool kSums = true;
+  float v = 0.0f, w = 0.0f;
+  __device__ __forceinline__ static double warp_sum(float x) {
+    double d = (double)x;
+    for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(kFull, d, o);
+    return d;
+  }
+  // Adds the warp's sums (the column slabs of a row follow one another).
+  __device__ __forceinline__ void put(const DotOut& o, uint32_t place) const {
+    const double dv = warp_sum(v), dw = warp_sum(w);
+    if ((threadIdx.x & 31) == 0) {
+      o.pv[place] += dv;
+      if (o.pw) o.pw[place] += dw;
+    }
+  }
+};
+
+// Adds a row's <x, D~ a> to the sums.
+template <int N>
+__device__ __forceinline__ void dot_v(const DotOut& o, const float4* __restrict__ coef, int64_t r, int e0,
+                                      const float (&x)[N], DotState& st) {
+  float a[N];
+  load_f32<N>(o.a, o.ld, r, e0, a);
+  const float dt = coef_dt(coef, r);
+#pragma unroll
+  for (int i = 0; i < N; ++i) st.v = fmaf(x[i], dt * a[i], st.v);
+}
+
+// Epilogues of the SpMM (spmm_core.cuh): load() fetches the row's operands
+// ahead of the gathers, store() applies the recursion to the finished sums.
+// With DOTS they also add the parameter gradients' sums.
+
 // tmp = M x: out = m_i x_i + o_i acc (operand x of type XT); FP32 and/or
-// 16-bit outputs.
-template <typename XT>
+// 16-bit outputs.  DOTS: <x, D~ a> and <M x, D~ a>.
+template <typename XT, bool DOTS = false>
 struct EpiApplyM {
   using HT = typename ShadowOf<XT>::type;
+  using State = typename std::conditional<DOTS, DotState, NoState>::type;
   const float4* __restrict__ coef;
   const XT* __restrict__ X;  // the operand (diagonal term)
   int64_t ld;
   float* __restrict__ out_f;
   HT* __restrict__ out_b;
+  DotOut dot;
   template <int N>
-  __device__ __forceinline__ void operator()(int64_t r, int e0, const float (&a)[N]) const {
-    const float4 c = __ldg(coef + r);
-    float x[N], y[N];
-    load_row<XT, N>(X, ld, r, e0, x);
+  struct Pre {
+    float2 c;
+    RawRow<XT, N> x;
+    float a[DOTS ? N : 1], dt;
+  };
+  template <int N>
+  __device__ __forceinline__ Pre<N> load(int64_t r, int e0) const {
+    Pre<N> q;
+    q.c = coef_mo(coef, r);
+    q.x.load(X, ld, r, e0);
+    if constexpr (DOTS) {
+      q.dt = coef_dt(coef, r);
+      load_f32<N>(dot.a, dot.ld, r, e0, q.a);
+    }
+    return q;
+  }
+  template <int N>
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&a)[N], const Pre<N>& q, State& st) const {
+    float y[N];
 #pragma unroll
-    for (int i = 0; i < N; ++i) y[i] = fmaf(c.x, x[i], c.y * a[i]);
+    for (int i = 0; i < N; ++i) y[i] = fmaf(q.c.x, q.x.at(i), q.c.y * a[i]);
     if (out_f) store_f32<N>(out_f, ld, r, e0, y);
     if (out_b) store_16<HT, N>(out_b, ld, r, e0, y);
+    if constexpr (DOTS) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const float da = q.dt * q.a[i];
+        st.v = fmaf(q.x.at(i), da, st.v);
+        st.w = fmaf(y[i], da, st.w);
+      }
+    }
   }
 };
 
-// Final vector of a filter: fin = base - (scale_dt ? d~_i : 1) * conv.
+// Final vector of a filter: fin = base_scale base - (scale_dt ? d~_i : 1)
+// conv, written as out_scale fin (FP32) and fin (16-bit); either may be null.
 template <typename HT>
 struct FinalOut {
-  const float* __restrict__ base;  // null: not the final step
-  bool scale_dt;
-  float* __restrict__ out;
-  HT* __restrict__ outb;
+  const float* __restrict__ base = nullptr;  // null: not the final step
+  bool scale_dt = false;
+  float* __restrict__ out = nullptr;
+  HT* __restrict__ outb = nullptr;
+  float base_scale = 1.0f, out_scale = 1.0f;
   template <int N>
-  __device__ __forceinline__ void apply(int64_t r, int e0, int64_t ld, const float4 c, const float (&cv)[N]) const {
+  __device__ __forceinline__ void apply(int64_t r, int e0, int64_t ld, const float4* __restrict__ coef,
+                                        const float (&cv)[N]) const {
     float b[N], f[N];
     load_f32<N>(base, ld, r, e0, b);
-    const float sc = scale_dt ? c.z : 1.0f;
+    const float sc = scale_dt ? coef_dt(coef, r) : 1.0f;
 #pragma unroll
-    for (int i = 0; i < N; ++i) f[i] = fmaf(-sc, cv[i], b[i]);
-    store_f32<N>(out, ld, r, e0, f);
+    for (int i = 0; i < N; ++i) f[i] = fmaf(-sc, cv[i], base_scale * b[i]);
     if (outb) store_16<HT, N>(outb, ld, r, e0, f);
+    if (out) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) f[i] *= out_scale;
+      store_f32<N>(out, ld, r, e0, f);
+    }
   }
 };
 
 // First order: Lx1 = 0.5 M tmp - x;  conv = c0 x + c1 Lx1 (conv may be null:
-// the tangent pass keeps no sum);  or the final vector when order <= 2.
-template <typename XT>
+// no sum is kept);  or the final vector when order <= 2.  x = x_scale A.
+// DOTS: <Lx1, D~ a>.
+template <typename XT, bool DOTS = false>
 struct EpiFirst {
   using HT = typename ShadowOf<XT>::type;
+  using State = typename std::conditional<DOTS, DotState, NoState>::type;
   const float4* __restrict__ coef;
   const XT* __restrict__ T;        // tmp (operand)
   const float* __restrict__ A;     // x (FP32)
@@ -187,41 +296,56 @@ struct EpiFirst {
   FinalOut<HT> fin;
   int64_t ld;
   float c0, c1;
+  float x_scale;
+  DotOut dot;
   template <int N>
-  __device__ __forceinline__ void operator()(int64_t r, int e0, const float (&acc)[N]) const {
-    const float4 c = __ldg(coef + r);
-    float t[N], a[N], l1[N], cv[N];
-    load_row<XT, N>(T, ld, r, e0, t);
-    load_f32<N>(A, ld, r, e0, a);
+  struct Pre {
+    float2 c;
+    RawRow<XT, N> t;
+    float a[N];
+  };
+  template <int N>
+  __device__ __forceinline__ Pre<N> load(int64_t r, int e0) const {
+    Pre<N> q;
+    q.c = coef_mo(coef, r);
+    q.t.load(T, ld, r, e0);
+    load_f32<N>(A, ld, r, e0, q.a);
+    return q;
+  }
+  template <int N>
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&acc)[N], const Pre<N>& q, State& st) const {
+    float l1[N], cv[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      const float mt = fmaf(c.x, t[i], c.y * acc[i]);
-      l1[i] = fmaf(0.5f, mt, -a[i]);
-      cv[i] = fmaf(c1, l1[i], c0 * a[i]);
+      const float a = x_scale * q.a[i];
+      const float mt = fmaf(q.c.x, q.t.at(i), q.c.y * acc[i]);
+      l1[i] = fmaf(0.5f, mt, -a);
+      cv[i] = fmaf(c1, l1[i], c0 * a);
     }
-    store_f32<N>(L1, ld, r, e0, l1);
+    if constexpr (DOTS) dot_v<N>(dot, coef, r, e0, l1, st);
+    if (L1) store_f32<N>(L1, ld, r, e0, l1);
     if (L1b) store_16<HT, N>(L1b, ld, r, e0, l1);
     if (fin.base)
-      fin.template apply<N>(r, e0, ld, c, cv);
+      fin.template apply<N>(r, e0, ld, coef, cv);
     else if (conv)
       store_f32<N>(conv, ld, r, e0, cv);
   }
 };
 
-// Order k >= 2: Lx2 = M tmp - Lx0 - 2 Lx1 [- 2 extra];  conv += ck Lx2 (conv
-// may be null);  or the final vector on the last order.  L0 == null means a
-// zero Lx0; `extra` (FP32, may be null) is the tangent pass's M T_k term.
+// Order k >= 2: Lx2 = M tmp - Lx0 - 2 Lx1;  conv += ck Lx2 (conv may be
+// null);  or the final vector on the last order.  Lx0 = l0_scale L0.
 // The sum is read and written every second order: `skip` leaves conv alone
 // and the next order adds ck_prev Lx1 (the skipped order's vector) as well.
-template <typename XT>
+// DOTS (the last order): <Lx2, D~ a>.
+template <typename XT, bool DOTS = false>
 struct EpiStep {
   using HT = typename ShadowOf<XT>::type;
+  using State = typename std::conditional<DOTS, DotState, NoState>::type;
   const float4* __restrict__ coef;
   const XT* __restrict__ T;
   const float* __restrict__ L0;
   const float* __restrict__ L1;
-  const float* __restrict__ extra;
-  float* __restrict__ L2;
+  float* __restrict__ L2;          // null: not stored (the last order)
   HT* __restrict__ L2b;
   float* __restrict__ conv;
   FinalOut<HT> fin;
@@ -229,98 +353,125 @@ struct EpiStep {
   float ck;
   float ck_prev = 0.0f;
   bool skip = false;
+  float l0_scale = 1.0f;
+  DotOut dot;
   template <int N>
-  __device__ __forceinline__ void operator()(int64_t r, int e0, const float (&acc)[N]) const {
-    const float4 c = __ldg(coef + r);
-    float t[N], l0[N], l1[N], l2[N], cv[N];
-    load_row<XT, N>(T, ld, r, e0, t);
-    if (L0) {
-      load_f32<N>(L0, ld, r, e0, l0);
-    } else {
-#pragma unroll
-      for (int i = 0; i < N; ++i) l0[i] = 0.0f;
-    }
-    load_f32<N>(L1, ld, r, e0, l1);
-    if (conv && !skip) {
-      load_f32<N>(conv, ld, r, e0, cv);
-#pragma unroll
-      for (int i = 0; i < N; ++i) cv[i] = fmaf(ck_prev, l1[i], cv[i]);
-    } else {
-#pragma unroll
-      for (int i = 0; i < N; ++i) cv[i] = 0.0f;
-    }
-    float ex[N];
-    if (extra) {
-      load_f32<N>(extra, ld, r, e0, ex);
-    } else {
-#pragma unroll
-      for (int i = 0; i < N; ++i) ex[i] = 0.0f;
-    }
+  struct Pre {
+    float2 c;
+    RawRow<XT, N> t;
+    float l0[N], l1[N], cv[N];
+  };
+  template <int N>
+  __device__ __forceinline__ Pre<N> load(int64_t r, int e0) const {
+    Pre<N> q;
+    q.c = coef_mo(coef, r);
+    q.t.load(T, ld, r, e0);
+    load_f32<N>(L0, ld, r, e0, q.l0);
+    load_f32<N>(L1, ld, r, e0, q.l1);
+    if (conv && !skip) load_f32<N>(conv, ld, r, e0, q.cv);
+    return q;
+  }
+  template <int N>
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&acc)[N], const Pre<N>& q, State& st) const {
+    float l2[N], cv[N];
+    const bool sum = conv && !skip;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      const float mt = fmaf(c.x, t[i], c.y * acc[i]);
-      l2[i] = fmaf(-2.0f, ex[i], fmaf(-2.0f, l1[i], mt - l0[i]));
-      cv[i] = fmaf(ck, l2[i], cv[i]);
+      const float mt = fmaf(q.c.x, q.t.at(i), q.c.y * acc[i]);
+      l2[i] = fmaf(-2.0f, q.l1[i], fmaf(-l0_scale, q.l0[i], mt));
+      cv[i] = fmaf(ck, l2[i], sum ? fmaf(ck_prev, q.l1[i], q.cv[i]) : 0.0f);
     }
+    if constexpr (DOTS) dot_v<N>(dot, coef, r, e0, l2, st);
     if (fin.base) {
-      fin.template apply<N>(r, e0, ld, c, cv);
+      fin.template apply<N>(r, e0, ld, coef, cv);
     } else {
-      store_f32<N>(L2, ld, r, e0, l2);
+      if (L2) store_f32<N>(L2, ld, r, e0, l2);
       if (L2b) store_16<HT, N>(L2b, ld, r, e0, l2);
-      if (conv && !skip) store_f32<N>(conv, ld, r, e0, cv);
+      if (sum) store_f32<N>(conv, ld, r, e0, cv);
     }
   }
 };
 
 // y = (A + I) x: out = out_scale * (x_i + acc), written with leading
 // dimension ldy for columns < d (out_scale undoes the input scaling of the
-// FP16 form; 1 otherwise).
+// FP16 form; 1 otherwise); vec: Y's rows are whole 16-byte vectors.
 template <typename XT>
 struct EpiAPlusI {
+  using State = NoState;
   const XT* __restrict__ X;
   int64_t ld;
   float* __restrict__ Y;
   int64_t ldy;
   int d;
   float out_scale;
+  bool vec;
   template <int N>
-  __device__ __forceinline__ void operator()(int64_t r, int e0, const float (&acc)[N]) const {
-    float x[N];
-    load_row<XT, N>(X, ld, r, e0, x);
+  struct Pre {
+    RawRow<XT, N> x;
+  };
+  template <int N>
+  __device__ __forceinline__ Pre<N> load(int64_t r, int e0) const {
+    Pre<N> q;
+    q.x.load(X, ld, r, e0);
+    return q;
+  }
+  template <int N>
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&acc)[N], const Pre<N>& q, State&) const {
+    float o[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) o[i] = out_scale * (q.x.at(i) + acc[i]);
+    if (vec) {
+      store_f32<N>(Y, ldy, r, e0, o);
+      return;
+    }
     float* y = Y + r * ldy + e0;
 #pragma unroll
     for (int i = 0; i < N; ++i)
-      if (e0 + i < d) y[i] = out_scale * (x[i] + acc[i]);
+      if (e0 + i < d) y[i] = o[i];
   }
 };
 
-// Adjoint start: h = (A + I) g;  b = h / d~_i (FP32 and BF16 copy).
+// Adjoint start: h = (A + I) g (H may be null), g = g_scale times the operand
+// (a power of two);  b = h / d~_i (FP32 and 16-bit copy).
 template <typename XT>
 struct EpiAdjInit {
   using HT = typename ShadowOf<XT>::type;
+  using State = NoState;
   const float4* __restrict__ coef;
   const XT* __restrict__ G;
   int64_t ld;
   float* __restrict__ H;
   float* __restrict__ Bf;
   HT* __restrict__ Bb;
+  float g_scale;
   template <int N>
-  __device__ __forceinline__ void operator()(int64_t r, int e0, const float (&acc)[N]) const {
-    const float4 c = __ldg(coef + r);
-    float gr[N], h[N], b[N];
-    load_row<XT, N>(G, ld, r, e0, gr);
+  struct Pre {
+    float inv_dt;
+    RawRow<XT, N> g;
+  };
+  template <int N>
+  __device__ __forceinline__ Pre<N> load(int64_t r, int e0) const {
+    Pre<N> q;
+    q.inv_dt = __ldg(reinterpret_cast<const float*>(coef + r) + 3);
+    q.g.load(G, ld, r, e0);
+    return q;
+  }
+  template <int N>
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&acc)[N], const Pre<N>& q, State&) const {
+    float h[N], b[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      h[i] = gr[i] + acc[i];
-      b[i] = h[i] * c.w;
+      h[i] = g_scale * (q.g.at(i) + acc[i]);
+      b[i] = h[i] * q.inv_dt;
     }
-    store_f32<N>(H, ld, r, e0, h);
+    if (H) store_f32<N>(H, ld, r, e0, h);
     store_f32<N>(Bf, ld, r, e0, b);
     if (Bb) store_16<HT, N>(Bb, ld, r, e0, b);
   }
 };
 
-// dst (n x ld, zero padding) = scale * src (n x d) and its 16-bit copy.
+// dst (n x ld, zero padding; may be null) = scale * src (n x d) and its
+// 16-bit copy.
 template <typename HT>
 __global__ void k_pad_copy(const float* __restrict__ src, int64_t n, int d, float scale, float* __restrict__ dst,
                            int64_t ld, HT* __restrict__ dstb) {
@@ -328,7 +479,7 @@ __global__ void k_pad_copy(const float* __restrict__ src, int64_t n, int d, floa
     const int64_t i = t / ld;
     const int j = (int)(t - i * ld);
     const float v = j < d ? scale * src[i * d + j] : 0.0f;
-    dst[t] = v;
+    if (dst) dst[t] = v;
     if (dstb) {
       if constexpr (std::is_same<HT, __half>::value)
         dstb[t] = __float2half_rn(v);
@@ -344,22 +495,6 @@ __global__ void k_unpad_copy(const float* __restrict__ src, int64_t ld, int64_t 
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n * d; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = t / d;
     dst[t] = scale * src[i * ld + (t - i * d)];
-  }
-}
-
-// y = alpha x (FP32) and its 16-bit copy.
-template <typename HT>
-__global__ void k_scale_copy(const float* __restrict__ x, int64_t total, float alpha, float* __restrict__ y,
-                             HT* __restrict__ yb) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const float v = alpha * x[t];
-    y[t] = v;
-    if (yb) {
-      if constexpr (std::is_same<HT, __half>::value)
-        yb[t] = __float2half_rn(v);
-      else
-        yb[t] = __float2bfloat16_rn(v);
-    }
   }
 }
 
@@ -383,16 +518,12 @@ __global__ void k_amax_partial(const float* __restrict__ x, int64_t total, float
   }
 }
 
-// <h, x> partial sums: FP32 within a thread, FP64 across threads, one
-// value per block (summed in block order on the host).
-static constexpr int kDotBlocks = 1024;
-__global__ void k_dot_partial(const float* __restrict__ h, const float* __restrict__ x, int64_t total,
-                              double* __restrict__ out) {
-  float s = 0.0f;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x)
-    s = fmaf(h[t], x[t], s);
-  double d = (double)s;
-  for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
+// out[slot] = sum of part[slot][0 .. count) in a fixed order (one block per slot).
+__global__ void k_dot_sum(const double* __restrict__ part, int64_t count, double* __restrict__ out) {
+  const double* p = part + (int64_t)blockIdx.x * count;
+  double d = 0.0;
+  for (int64_t t = threadIdx.x; t < count; t += blockDim.x) d += p[t];
+  for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(kFull, d, o);
   __shared__ double ws[32];
   if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = d;
   __syncthreads();
@@ -420,6 +551,19 @@ struct Bufs {
   }
 };
 
+// The parameter gradients' sums of one recursion: slot k holds the parts of
+// <V_k, D~ a>, slot K + k those of <M V_k, D~ a>.
+struct Dots {
+  const float* a = nullptr;  // n x ld
+  int64_t ld = 0;
+  double* part = nullptr;    // [2 K][places]
+  int64_t places = 0;
+  int K = 0;
+  DotOut slots(int k, bool with_m) const {
+    return DotOut{a, ld, part + (int64_t)k * places, with_m ? part + (int64_t)(K + k) * places : nullptr};
+  }
+};
+
 // Shared state of one filter evaluation.
 template <typename XT>
 struct Filter {
@@ -427,32 +571,41 @@ struct Filter {
   using HT = typename ShadowOf<XT>::type;
   lne_ctx* ctx;
   lne_graph* g;
-  GraphRows R;
   int64_t n, ld;
   const float4* coef;
   int* launches;
   Bufs* B;
+  const SpmmWork* work;
   size_t sz() const { return (size_t)n * ld; }
 
   // operand view of an FP32 vector with an optional 16-bit copy
   const XT* op(const float* f, const HT* b) const { return k16 ? (const XT*)b : (const XT*)f; }
 
-  int apply_m(const XT* X, float* out_f, HT* out_b) {
-    EpiApplyM<XT> epi{coef, X, ld, out_f, out_b};
-    return spmm_run<XT>(ctx, R, g->plan, X, ld, ld, epi, launches);
+  template <class Epi>
+  int spmm(const XT* X, const Epi& epi) {
+    return spmm_run<XT, false>(ctx, g->plan, g->nbrs, nullptr, X, ld, ld, epi, launches, 0, work);
   }
 
-  // The Chebyshev filter on x (FP32 xf, operand copy xb): fin = base -
-  // scale * sum_k c_k T_k(X) x written to finf / finb.
-  int run(const float* xf, const HT* xb, int order, const std::vector<float>& c, const float* base,
-          bool scale_dt, float* finf, HT* finb) {
+  int apply_m(const XT* X, float* out_f, HT* out_b, const Dots* dots, int k) {
+    if constexpr (!k16) {
+      if (dots) return spmm(X, EpiApplyM<XT, true>{coef, X, ld, out_f, out_b, dots->slots(k, true)});
+    }
+    return spmm(X, EpiApplyM<XT>{coef, X, ld, out_f, out_b, DotOut()});
+  }
+
+  // The Chebyshev filter on x = x_scale xf (operand copy xb):
+  // fin.base_scale fin.base - scale * sum_k c_k T_k(X) x written as `fin`
+  // says.  With a null fin.base only the recursion runs, for its dots (FP32
+  // operands).
+  int run(const float* xf, const HT* xb, float x_scale, int order, const std::vector<float>& c,
+          const FinalOut<HT>& fin, const Dots* dots = nullptr) {
     int rc;
     float *conv = nullptr, *Tf = nullptr;
     HT* Tb = nullptr;
     float* ring[3] = {nullptr, nullptr, nullptr};
     HT* ringb[3] = {nullptr, nullptr, nullptr};
-    const int nring = order > 2 ? 3 : 1;
-    if ((rc = B->get(&conv, sz(), "conv"))) return rc;
+    const int nring = order > 2 ? 3 : 0;
+    if (order > 2 && fin.base && (rc = B->get(&conv, sz(), "conv"))) return rc;
     for (int i = 0; i < nring; ++i) {
       if ((rc = B->get(&ring[i], sz(), "Chebyshev vector"))) return rc;
       if (k16 && (rc = B->get(&ringb[i], sz(), "Chebyshev vector 16-bit"))) return rc;
@@ -464,27 +617,46 @@ struct Filter {
     }
     const XT* X0 = op(xf, xb);
     const XT* Tx = k16 ? (const XT*)Tb : (const XT*)Tf;
-    if ((rc = apply_m(X0, k16 ? nullptr : Tf, k16 ? Tb : nullptr))) return rc;  // tmp = M x
-    const bool first_is_last = order <= 2;
+    if ((rc = apply_m(X0, k16 ? nullptr : Tf, k16 ? Tb : nullptr, dots, 0))) return rc;  // tmp = M x
     {
-      FinalOut<HT> fo{first_is_last ? base : nullptr, scale_dt, finf, finb};
-      EpiFirst<XT> epi{coef, Tx, xf, ring[0], ringb[0], conv, fo, ld, c[0], c[1]};
-      if ((rc = spmm_run<XT>(ctx, R, g->plan, Tx, ld, ld, epi, launches))) return rc;
+      // the sums of the last vector are taken as it is formed, those of the
+      // others when M is applied to them
+      const bool last = order <= 2;
+      const FinalOut<HT> fo = last ? fin : FinalOut<HT>();
+      if constexpr (!k16) {
+        if (last && dots) {
+          EpiFirst<XT, true> epi{coef, Tx, xf, ring[0], ringb[0], conv, fo, ld, c[0], c[1], x_scale, dots->slots(1, false)};
+          return spmm(Tx, epi);
+        }
+      }
+      EpiFirst<XT> epi{coef, Tx, xf, ring[0], ringb[0], conv, fo, ld, c[0], c[1], x_scale, DotOut()};
+      if ((rc = spmm(Tx, epi))) return rc;
     }
     const float* l0 = xf;
+    float l0_scale = x_scale;
     int j1 = 0;
     for (int k = 2; k < order; ++k) {
       const int j2 = (j1 + 1) % 3;
-      if ((rc = apply_m(op(ring[j1], ringb[j1]), k16 ? nullptr : Tf, k16 ? Tb : nullptr))) return rc;
+      if ((rc = apply_m(op(ring[j1], ringb[j1]), k16 ? nullptr : Tf, k16 ? Tb : nullptr, dots, k - 1))) return rc;
       const bool last = k == order - 1;
-      FinalOut<HT> fo{last ? base : nullptr, scale_dt, finf, finb};
+      const FinalOut<HT> fo = last ? fin : FinalOut<HT>();
       // conv is updated on odd orders (and on the last): even orders are
       // added with the next one
       const bool skip = !last && (k % 2 == 0);
       const float ck_prev = (k % 2 == 1) ? c[k - 1] : 0.0f;
-      EpiStep<XT> epi{coef, Tx, l0, ring[j1], nullptr, ring[j2], ringb[j2], conv, fo, ld, c[k], ck_prev, skip};
-      if ((rc = spmm_run<XT>(ctx, R, g->plan, Tx, ld, ld, epi, launches))) return rc;
+      float* out = last ? nullptr : ring[j2];
+      HT* outb = last ? nullptr : ringb[j2];
+      if constexpr (!k16) {
+        if (last && dots) {
+          EpiStep<XT, true> epi{coef, Tx,   l0,      ring[j1], out,      outb, conv, fo,
+                                ld,   c[k], ck_prev, skip,     l0_scale, dots->slots(k, false)};
+          return spmm(Tx, epi);
+        }
+      }
+      EpiStep<XT> epi{coef, Tx, l0, ring[j1], out, outb, conv, fo, ld, c[k], ck_prev, skip, l0_scale, DotOut()};
+      if ((rc = spmm(Tx, epi))) return rc;
       l0 = ring[j1];
+      l0_scale = 1.0f;
       j1 = j2;
     }
     return LNE_OK;
@@ -492,17 +664,25 @@ struct Filter {
 };
 
 template <typename XT>
-int setup_filter(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, Bufs& B, int* launches, Filter<XT>& F,
-                 float4** coef_out) {
-  const int64_t n = g->n;
+int setup_filter(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, Bufs& B, SpmmWork* work, int* launches,
+                 Filter<XT>& F) {
+  const int64_t n = g->n, ld = pad_ld(p->dim);
   float4* coef = nullptr;
   int rc;
   if ((rc = B.get(&coef, n, "operator coefficients"))) return rc;
+  // the partial sums of the long rows, as wide as the FP32 form needs them
+  if ((rc = spmm_work_alloc(ctx, g->plan, std::max(spmm_work_width<XT>(ld), spmm_work_width<float>(ld)), work))) return rc;
+  B.ptrs.push_back(work->partial);
   k_op_coef<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(g->vdata, n, (float)p->mu, coef);
   *launches += 1;
-  F = Filter<XT>{ctx, g, GraphRows{g->vdata, g->nbrs}, n, pad_ld(p->dim), coef, launches, &B};
-  *coef_out = coef;
+  F = Filter<XT>{ctx, g, n, ld, coef, launches, &B, work};
   return LNE_OK;
+}
+
+// An n x ld FP32 matrix the kernels can read and write in 16-byte vectors.
+bool rows_direct(const void* p, int64_t d, int64_t ld) { return d == ld && ((uintptr_t)p & 15) == 0; }
+bool ranges_overlap(const void* a, const void* b, size_t bytes) {
+  return (uintptr_t)a < (uintptr_t)b + bytes && (uintptr_t)b < (uintptr_t)a + bytes;
 }
 
 // Power-of-two input scale of the FP16 form.  The propagation is linear in
@@ -538,6 +718,16 @@ int input_scale(lne_ctx* ctx, const float* x, int64_t total, Bufs& B, int* launc
   }
 }
 
+struct TimedEvents {
+  cudaEvent_t e[2] = {};
+  TimedEvents() {
+    for (auto& x : e) cudaEventCreate(&x);
+  }
+  ~TimedEvents() {
+    for (auto& x : e) cudaEventDestroy(x);
+  }
+};
+
 template <typename XT>
 int propagate_impl(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, const float* d_a, float* d_y,
                    float* d_a_out, lne_propagate_stats* stats) {
@@ -552,46 +742,61 @@ int propagate_impl(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, co
   chebyshev_coeffs(p->order, p->s, c);
   Bufs B(ctx);
   Filter<XT> F;
-  float4* coef = nullptr;
+  SpmmWork work;
   int rc;
-  cudaEvent_t ev0, ev1;
-  cudaEventCreate(&ev0);
-  cudaEventCreate(&ev1);
-  cudaEventRecord(ev0, st);
-  if ((rc = setup_filter<XT>(ctx, g, p, B, &launches, F, &coef))) return rc;
+  TimedEvents ev;
+  cudaEventRecord(ev.e[0], st);
+  if ((rc = setup_filter<XT>(ctx, g, p, B, &work, &launches, F))) return rc;
   float sc = 1.0f;
   if ((rc = input_scale<XT>(ctx, d_a, n * d, B, &launches, &sc))) return rc;
-  float *A = nullptr, *Af = nullptr;
-  HT *Ab = nullptr, *Afb = nullptr;
   const size_t sz = (size_t)n * ld;
-  if ((rc = B.get(&A, sz, "a")) || (rc = B.get(&Af, sz, "a - conv"))) return rc;
+  // The caller's rows are read in place where they are whole 16-byte
+  // vectors, else a zero-padded copy; the 16-bit forms gather a scaled copy.
+  const bool direct = rows_direct(d_a, d, ld);
+  float* Acopy = nullptr;
+  HT *Ab = nullptr, *Afb = nullptr;
+  if (!direct && (rc = B.get(&Acopy, sz, "a"))) return rc;
   if (k16 && ((rc = B.get(&Ab, sz, "a 16-bit")) || (rc = B.get(&Afb, sz, "a - conv 16-bit")))) return rc;
   const unsigned pg = (unsigned)std::min<int64_t>((n * ld + 255) / 256, (int64_t)ctx->num_sms * 32);
-  k_pad_copy<HT><<<pg, 256, 0, st>>>(d_a, n, d, sc, A, ld, Ab);
-  launches += 1;
-  // a - conv, then y = (A + I)(a - conv)
-  if ((rc = F.run(A, Ab, p->order, c, A, false, Af, Afb))) return rc;
-  {
-    const XT* Xf = F.op(Af, Afb);
-    EpiAPlusI<XT> epi{Xf, ld, d_y, d, d, 1.0f / sc};
-    if ((rc = spmm_run<XT>(ctx, F.R, g->plan, Xf, ld, ld, epi, &launches))) return rc;
+  if (!direct || k16) {
+    k_pad_copy<HT><<<pg, 256, 0, st>>>(d_a, n, d, sc, Acopy, ld, Ab);
+    launches += 1;
   }
-  if (d_a_out) {
+  const float* A = direct ? d_a : Acopy;
+  const float a_scale = direct ? sc : 1.0f;
+  // a - conv: to the caller's buffer where it can be written in place (the
+  // (A + I) product gathers it in the FP32 form, so it must not be y)
+  const bool out_direct =
+      d_a_out && rows_direct(d_a_out, d, ld) && !ranges_overlap(d_a_out, d_y, sizeof(float) * (size_t)n * d);
+  float* Af = nullptr;
+  if (!out_direct && (!k16 || d_a_out) && (rc = B.get(&Af, sz, "a - conv"))) return rc;
+  FinalOut<HT> fin;
+  fin.base = A;
+  fin.base_scale = a_scale;
+  fin.out = out_direct ? d_a_out : Af;
+  fin.out_scale = out_direct ? 1.0f / sc : 1.0f;
+  fin.outb = Afb;
+  // a - conv, then y = (A + I)(a - conv)
+  if ((rc = F.run(A, Ab, a_scale, p->order, c, fin))) return rc;
+  {
+    const XT* Xf = F.op(fin.out, Afb);
+    EpiAPlusI<XT> epi{Xf, ld, d_y, d, d, 1.0f / sc, rows_direct(d_y, d, ld)};
+    if ((rc = F.spmm(Xf, epi))) return rc;
+  }
+  if (d_a_out && !out_direct) {
     k_unpad_copy<<<pg, 256, 0, st>>>(Af, ld, n, d, 1.0f / sc, d_a_out);
     launches += 1;
   }
-  cudaEventRecord(ev1, st);
-  LNE_CUDA_TRY(cudaEventSynchronize(ev1));
+  cudaEventRecord(ev.e[1], st);
+  LNE_CUDA_TRY(cudaEventSynchronize(ev.e[1]));
   LNE_CUDA_TRY(cudaGetLastError());
   if (stats) {
     memset(stats, 0, sizeof(*stats));
-    cudaEventElapsedTime(&stats->ms_total, ev0, ev1);
+    cudaEventElapsedTime(&stats->ms_total, ev.e[0], ev.e[1]);
     stats->kernel_launches = launches;
     stats->spmm_calls = 2 * (p->order > 2 ? p->order - 1 : 1) + 1;
   }
   ctx->launch_count += launches;
-  cudaEventDestroy(ev0);
-  cudaEventDestroy(ev1);
   return LNE_OK;
 }
 
@@ -605,92 +810,39 @@ void chebyshev_coeffs_ds(int order, double s, std::vector<double>& dc) {
     dc[k] = ((k & 1) ? -1.0 : 1.0) * (bessel_i(k - 1, sf) + bessel_i(k + 1, sf));
 }
 
-// dL/dmu and dL/ds in FP32 (P3): the forward pass on a with the mu-tangent
-// T'_1 = -M a, T'_{k+1} = M(M T'_k) - 2 T'_k - T'_{k-1} - 2 M T_k, and the
-// dots <h, T_k a>, <h, T'_k> (h = hscale^-1 H): dL/ds = -sum_k c_k'(s)
-// <h, T_k a>, dL/dmu = -sum_k c_k <h, T'_k>.
-int param_grads(lne_ctx* ctx, Filter<float>& F, const lne_propagate_params* p, const std::vector<float>& c,
-                const float* H, const float* d_a, double hscale, double* h_dmu, double* h_ds) {
-  const int64_t n = F.n, ld = F.ld;
-  const int d = (int)p->dim;
-  const int order = p->order;
-  const size_t sz = (size_t)n * ld;
-  const int64_t total = (int64_t)sz;
-  cudaStream_t st = ctx->stream;
-  Bufs& B = *F.B;
-  int& launches = *F.launches;
-  const float4* coef = F.coef;
+// dL/dmu and dL/ds (P3) from the sums the adjoint's recursion leaves:
+// with f(M) = sum_k c_k T_k(X), X = M^2/2 - I, L = <h, a - f(M) a>:
+//   dL/ds  = -sum_k c_k'(s) <h, T_k a>,
+//   dL/dmu = <h, f'(M) a>  (dM/dmu = -I),
+//   f'(M)  = sum_k k c_k U_{k-1}(X) M = sum_j e_j T_j(X) M,
+// U_n being 2 (T_n + T_{n-2} + ...), T_0 counted once.  All of these are
+// polynomials in M, and M^T = D~ M D~^-1, so with V_k = T_k(X) D~^-1 h (the
+// vectors the adjoint's recursion forms anyway)
+//   <h, T_k a> = <V_k, D~ a>,  <h, T_j M a> = <M V_j, D~ a>:
+// no recursion on a is run (the tangent recursion this replaces took 36
+// products with the graph per gradient; these sums take none of their own).
+int param_grads(lne_ctx* ctx, const lne_propagate_params* p, const std::vector<float>& c, const Dots& dots,
+                Bufs& B, int* launches, double hscale, double* h_dmu, double* h_ds) {
+  const int K = dots.K;
+  double* d_sum = nullptr;
   int rc;
-  const int K = order > 2 ? order : 2;
-  double* partial = nullptr;
-  if ((rc = B.get(&partial, (size_t)2 * K * kDotBlocks, "dot partials"))) return rc;
-  LNE_CUDA_TRY(cudaMemsetAsync(partial, 0, sizeof(double) * 2 * K * kDotBlocks, st));
-  auto dot = [&](int slot, const float* x) {
-    k_dot_partial<<<kDotBlocks, 256, 0, st>>>(H, x, total, partial + (int64_t)slot * kDotBlocks);
-    launches += 1;
-  };
-  float *A = nullptr, *Tm = nullptr, *Tpm = nullptr;  // a, M T_k, M T'_k
-  float* T[3];
-  float* Tp[3];
-  if ((rc = B.get(&A, sz, "a")) || (rc = B.get(&Tm, sz, "M T")) || (rc = B.get(&Tpm, sz, "M T'"))) return rc;
-  for (int i = 0; i < 3; ++i)
-    if ((rc = B.get(&T[i], sz, "T")) || (rc = B.get(&Tp[i], sz, "T'"))) return rc;
-  const unsigned pg = (unsigned)std::min<int64_t>((total + 255) / 256, (int64_t)ctx->num_sms * 32);
-  k_pad_copy<__nv_bfloat16><<<pg, 256, 0, st>>>(d_a, n, d, 1.0f, A, ld, nullptr);
-  launches += 1;
-  dot(0, A);  // <h, T_0>
-  // tmp = M a;  T_1 = 0.5 M tmp - a;  T'_1 = -tmp
-  if ((rc = F.apply_m(A, Tm, nullptr))) return rc;
-  {
-    FinalOut<__nv_bfloat16> fo{nullptr, false, nullptr, nullptr};
-    EpiFirst<float> epi{coef, Tm, A, T[0], nullptr, nullptr, fo, ld, 0.0f, 0.0f};
-    if ((rc = spmm_run<float>(ctx, F.R, F.g->plan, Tm, ld, ld, epi, &launches))) return rc;
-  }
-  k_scale_copy<__nv_bfloat16><<<pg, 256, 0, st>>>(Tm, total, -1.0f, Tp[0], nullptr);
-  launches += 1;
-  dot(1, T[0]);
-  dot(K + 1, Tp[0]);
-  const float* t0 = A;         // T_{k-1}
-  const float* tp0 = nullptr;  // T'_{k-1} (T'_0 = 0)
-  int j1 = 0;
-  for (int k = 1; k + 1 < order; ++k) {
-    const int j2 = (j1 + 1) % 3;
-    // tmp = M T_k; T_{k+1} = M tmp - 2 T_k - T_{k-1}
-    if ((rc = F.apply_m(T[j1], Tm, nullptr))) return rc;
-    {
-      FinalOut<__nv_bfloat16> fo{nullptr, false, nullptr, nullptr};
-      EpiStep<float> epi{coef, Tm, t0, T[j1], nullptr, T[j2], nullptr, nullptr, fo, ld, 0.0f};
-      if ((rc = spmm_run<float>(ctx, F.R, F.g->plan, Tm, ld, ld, epi, &launches))) return rc;
-    }
-    // tmp' = M T'_k; T'_{k+1} = M tmp' - 2 T'_k - T'_{k-1} - 2 M T_k
-    if ((rc = F.apply_m(Tp[j1], Tpm, nullptr))) return rc;
-    {
-      FinalOut<__nv_bfloat16> fo{nullptr, false, nullptr, nullptr};
-      EpiStep<float> epi{coef, Tpm, tp0, Tp[j1], Tm, Tp[j2], nullptr, nullptr, fo, ld, 0.0f};
-      if ((rc = spmm_run<float>(ctx, F.R, F.g->plan, Tpm, ld, ld, epi, &launches))) return rc;
-    }
-    dot(k + 1, T[j2]);
-    dot(K + k + 1, Tp[j2]);
-    t0 = T[j1];
-    tp0 = Tp[j1];
-    j1 = j2;
-  }
-  std::vector<double> hp((size_t)2 * K * kDotBlocks);
-  LNE_CUDA_TRY(cudaMemcpyAsync(hp.data(), partial, sizeof(double) * hp.size(), cudaMemcpyDeviceToHost, st));
-  LNE_CUDA_TRY(cudaStreamSynchronize(st));
-  std::vector<double> dots(2 * K, 0.0);
-  for (int sidx = 0; sidx < 2 * K; ++sidx) {
-    for (int b = 0; b < kDotBlocks; ++b) dots[sidx] += hp[(size_t)sidx * kDotBlocks + b];
-    dots[sidx] *= hscale;
-  }
+  if ((rc = B.get(&d_sum, (size_t)2 * K, "dot sums"))) return rc;
+  k_dot_sum<<<2 * K, 256, 0, ctx->stream>>>(dots.part, dots.places, d_sum);
+  *launches += 1;
+  std::vector<double> h((size_t)2 * K);
+  LNE_CUDA_TRY(cudaMemcpyAsync(h.data(), d_sum, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, ctx->stream));
+  LNE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   std::vector<double> dc;
-  chebyshev_coeffs_ds(order, p->s, dc);
-  // only the terms the forward filter uses: k < max(order, 2)
+  chebyshev_coeffs_ds(p->order, p->s, dc);
   double gs = 0.0, gmu = 0.0;
-  for (int k = 0; k < K; ++k) gs -= dc[k] * dots[k];
-  for (int k = 1; k < K; ++k) gmu -= (double)c[k] * dots[K + k];
-  if (h_ds) *h_ds = gs;
-  if (h_dmu) *h_dmu = gmu;
+  for (int k = 0; k < K; ++k) gs -= dc[k] * h[k];
+  for (int j = 0; j + 1 < K; ++j) {
+    double e = 0.0;
+    for (int k = j + 1; k < K; k += 2) e += (double)k * (double)c[k];
+    gmu += (j == 0 ? 1.0 : 2.0) * e * h[K + j];
+  }
+  if (h_ds) *h_ds = gs * hscale;
+  if (h_dmu) *h_dmu = gmu * hscale;
   return LNE_OK;
 }
 
@@ -709,67 +861,92 @@ int adjoint_impl(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, cons
   chebyshev_coeffs(order, p->s, c);
   Bufs B(ctx);
   Filter<XT> F;
-  float4* coef = nullptr;
+  SpmmWork work;
   int rc;
-  cudaEvent_t ev0, ev1;
-  cudaEventCreate(&ev0);
-  cudaEventCreate(&ev1);
-  cudaEventRecord(ev0, st);
-  if ((rc = setup_filter<XT>(ctx, g, p, B, &launches, F, &coef))) return rc;
+  TimedEvents ev;
+  cudaEventRecord(ev.e[0], st);
+  if ((rc = setup_filter<XT>(ctx, g, p, B, &work, &launches, F))) return rc;
   const size_t sz = (size_t)n * ld;
-  const int64_t total = (int64_t)sz;
+  const bool params = h_dmu || h_ds;
   // the FP16 form runs on a scaled output gradient sg * g (dL/da is linear
-  // in g; the FP32 parameter-gradient pass unscales its dots by 1 / sg)
+  // in g; the FP32 parameter-gradient pass unscales its sums by 1 / sg)
   float sg = 1.0f;
   if ((rc = input_scale<XT>(ctx, d_gy, n * d, B, &launches, &sg))) return rc;
-  float *G = nullptr, *H = nullptr, *Bf = nullptr, *GA = nullptr;
+  // g is read in place where its rows are whole 16-byte vectors
+  const bool g_direct = rows_direct(d_gy, d, ld);
+  float *Gcopy = nullptr, *H = nullptr, *Bf = nullptr;
   HT *Gb = nullptr, *Bb = nullptr;
-  if ((rc = B.get(&G, sz, "g")) || (rc = B.get(&H, sz, "h")) || (rc = B.get(&Bf, sz, "b")) ||
-      (rc = B.get(&GA, sz, "grad a")))
+  if ((!g_direct && (!k16 || params) && (rc = B.get(&Gcopy, sz, "g"))) || (rc = B.get(&H, sz, "h")) ||
+      (rc = B.get(&Bf, sz, "b")))
     return rc;
   if (k16 && ((rc = B.get(&Gb, sz, "g 16-bit")) || (rc = B.get(&Bb, sz, "b 16-bit")))) return rc;
-  const unsigned pg = (unsigned)std::min<int64_t>((total + 255) / 256, (int64_t)ctx->num_sms * 32);
-  k_pad_copy<HT><<<pg, 256, 0, st>>>(d_gy, n, d, sg, G, ld, Gb);
-  launches += 1;
+  const unsigned pg = (unsigned)std::min<int64_t>(((int64_t)sz + 255) / 256, (int64_t)ctx->num_sms * 32);
+  if (k16 || !g_direct) {
+    k_pad_copy<HT><<<pg, 256, 0, st>>>(d_gy, n, d, sg, Gcopy, ld, Gb);
+    launches += 1;
+  }
+  const float* G = g_direct ? d_gy : Gcopy;  // (Gcopy holds sg * g)
+  // the parameter gradients' sums
+  Dots dots;
+  if (params) {
+    dots.K = order > 2 ? order : 2;
+    dots.places = spmm_places(ctx, g->plan);
+    if ((rc = B.get(&dots.part, (size_t)2 * dots.K * dots.places, "dot partials"))) return rc;
+    LNE_CUDA_TRY(cudaMemsetAsync(dots.part, 0, sizeof(double) * 2 * dots.K * dots.places, st));
+    dots.ld = ld;
+    dots.a = d_a;
+    if (!rows_direct(d_a, d, ld)) {
+      float* Acopy = nullptr;
+      if ((rc = B.get(&Acopy, sz, "a"))) return rc;
+      k_pad_copy<__nv_bfloat16><<<pg, 256, 0, st>>>(d_a, n, d, 1.0f, Acopy, ld, nullptr);
+      launches += 1;
+      dots.a = Acopy;
+    }
+  }
+  if (k16 && params) {
+    // The parameter gradients run in FP32 in every form: they are sums over
+    // the orders whose terms cancel, so 16-bit gathers would cost them far
+    // more relative accuracy than they cost dL/da.  The 16-bit forms run an
+    // FP32 recursion for them, before dL/da is written.
+    Filter<float> F32{ctx, g, n, ld, F.coef, &launches, &B, &work};
+    float* B32 = nullptr;
+    if ((rc = B.get(&B32, sz, "b fp32"))) return rc;
+    EpiAdjInit<float> epi{F.coef, G, ld, nullptr, B32, nullptr, g_direct ? sg : 1.0f};
+    if ((rc = F32.spmm(G, epi))) return rc;
+    if ((rc = F32.run(B32, nullptr, 1.0f, order, c, FinalOut<__nv_bfloat16>(), &dots))) return rc;
+  }
   // h = (A + I) g, b = D~^-1 h
   {
     const XT* Gx = F.op(G, Gb);
-    EpiAdjInit<XT> epi{coef, Gx, ld, H, Bf, Bb};
-    if ((rc = spmm_run<XT>(ctx, F.R, g->plan, Gx, ld, ld, epi, &launches))) return rc;
+    EpiAdjInit<XT> epi{F.coef, Gx, ld, H, Bf, Bb, 1.0f};
+    if ((rc = F.spmm(Gx, epi))) return rc;
   }
   // grad a = h - D~ sum_k c_k T_k(X) b      (M^T = D~ M D~^-1)
-  if ((rc = F.run(Bf, Bb, order, c, H, true, GA, nullptr))) return rc;
-  if (d_ga) {
+  const bool out_direct = d_ga && rows_direct(d_ga, d, ld);
+  float* GA = nullptr;
+  if (!out_direct && (rc = B.get(&GA, sz, "grad a"))) return rc;
+  FinalOut<HT> fin;
+  fin.base = H;
+  fin.scale_dt = true;
+  fin.out = out_direct ? d_ga : GA;
+  fin.out_scale = out_direct ? 1.0f / sg : 1.0f;
+  if ((rc = F.run(Bf, Bb, 1.0f, order, c, fin, !k16 && params ? &dots : nullptr))) return rc;
+  if (d_ga && !out_direct) {
     k_unpad_copy<<<pg, 256, 0, st>>>(GA, ld, n, d, 1.0f / sg, d_ga);
     launches += 1;
   }
-  if (h_dmu || h_ds) {
-    // The parameter gradients run in FP32 in every form: they are sums over
-    // the orders whose terms cancel, so 16-bit gathers would cost them far
-    // more relative accuracy than they cost dL/da.  The 16-bit forms first
-    // form an FP32 h = (A + I) g from the FP32 copy of (scaled) g.
-    Filter<float> F32{ctx, g, F.R, n, ld, coef, &launches, &B};
-    const float* H32 = H;
-    if (k16) {
-      float *H2 = nullptr, *Bs = nullptr;
-      if ((rc = B.get(&H2, sz, "h fp32")) || (rc = B.get(&Bs, sz, "b fp32"))) return rc;
-      EpiAdjInit<float> epi{coef, G, ld, H2, Bs, nullptr};
-      if ((rc = spmm_run<float>(ctx, F32.R, g->plan, G, ld, ld, epi, &launches))) return rc;
-      H32 = H2;
-    }
-    if ((rc = param_grads(ctx, F32, p, c, H32, d_a, 1.0 / (double)sg, h_dmu, h_ds))) return rc;
+  if (params) {
+    if ((rc = param_grads(ctx, p, c, dots, B, &launches, 1.0 / (double)sg, h_dmu, h_ds))) return rc;
   }
-  cudaEventRecord(ev1, st);
-  LNE_CUDA_TRY(cudaEventSynchronize(ev1));
+  cudaEventRecord(ev.e[1], st);
+  LNE_CUDA_TRY(cudaEventSynchronize(ev.e[1]));
   LNE_CUDA_TRY(cudaGetLastError());
   if (stats) {
     memset(stats, 0, sizeof(*stats));
-    cudaEventElapsedTime(&stats->ms_total, ev0, ev1);
+    cudaEventElapsedTime(&stats->ms_total, ev.e[0], ev.e[1]);
     stats->kernel_launches = launches;
   }
   ctx->launch_count += launches;
-  cudaEventDestroy(ev0);
-  cudaEventDestroy(ev1);
   return LNE_OK;
 }
 

@@ -58,8 +58,15 @@ struct EpiStore {
   int d;
   bool add;
   float scale = 1.0f;
+  using State = NoState;
   template <int N>
-  __device__ __forceinline__ void operator()(int64_t r, int e0, const float (&a)[N]) const {
+  using Pre = NoPre;
+  template <int N>
+  __device__ __forceinline__ NoPre load(int64_t, int) const {
+    return NoPre();
+  }
+  template <int N>
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&a)[N], const NoPre&, NoState&) const {
     float* y = Y + r * ldy + e0;
 #pragma unroll
     for (int i = 0; i < N; ++i)

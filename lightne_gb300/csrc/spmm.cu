@@ -12,74 +12,79 @@
 
 namespace lne {
 
+// Items of a row by class (SpmmPlan): `heavy` counts the big items in the
+// high half and the other heavy ones in the low half, `light` the rest.
 template <class Rows>
-__global__ void k_plan_count(Rows R, int64_t n, int64_t* __restrict__ is_short, int64_t* __restrict__ nchunk,
-                             int64_t* __restrict__ is_long) {
+__global__ void k_plan_count(Rows R, int64_t n, int warp_max, int64_t* __restrict__ heavy, int64_t* __restrict__ light) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
   const int64_t len = R.end(r) - R.begin(r);
-  const bool lg = len > kChunkNnz;
-  is_short[r] = lg ? 0 : 1;
-  is_long[r] = lg ? 1 : 0;
-  nchunk[r] = lg ? (len + kChunkNnz - 1) / kChunkNnz : 0;
+  const bool big = len > kChunkNnz || len > max(kBigNnz, warp_max);
+  heavy[r] = big ? ((len + kChunkNnz - 1) / kChunkNnz) << 32 : (len > warp_max ? 1 : 0);
+  light[r] = len > warp_max ? 0 : 1;
 }
 
 template <class Rows>
-__global__ void k_plan_fill(Rows R, int64_t n, const int64_t* __restrict__ pos_short,
-                            const int64_t* __restrict__ pos_chunk, const int64_t* __restrict__ pos_long,
-                            SpmmPlan p) {
+__global__ void k_plan_fill(Rows R, int64_t n, int warp_max, const int64_t* __restrict__ heavy,
+                            const int64_t* __restrict__ light, SpmmPlan p) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
   const int64_t b = R.begin(r), len = R.end(r) - b;
-  if (len <= kChunkNnz) {
-    p.short_rows[pos_short[r]] = (uint32_t)r;
+  if (len <= warp_max) {
+    p.items[p.n_heavy + light[r]] = SpmmItem{b, (uint32_t)r, (uint32_t)len};
+  } else if (len <= kChunkNnz && len <= max(kBigNnz, warp_max)) {
+    p.items[p.n_big + (heavy[r] & 0xffffffffLL)] = SpmmItem{b, (uint32_t)r, (uint32_t)len};
   } else {
-    const int64_t L = pos_long[r], c0 = pos_chunk[r];
-    p.long_rows[L] = (uint32_t)r;
-    p.long_first[L] = c0;
-    const int64_t nc = (len + kChunkNnz - 1) / kChunkNnz;
-    for (int64_t c = 0; c < nc; ++c) {
-      p.chunk_row[c0 + c] = (uint32_t)r;
-      p.chunk_begin[c0 + c] = b + c * kChunkNnz;
+    const uint32_t c0 = (uint32_t)(heavy[r] >> 32), nc = (uint32_t)((len + kChunkNnz - 1) / kChunkNnz);
+    for (uint32_t c = 0; c < nc; ++c) {
+      const int64_t o = (int64_t)c * kChunkNnz;
+      p.items[c0 + c] = SpmmItem{b + o, (uint32_t)r, (uint32_t)(len - o < kChunkNnz ? len - o : kChunkNnz)};
+      p.span[c0 + c] = make_uint2(c0, nc);
     }
   }
-  if (r == n - 1) p.long_first[pos_long[n]] = pos_chunk[n];
+}
+
+// Longest row a single warp takes: a quarter of a resident warp's share of
+// the matrix (32 warps per SM), so that no warp's row outlasts the rest of
+// the launch.
+static int plan_warp_max(const lne_ctx* ctx, int64_t nnz) {
+  const int64_t share = nnz / ((int64_t)ctx->num_sms * 32 * 4);
+  int w = kWarpNnzMin;
+  while (w < kChunkNnz && 2 * (int64_t)w <= share) w *= 2;
+  return w;
 }
 
 template <class Rows>
-static int build_plan(lne_ctx* ctx, Rows R, int64_t n, SpmmPlan& plan) {
+static int build_plan(lne_ctx* ctx, Rows R, int64_t n, int64_t nnz, SpmmPlan& plan) {
   cudaStream_t st = ctx->stream;
-  int64_t* cnt = nullptr;  // 3 count arrays + 3 position arrays (n+1 each)
+  int64_t* cnt = nullptr;  // two counts and their positions (n + 1 each)
   void* tmp = nullptr;
   int rc;
-  if ((rc = dalloc(ctx, (void**)&cnt, sizeof(int64_t) * 6 * (n + 1), "spmm plan counts"))) return rc;
+  if ((rc = dalloc(ctx, (void**)&cnt, sizeof(int64_t) * 4 * (n + 1), "spmm plan counts"))) return rc;
   if ((rc = dalloc(ctx, &tmp, scan_tmp_bytes(n), "spmm plan scan"))) { dfree(ctx, cnt); return rc; }
-  int64_t *is_short = cnt, *nchunk = cnt + (n + 1), *is_long = cnt + 2 * (n + 1);
-  int64_t *pos_short = cnt + 3 * (n + 1), *pos_chunk = cnt + 4 * (n + 1), *pos_long = cnt + 5 * (n + 1);
+  int64_t *heavy = cnt, *light = cnt + (n + 1), *pos_heavy = cnt + 2 * (n + 1), *pos_light = cnt + 3 * (n + 1);
   const unsigned g = (unsigned)((n + 255) / 256);
-  k_plan_count<<<g, 256, 0, st>>>(R, n, is_short, nchunk, is_long);
-  scan_exclusive_i64(is_short, pos_short, n, tmp, st);
-  scan_exclusive_i64(nchunk, pos_chunk, n, tmp, st);
-  scan_exclusive_i64(is_long, pos_long, n, tmp, st);
-  int64_t tot[3];
-  LNE_CUDA_TRY(cudaMemcpyAsync(&tot[0], pos_short + n, 8, cudaMemcpyDeviceToHost, st));
-  LNE_CUDA_TRY(cudaMemcpyAsync(&tot[1], pos_chunk + n, 8, cudaMemcpyDeviceToHost, st));
-  LNE_CUDA_TRY(cudaMemcpyAsync(&tot[2], pos_long + n, 8, cudaMemcpyDeviceToHost, st));
+  plan.warp_max = plan_warp_max(ctx, nnz);
+  k_plan_count<<<g, 256, 0, st>>>(R, n, plan.warp_max, heavy, light);
+  scan_exclusive_i64(heavy, pos_heavy, n, tmp, st);
+  scan_exclusive_i64(light, pos_light, n, tmp, st);
+  int64_t tot[2] = {0, 0};
+  LNE_CUDA_TRY(cudaMemcpyAsync(&tot[0], pos_heavy + n, 8, cudaMemcpyDeviceToHost, st));
+  LNE_CUDA_TRY(cudaMemcpyAsync(&tot[1], pos_light + n, 8, cudaMemcpyDeviceToHost, st));
   LNE_CUDA_TRY(cudaStreamSynchronize(st));
-  plan.n_short = tot[0];
-  plan.n_chunks = tot[1];
-  plan.n_long = tot[2];
-  const size_t bytes = sizeof(uint32_t) * (plan.n_short + plan.n_chunks + plan.n_long) +
-                       sizeof(int64_t) * (plan.n_chunks + plan.n_long + 1) + 64;
+  plan.n_big = tot[0] >> 32;
+  plan.n_heavy = plan.n_big + (tot[0] & 0xffffffffLL);
+  plan.n_items = plan.n_heavy + tot[1];
   char* m = nullptr;
-  if ((rc = dalloc(ctx, (void**)&m, bytes, "spmm plan"))) { dfree(ctx, tmp); dfree(ctx, cnt); return rc; }
+  if ((rc = dalloc(ctx, (void**)&m, sizeof(SpmmItem) * plan.n_items + sizeof(uint2) * plan.n_big + 64, "spmm plan"))) {
+    dfree(ctx, tmp);
+    dfree(ctx, cnt);
+    return rc;
+  }
   plan.mem = m;
-  plan.chunk_begin = (int64_t*)m;
-  plan.long_first = plan.chunk_begin + plan.n_chunks;
-  plan.short_rows = (uint32_t*)(plan.long_first + plan.n_long + 1);
-  plan.chunk_row = plan.short_rows + plan.n_short;
-  plan.long_rows = plan.chunk_row + plan.n_chunks;
-  k_plan_fill<<<g, 256, 0, st>>>(R, n, pos_short, pos_chunk, pos_long, plan);
+  plan.items = reinterpret_cast<SpmmItem*>(m);
+  plan.span = reinterpret_cast<uint2*>(plan.items + plan.n_items);
+  k_plan_fill<<<g, 256, 0, st>>>(R, n, plan.warp_max, pos_heavy, pos_light, plan);
   dfree(ctx, tmp);
   dfree(ctx, cnt);
   LNE_CUDA_TRY(cudaGetLastError());
@@ -88,16 +93,14 @@ static int build_plan(lne_ctx* ctx, Rows R, int64_t n, SpmmPlan& plan) {
 
 int build_plan_csr(lne_ctx* ctx, lne_csr* c) {
   if (c->plan_ready) return LNE_OK;
-  CsrRows R{c->row_ptr, c->col, c->val};
-  int rc = build_plan(ctx, R, c->n, c->plan);
+  int rc = build_plan(ctx, CsrRows{c->row_ptr}, c->n, c->nnz, c->plan);
   if (rc == LNE_OK) c->plan_ready = true;
   return rc;
 }
 
 int build_plan_graph(lne_ctx* ctx, lne_graph* g) {
   if (g->plan_ready) return LNE_OK;
-  GraphRows R{g->vdata, g->nbrs};
-  int rc = build_plan(ctx, R, g->n, g->plan);
+  int rc = build_plan(ctx, GraphRows{g->vdata}, g->n, g->m_dir, g->plan);
   if (rc == LNE_OK) g->plan_ready = true;
   return rc;
 }
@@ -195,8 +198,8 @@ int build_panels(lne_ctx* ctx, lne_csr* c, const std::vector<int64_t>& bounds) {
   c->panel_bounds = bounds;
   c->panel_plans.resize(np);
   for (int p = 0; p < np; ++p) {
-    PanelRows R{c->row_ptr, seg, c->col, c->val, np + 1, p};
-    if ((rc = build_plan(ctx, R, n, c->panel_plans[p]))) {
+    PanelRows R{c->row_ptr, seg, np + 1, p};
+    if ((rc = build_plan(ctx, R, n, c->nnz, c->panel_plans[p]))) {
       free_panels(c);
       return rc;
     }
@@ -212,8 +215,15 @@ struct EpiAxpby {
   int64_t ldy;
   int d;
   bool add;
+  using State = NoState;
   template <int N>
-  __device__ __forceinline__ void operator()(int64_t r, int e0, const float (&a)[N]) const {
+  using Pre = NoPre;
+  template <int N>
+  __device__ __forceinline__ NoPre load(int64_t, int) const {
+    return NoPre();
+  }
+  template <int N>
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&a)[N], const NoPre&, NoState&) const {
     float* y = Y + r * ldy + e0;
 #pragma unroll
     for (int i = 0; i < N; ++i) {

@@ -1,17 +1,27 @@
 // Row-parallel SpMM core: Y[i,:] = epi(i, sum_j v_ij * X[c_ij, :]).
 //
-// Work is split into items so that no warp walks more than kChunkNnz
-// nonzeros: a row with at most kChunkNnz entries is one item; a longer row
-// is cut into chunks whose partial sums go to a scratch buffer and are added
-// in chunk order by a second kernel.  Every output is therefore a sum in a
-// fixed order: results are bitwise reproducible run to run.
+// Work is split into items (SpmmItem: first nonzero, row, length) of at most
+// kChunkNnz nonzeros; the partial sums of a longer row's chunks go to a
+// scratch buffer, and whoever finishes the row's last chunk adds them in
+// chunk order.  Every output is a sum in a fixed order, whichever kernel
+// takes the item: P = 32/G strands, strand g adding the nonzeros t with
+// t % P == g of the item one after the other in FP32, then the strands in a
+// balanced tree.  Results are bitwise reproducible run to run.
 //
-// Within an item the warp is split into P = 32/G groups of G lanes; lane gl
-// of a group owns the 16-byte column vectors gl, gl+G, ... of the row, and
-// group g takes the nonzeros t with t % P == g.  Column ids (and values) are
-// loaded up to 32 at a time, one per lane, and broadcast with shuffles; the
-// gathers of several nonzeros are issued before their FMAs so that every
-// lane keeps several 16-byte loads in flight (SpmmTune).
+// In a warp, lane gl of group g owns the 16-byte column vectors gl, gl+G, ...
+// of the rows of strand g.  Column ids (and values) are loaded up to 32 at a
+// time, one per lane, and broadcast with shuffles; the gathers of several
+// nonzeros are issued before their FMAs so that every lane keeps several
+// 16-byte loads in flight (SpmmTune).
+//
+// On a sparse graph an item is a handful of gathers, and a warp that loads
+// the item, then its ids, then the rows, then the epilogue's operands waits
+// out four dependent latencies per row.  So the items run as a pipeline: while
+// one is gathered, the ids of the next are in flight, and the epilogue's
+// operands (Epi::load) are issued before the gathers.
+//
+// On graphs, and on matrices too small to hide a warp that walks a 2048-entry
+// row, the longer rows are taken first, by several warps each (balanced form).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -25,24 +35,23 @@ namespace lne {
 
 static constexpr unsigned kFull = 0xffffffffu;
 
-// Access to a sparse operator's rows.
-struct CsrRows {  // explicit CSR: int64 row_ptr, int32 col, float val
+// An epilogue without operands to load ahead, and without sums over rows.
+struct NoPre {};
+struct NoState {
+  static constexpr bool kSums = false;
+};
+
+// Row ranges of a sparse operator, from which a work list is built.
+struct CsrRows {  // explicit CSR: int64 row_ptr
   const int64_t* __restrict__ row_ptr;
-  const int32_t* __restrict__ col;
-  const float* __restrict__ val;
   __device__ __forceinline__ int64_t begin(int64_t r) const { return __ldg(row_ptr + r); }
   __device__ __forceinline__ int64_t end(int64_t r) const { return __ldg(row_ptr + r + 1); }
-  __device__ __forceinline__ uint32_t c(int64_t j) const { return (uint32_t)__ldg(col + j); }
-  __device__ __forceinline__ float v(int64_t j) const { return __ldg(val + j); }
-  static constexpr bool kHasVal = true;
 };
 
 // The entries of a CSR row whose columns fall in one column panel.
 struct PanelRows {
   const int64_t* __restrict__ row_ptr;
   const int32_t* __restrict__ seg;  // n x (np1) relative panel starts
-  const int32_t* __restrict__ col;
-  const float* __restrict__ val;
   int np1;                          // panels + 1
   int p;                            // this panel
   __device__ __forceinline__ int64_t begin(int64_t r) const {
@@ -51,111 +60,408 @@ struct PanelRows {
   __device__ __forceinline__ int64_t end(int64_t r) const {
     return __ldg(row_ptr + r) + __ldg(seg + r * np1 + p + 1);
   }
-  __device__ __forceinline__ uint32_t c(int64_t j) const { return (uint32_t)__ldg(col + j); }
-  __device__ __forceinline__ float v(int64_t j) const { return __ldg(val + j); }
-  static constexpr bool kHasVal = true;
 };
 
-struct GraphRows {  // graph adjacency: {offset, degree} per vertex, unit values
+struct GraphRows {  // graph adjacency: {offset, degree} per vertex
   const Vertex* __restrict__ vdata;
-  const uint32_t* __restrict__ nbrs;
   __device__ __forceinline__ int64_t begin(int64_t r) const { return (int64_t)__ldg(&vdata[r].off); }
   __device__ __forceinline__ int64_t end(int64_t r) const {
     return (int64_t)__ldg(&vdata[r].off) + (int64_t)__ldg(&vdata[r].deg);
   }
-  __device__ __forceinline__ uint32_t c(int64_t j) const { return __ldg(nbrs + j); }
-  __device__ __forceinline__ float v(int64_t) const { return 1.0f; }
-  static constexpr bool kHasVal = false;
 };
 
-// Gather depth of the raw-staged path (FP8 operands, 9-lane groups and
-// 128-element 16-bit rows): each lane issues the gathers of kU nonzeros
-// before their FMAs, kept as raw 16-byte words (4 registers each).  Column
-// ids are loaded in batches of kBatch <= 32, a multiple of the P kU
-// nonzeros a warp takes per step, so that no step of a batch runs
-// part-empty, and a step whose nonzeros are all in the batch loads without
-// predicates.  Measured at n = 1.14M, nnz = 351M (`B = A Q`, the sketch
-// product, the 19 SpMMs of the propagation), unpredicated full steps
-// included: a 144-element FP16 row at kU = 2 (batch 30) 11.1 ms against
-// 11.6 at 3 and 12.8 at 4; 144-element FP8 rows at kU = 5 (batch 30) 8.0
-// against 8.4 at 4 and 9.2 at 6; 128-element 16-bit rows on the graph
-// (the propagation) at kU = 5 (batch 30) 13.0 against 13.2 at 4 and 13.3
-// at 6.  Deeper staging spills (64 registers a thread at 4 CTAs of 256 per
-// SM); compiled for 3 CTAs per SM it lost more warps than it gained in
-// flight.  Other operands are widened at the load and staged kUnroll deep.
+// Gather depth: each lane issues the gathers of kU nonzeros before their
+// FMAs, kept as raw 16-byte words (4 registers each).  Column ids are loaded
+// in batches of kBatch <= 32, a multiple of the P kU nonzeros a warp takes
+// per step, so that no step of a batch runs part-empty, and a step whose
+// nonzeros are all in the batch loads without predicates.  Measured at
+// n = 1.14M, nnz = 351M (`B = A Q`, the sketch product, the 19 SpMMs of the
+// propagation), unpredicated full steps included: a 144-element FP16 row at
+// kU = 2 (batch 30) 11.1 ms against 11.6 at 3 and 12.8 at 4; 144-element FP8
+// rows at kU = 5 (batch 30) 8.0 against 8.4 at 4 and 9.2 at 6.  Deeper
+// staging spills (64 registers a thread at 4 CTAs of 256 per SM); compiled
+// for 3 CTAs per SM it lost more warps than it gained in flight.
 template <typename XT, int G, int VPL>
 struct SpmmTune {
   static constexpr int E = Vec16<XT>::E;
   static constexpr int P = 32 / G;
-  static constexpr bool kRaw = E == 16 || (G & (G - 1)) != 0 || (E == 8 && G == 16 && VPL == 1);
-  static constexpr int kWant = (G == 9 && VPL == 2)                               ? 2
-                               : VPL == 1 && (G == 9 || (G == 16 && E == 8)) ? 5
-                                                                                  : (VPL >= 4 ? 1 : 4 / VPL);
+  static constexpr int kWant = VPL == 1 ? (G == 9 ? 5 : 4) : (VPL == 2 ? (E == 8 && G == 32 ? 1 : 2) : 1);
   static constexpr int kU = kWant * P <= 32 ? kWant : 32 / P;
   static constexpr int kBatch = (32 / (P * kU)) * (P * kU);
   static_assert(kBatch >= 1 && kBatch <= 32, "a batch of column ids is one per lane");
+  // 16-bit vectors of one per lane: two groups share the epilogue, four
+  // elements of a vector each
+  static constexpr bool kSplit = E == 8 && VPL == 1 && G <= 16 && (G & (G - 1)) == 0;
+  static constexpr int kEpi = kSplit ? 4 : E;  // elements per epilogue call
 };
 
-template <typename XT, int VPL>
-struct Acc {
-  static constexpr int E = Vec16<XT>::E;
-  float a[VPL][E];
-  __device__ __forceinline__ void zero() {
+// What one SpMM launch reads besides the epilogue.
+template <typename XT>
+struct SpmmArgs {
+  const SpmmItem* __restrict__ items;
+  uint32_t n_items, n_big, n_heavy;    // see SpmmPlan
+  const uint2* __restrict__ span;      // [n_big] {first item of its row, items of its row}
+  const uint32_t* __restrict__ col;
+  const float* __restrict__ val;       // null: unit values
+  const XT* __restrict__ X;
+  int64_t ldx;
+  int C;                               // 16-byte vectors of the slab
+  float* partial;                      // [n_big][ldp]
+  int64_t ldp;
+  unsigned* done;                      // arrivals per long row (and part), zero between launches
+  int e_base;                          // first column of the slab
+};
+
+__device__ __forceinline__ int64_t item_begin(const uint4& it) {
+  return (int64_t)(((uint64_t)it.y << 32) | it.x);
+}
+
+static constexpr int kSpmmThreads = 256;
+static constexpr int kSpmmWarps = kSpmmThreads / 32;
+
+// ---------------------------------------------------------------------------
+// Balanced form (one 16-byte vector per lane, G a power of two): the rows
+// above warp_max go to k_spmm_heavy, with one 32-bit column word per lane
+// instead of one 16-byte vector, so that a 512-byte row is the work of four
+// warps and each lane keeps 96 rows in flight instead of four; a lane adds
+// its strands' rows in order, so the sums are those of k_spmm.  The rest go
+// to k_spmm (BAL), which starts beside it.  On a graph of 10,312 vertices
+// and 668K entries (128 FP32 columns) one product took 200 us with a warp
+// per row: a 2048-entry row is a chain of gathers that four rows in flight
+// leave waiting.  Passing the rows through shared memory to adding threads
+// took 110 us (51 instructions per entry), 32 rows in flight in registers
+// 110 us (about 1 us per 32 rows).
+// ---------------------------------------------------------------------------
+template <int G>
+struct HeavyTune {
+  static constexpr int P = 32 / G;
+  static constexpr int W = G * 4 < 32 ? G * 4 : 32;  // lanes of one row
+  static constexpr int LG = 32 / W;                  // rows side by side in a warp
+  static constexpr int A = P / LG;                   // strands per lane
+  static constexpr int kParts = G * 4 / W;           // warps of one row
+  static constexpr int kSets = 2;                    // sets of 32 rows in flight per lane
+};
+static constexpr int kHeavyWarps = 4;
+
+// Elements of one 32-bit word of a dense row, widened.
+template <typename XT>
+struct Word32;
+template <>
+struct Word32<float> {
+  static constexpr int E = 1;
+  __device__ __forceinline__ static void unpack(uint32_t w, float (&o)[1]) { o[0] = __uint_as_float(w); }
+};
+template <>
+struct Word32<__nv_bfloat16> {
+  static constexpr int E = 2;
+  __device__ __forceinline__ static void unpack(uint32_t w, float (&o)[2]) {
+    o[0] = __uint_as_float(w << 16);
+    o[1] = __uint_as_float(w & 0xffff0000u);
+  }
+};
+template <>
+struct Word32<__half> {
+  static constexpr int E = 2;
+  __device__ __forceinline__ static void unpack(uint32_t w, float (&o)[2]) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+    o[0] = f.x;
+    o[1] = f.y;
+  }
+};
+template <>
+struct Word32<__nv_fp8_e4m3> {
+  static constexpr int E = 4;
+  __device__ __forceinline__ static void unpack(uint32_t w, float (&o)[4]) {
 #pragma unroll
-    for (int k = 0; k < VPL; ++k)
-#pragma unroll
-      for (int e = 0; e < E; ++e) a[k][e] = 0.f;
+    for (int h = 0; h < 2; ++h) {
+      const __half2_raw r = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w >> (16 * h)), __NV_E4M3);
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&r));
+      o[2 * h] = f.x;
+      o[2 * h + 1] = f.y;
+    }
   }
 };
 
-// Accumulate nonzeros [j0, j1) of the operator into acc (per group), then
-// reduce across the P groups so that the lanes of group 0 hold the sums.
-template <typename XT, int G, int VPL, class Rows>
-__device__ __forceinline__ void spmm_accumulate(const Rows& R, int64_t j0, int64_t j1, const XT* __restrict__ X,
-                                                int64_t ldx, int C, Acc<XT, VPL>& acc) {
-  constexpr int P = 32 / G;
-  constexpr int E = Vec16<XT>::E;
+// One warp per part of a heavy item: lane group lg (W lanes) takes the
+// nonzeros t % LG == lg, lane q the word part * 32 + q of their rows.  The
+// hardware hands out the blocks in order, so the longest items start first.
+template <typename XT, int G, bool VAL, class Epi>
+__global__ void __launch_bounds__(kHeavyWarps * 32, 4) k_spmm_heavy(const SpmmArgs<XT> s, const Epi epi) {
+  using Tune = HeavyTune<G>;
+  constexpr int W = Tune::W, LG = Tune::LG, A = Tune::A, kSets = Tune::kSets, EW = Word32<XT>::E;
+  constexpr int kStep = 32 * LG;  // nonzeros of a set
+  // the light rows' kernel may start: it does not read what this one writes
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const uint32_t unit = blockIdx.x * kHeavyWarps + (threadIdx.x >> 5);
+  if (unit >= s.n_heavy * Tune::kParts) return;
+  const uint32_t it = unit / Tune::kParts;
+  const int part = (int)(unit % Tune::kParts);
+  const int lane = threadIdx.x & 31, lg = lane / W;
+  const int q = part * 32 + lane % W;
+  const bool on = q < s.C * 4;
+  const uint4 rec = __ldg(reinterpret_cast<const uint4*>(s.items) + it);
+  const uint32_t r = rec.z;
+  const int len = (int)rec.w;
+  const uint32_t* col = s.col + item_begin(rec);
+  const float* val = VAL ? s.val + item_begin(rec) : nullptr;
+  const uint32_t* X = reinterpret_cast<const uint32_t*>(s.X) + (on ? q : 0);
+  const uint32_t ldw = (uint32_t)(s.ldx * (int64_t)sizeof(XT) / 4);
+  float acc[A][EW];
+#pragma unroll
+  for (int a = 0; a < A; ++a)
+#pragma unroll
+    for (int e = 0; e < EW; ++e) acc[a][e] = 0.0f;
+  // Ids and values pass through shared memory, each lane group's together,
+  // so that one 16-byte broadcast serves four rows (a shuffle per row made
+  // a chain of 30 cycles each); 36 words apart the groups meet no bank twice.
+  __shared__ __align__(16) uint32_t sid[kHeavyWarps][LG * 36];
+  __shared__ __align__(16) float sva[VAL ? kHeavyWarps : 1][VAL ? kSets : 1][VAL ? LG * 36 : 1];
+  uint32_t* my_id = sid[threadIdx.x >> 5];
+  uint32_t w[kSets][32];  // words in flight
+  uint32_t c[LG];         // ids (and values) of the set after those
+  float v[LG];
+  auto load_ids = [&](int base) {
+#pragma unroll
+    for (int i = 0; i < LG; ++i) {
+      const int j = base + 32 * i + lane;
+      c[i] = j < len ? __ldg(col + j) : 0u;
+      if (VAL) v[i] = j < len ? __ldg(val + j) : 0.0f;
+    }
+  };
+  // the ids in c to shared memory, the next ones on their way, the gathers
+  auto gather = [&](int base, int set, uint32_t (&o)[32]) {
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < LG; ++i) {
+      const int at = 32 * i + lane;  // nonzero of the set: group at % LG, its at / LG-th
+      my_id[(at % LG) * 36 + at / LG] = c[i];
+      if (VAL) sva[threadIdx.x >> 5][set][(at % LG) * 36 + at / LG] = v[i];
+    }
+    __syncwarp();
+    load_ids(base + kStep);
+    const uint4* ids = reinterpret_cast<const uint4*>(my_id + lg * 36);
+    if (base + kStep <= len) {
+#pragma unroll
+      for (int u = 0; u < 32; u += 4) {
+        const uint4 cc = ids[u / 4];
+        o[u] = __ldg(X + (uint64_t)cc.x * ldw);
+        o[u + 1] = __ldg(X + (uint64_t)cc.y * ldw);
+        o[u + 2] = __ldg(X + (uint64_t)cc.z * ldw);
+        o[u + 3] = __ldg(X + (uint64_t)cc.w * ldw);
+      }
+    } else if (base < len) {
+#pragma unroll
+      for (int u = 0; u < 32; u += 4) {
+        const uint4 cc = ids[u / 4];
+        const uint32_t id[4] = {cc.x, cc.y, cc.z, cc.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          o[u + i] = base + (u + i) * LG + lg < len ? __ldg(X + (uint64_t)id[i] * ldw) : 0u;
+      }
+    }
+  };
+  auto add = [&](int base, int set, const uint32_t (&o)[32]) {
+    const float4* vs = reinterpret_cast<const float4*>(sva[VAL ? threadIdx.x >> 5 : 0][VAL ? set : 0] + (VAL ? lg * 36 : 0));
+    auto four = [&](int u, auto whole) {
+      const float4 m4 = VAL ? vs[u / 4] : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+      const float m[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float x[EW];
+        Word32<XT>::unpack(o[u + i], x);
+        if (decltype(whole)::value || base + (u + i) * LG + lg < len) {
+#pragma unroll
+          for (int e = 0; e < EW; ++e) acc[(u + i) % A][e] = fmaf(m[i], x[e], acc[(u + i) % A][e]);
+        }
+      }
+    };
+    if (base + kStep <= len) {
+#pragma unroll
+      for (int u = 0; u < 32; u += 4) four(u, std::true_type{});
+    } else if (base < len) {
+#pragma unroll
+      for (int u = 0; u < 32; u += 4) four(u, std::false_type{});
+    }
+  };
+  load_ids(0);
+#pragma unroll
+  for (int k = 0; k < kSets; ++k) gather(k * kStep, k, w[k]);
+  for (int base = 0; base < len; base += kSets * kStep) {
+#pragma unroll
+    for (int k = 0; k < kSets; ++k) {
+      add(base + k * kStep, k, w[k]);
+      __syncwarp();
+      gather(base + (k + kSets) * kStep, k, w[k]);
+    }
+  }
+  // the strands in a balanced tree: strand lg + LG a is acc[a] of group lg
+#pragma unroll
+  for (int o = W; o < 32; o <<= 1)
+#pragma unroll
+    for (int a = 0; a < A; ++a)
+#pragma unroll
+      for (int e = 0; e < EW; ++e) acc[a][e] += __shfl_xor_sync(kFull, acc[a][e], o);
+#pragma unroll
+  for (int o = 1; o < A; o <<= 1)
+#pragma unroll
+    for (int a = 0; a + o < A; a += 2 * o)
+#pragma unroll
+      for (int e = 0; e < EW; ++e) acc[a][e] += acc[a + o][e];
+  const bool out = on && lane < W;
+  const int e0 = q * EW;
+  uint32_t place = it;
+  const uint2 sp = it < s.n_big ? __ldg(s.span + it) : make_uint2(it, 1);
+  if (sp.y > 1) {
+    // a chunk: the warp that completes its row's last one adds them, in order
+    place = sp.x;
+    if (out) {
+#pragma unroll
+      for (int e = 0; e < EW; ++e) __stcg(s.partial + (int64_t)it * s.ldp + e0 + e, acc[0][e]);
+    }
+    __threadfence();
+    __syncwarp();
+    unsigned* done = s.done + (int64_t)sp.x * Tune::kParts + part;
+    unsigned before = 0;
+    if (lane == 0) before = atomicAdd(done, 1u);
+    before = __shfl_sync(kFull, before, 0);
+    if (before + 1 != sp.y) return;
+    __threadfence();
+    if (lane == 0) *done = 0;  // ready for the next launch
+    if (out) {
+      const float* p = s.partial + (int64_t)sp.x * s.ldp + e0;
+#pragma unroll
+      for (int e = 0; e < EW; ++e) acc[0][e] = 0.0f;
+      constexpr int kD = 8;  // chunks in flight
+      for (unsigned i = 0; i < sp.y; i += kD) {
+        float t[kD][EW];
+#pragma unroll
+        for (int d = 0; d < kD; ++d)
+#pragma unroll
+          for (int e = 0; e < EW; ++e) t[d][e] = i + d < sp.y ? __ldcg(p + (int64_t)(i + d) * s.ldp + e) : 0.0f;
+#pragma unroll
+        for (int d = 0; d < kD; ++d)
+          if (i + d < sp.y)
+#pragma unroll
+            for (int e = 0; e < EW; ++e) acc[0][e] += t[d][e];
+      }
+    }
+  }
+  typename Epi::State state;
+  if (out) {
+    const auto pre = epi.template load<EW>(r, s.e_base + e0);
+    epi.template store<EW>(r, s.e_base + e0, acc[0], pre, state);
+  }
+  if constexpr (Epi::State::kSums) state.put(epi.dot, place * Tune::kParts + part);
+}
+
+// Every item to a warp, or (BAL) the rows of at most warp_max entries.
+template <typename XT, int G, int VPL, bool VAL, bool BAL, class Epi>
+__global__ void __launch_bounds__(kSpmmThreads, 4) k_spmm(const SpmmArgs<XT> s, const Epi epi) {
+  using Tune = SpmmTune<XT, G, VPL>;
+  constexpr int E = Tune::E, P = Tune::P, kU = Tune::kU, kB = Tune::kBatch, N = Tune::kEpi;
+  constexpr bool kSplit = Tune::kSplit;
+  // The operands of wider epilogues would not fit the registers beside the
+  // gathers, nor would the next ids beside 16 sums per lane (whose matrices,
+  // the sparsifier's, have hundreds of entries per row).
+  constexpr bool kHoist = VPL == 1 && N == 4;
+  constexpr bool kPipe = !VAL || VPL * E < 16;
   const int lane = threadIdx.x & 31;
   const int grp = lane / G, gl = lane % G;
-  if constexpr (SpmmTune<XT, G, VPL>::kRaw) {
-    // FP8 vectors, a group of 9 lanes or 16 lanes of 16-bit vectors: the
-    // gathers of kU nonzeros are staged as raw 16-byte words, widened at
-    // the FMAs
-    constexpr int kU = SpmmTune<XT, G, VPL>::kU;
-    // G = 9 (a 144-element row: 9 FP8 vectors, or 18 BF16 / FP16 vectors
-    // at two per lane): three groups of 9 lanes, lanes 27..31 idle
-    const bool in_grp = grp < P;
-    constexpr int kB = SpmmTune<XT, G, VPL>::kBatch;
-    // a step whose P kU nonzeros are all in the batch, on a slab that fills
-    // the lane layout, loads without predicates: lanes past the groups
-    // (27..31) read rows of valid columns too and their sums are not used
-    const bool full_cols = C == G * VPL;
-    for (int64_t base = j0; base < j1; base += kB) {
-      const int cnt = (int)((j1 - base) < kB ? (j1 - base) : kB);
-      const uint32_t c = lane < cnt ? R.c(base + lane) : 0u;
-      const float v = Rows::kHasVal ? (lane < cnt ? R.v(base + lane) : 0.f) : 1.f;
+  // G = 9: three groups of 9 lanes, lanes 27..31 idle
+  const bool in_grp = grp < P;
+  const bool epi_lane = lane < (kSplit ? 2 * G : G);
+  const int e_lane = kSplit ? 4 * (grp & 1) : 0;
+  // a step whose P kU nonzeros are all in the batch, on a slab that fills
+  // the lane layout, loads without predicates: lanes past the groups
+  // (27..31) read rows of valid columns too and their sums are not used
+  const bool full_cols = s.C == G * VPL;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  uint32_t it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if constexpr (BAL) {
+    static_assert(VPL == 1 && (G & (G - 1)) == 0, "the balanced form has one vector per lane");
+    it += s.n_heavy;
+  }
+  static_assert(BAL || !Epi::State::kSums, "sums over rows are taken by the balanced form");
+  typename Epi::State state;
+  const uint4* items = reinterpret_cast<const uint4*>(s.items);
+  const uint4 none = make_uint4(0, 0, 0, 0);
+  uint4 nxt = it < s.n_items ? __ldg(items + it) : none;
+  uint32_t c = 0;
+  float v = 1.0f;
+  if constexpr (kPipe) {
+    const int cnt = (int)nxt.w < kB ? (int)nxt.w : kB;
+    if (lane < cnt) c = __ldg(s.col + item_begin(nxt) + lane);
+    if (VAL) v = lane < cnt ? __ldg(s.val + item_begin(nxt) + lane) : 0.0f;
+  }
+  for (; it < s.n_items; it += nwarps) {
+    const uint2 sp = !BAL && it < s.n_big ? __ldg(s.span + it) : make_uint2(it, 1);
+    const bool chunk = !BAL && sp.y > 1;
+    const uint32_t r = nxt.z;
+    int left = (int)nxt.w;               // nonzeros from jb on
+    int64_t jb = item_begin(nxt);
+    if constexpr (kPipe) nxt = it + nwarps < s.n_items ? __ldg(items + it + nwarps) : none;
+    typename Epi::template Pre<N> pre[VPL];
+    if (kHoist && !chunk && epi_lane) {
+#pragma unroll
+      for (int k = 0; k < VPL; ++k) {
+        const int ch = gl + G * k;
+        if (ch < s.C) pre[k] = epi.template load<N>(r, s.e_base + ch * E + e_lane);
+      }
+    }
+    float acc[VPL][E];
+#pragma unroll
+    for (int k = 0; k < VPL; ++k)
+#pragma unroll
+      for (int e = 0; e < E; ++e) acc[k][e] = 0.f;
+    do {
+      const int cnt = left < kB ? left : kB;
+      if constexpr (!kPipe) {
+        c = lane < cnt ? __ldg(s.col + jb + lane) : 0u;
+        if (VAL) v = lane < cnt ? __ldg(s.val + jb + lane) : 0.0f;
+      }
+      uint32_t c2 = 0;
+      float v2 = 1.0f;
+      bool fetched = !kPipe;
+      // the ids after these: the item's next batch, or the next item's first
+      auto fetch = [&]() {
+        fetched = true;
+        const bool last = left <= kB;
+        const int64_t j2 = last ? item_begin(nxt) : jb + kB;
+        int cnt2 = last ? (int)nxt.w : left - kB;
+        cnt2 = cnt2 < kB ? cnt2 : kB;
+        if (lane < cnt2) c2 = __ldg(s.col + j2 + lane);
+        if (VAL) v2 = lane < cnt2 ? __ldg(s.val + j2 + lane) : 0.0f;
+      };
       auto step = [&](int t0, auto checked) {
         constexpr bool kChecked = decltype(checked)::value;
         uint4 raw[kU][VPL];
         float vv[kU];
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
+          if (kChecked && u > 0 && t0 + u * P >= cnt) {  // the same for the whole warp
+            vv[u] = 0.0f;
+#pragma unroll
+            for (int k = 0; k < VPL; ++k) raw[u][k] = make_uint4(0, 0, 0, 0);
+            continue;
+          }
           const int t = t0 + u * P + grp;
           const uint32_t cc = __shfl_sync(kFull, c, t & 31);
-          vv[u] = Rows::kHasVal ? __shfl_sync(kFull, v, t & 31) : 1.f;
-          const XT* xr = X + (int64_t)cc * ldx;
+          vv[u] = VAL ? __shfl_sync(kFull, v, t & 31) : 1.f;
+          const XT* xr = s.X + (int64_t)cc * s.ldx;
 #pragma unroll
           for (int k = 0; k < VPL; ++k) {
             const int ch = gl + G * k;
             if constexpr (kChecked)
-              raw[u][k] = (in_grp && t < cnt && ch < C) ? __ldg(reinterpret_cast<const uint4*>(xr + ch * E))
-                                                         : make_uint4(0, 0, 0, 0);
+              raw[u][k] = (in_grp && t < cnt && ch < s.C) ? __ldg(reinterpret_cast<const uint4*>(xr + ch * E))
+                                                          : make_uint4(0, 0, 0, 0);
             else
               raw[u][k] = __ldg(reinterpret_cast<const uint4*>(xr + ch * E));
           }
         }
+        if (!fetched) fetch();  // behind the first gathers, ahead of their FMAs
 #pragma unroll
-        for (int u = 0; u < kU; ++u)
+        for (int u = 0; u < kU; ++u) {
+          if (kChecked && u > 0 && t0 + u * P >= cnt) break;
 #pragma unroll
           for (int k = 0; k < VPL; ++k) {
             float x[E];
@@ -163,12 +469,13 @@ __device__ __forceinline__ void spmm_accumulate(const Rows& R, int64_t j0, int64
             // paired FP32 FMAs: each element rounded as by fmaf
 #pragma unroll
             for (int e = 0; e < E; e += 2) {
-              const float2 r = __ffma2_rn(make_float2(vv[u], vv[u]), make_float2(x[e], x[e + 1]),
-                                          make_float2(acc.a[k][e], acc.a[k][e + 1]));
-              acc.a[k][e] = r.x;
-              acc.a[k][e + 1] = r.y;
+              const float2 q = __ffma2_rn(make_float2(vv[u], vv[u]), make_float2(x[e], x[e + 1]),
+                                          make_float2(acc[k][e], acc[k][e + 1]));
+              acc[k][e] = q.x;
+              acc[k][e + 1] = q.y;
             }
           }
+        }
       };
       for (int t0 = 0; t0 < cnt; t0 += P * kU) {
         if (full_cols && t0 + P * kU <= cnt)
@@ -176,140 +483,122 @@ __device__ __forceinline__ void spmm_accumulate(const Rows& R, int64_t j0, int64
         else
           step(t0, std::true_type{});
       }
-    }
-    if constexpr ((G & (G - 1)) == 0) {
+      if (kPipe && !fetched) fetch();  // an empty row
+      left -= kB;
+      jb += kB;
+      if constexpr (kPipe) {
+        c = c2;
+        v = v2;
+      }
+    } while (left > 0);
+    if constexpr (!kPipe) nxt = it + nwarps < s.n_items ? __ldg(items + it + nwarps) : none;
+
+    // add the groups' sums: in sum[k], the elements of this lane's epilogue
+    float sum[VPL][N];
+    if constexpr (kSplit) {
+      // the two halves of a vector change places between neighbouring groups
+      const bool hi = grp & 1;
 #pragma unroll
-      for (int o = G; o < 32; o <<= 1)
+      for (int e = 0; e < 4; ++e) {
+        const float give = hi ? acc[0][e] : acc[0][4 + e];
+        const float keep = hi ? acc[0][4 + e] : acc[0][e];
+        sum[0][e] = keep + __shfl_xor_sync(kFull, give, G);
+      }
 #pragma unroll
-        for (int k = 0; k < VPL; ++k)
+      for (int o = 2 * G; o < 32; o <<= 1)
 #pragma unroll
-          for (int e = 0; e < E; ++e) acc.a[k][e] += __shfl_xor_sync(kFull, acc.a[k][e], o);
+        for (int e = 0; e < 4; ++e) sum[0][e] += __shfl_xor_sync(kFull, sum[0][e], o);
     } else {
-      static_assert(P == 3, "non-power-of-two groups: three groups per warp");
+      if constexpr ((G & (G - 1)) == 0) {
 #pragma unroll
-      for (int k = 0; k < VPL; ++k)
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-          const float g1 = __shfl_down_sync(kFull, acc.a[k][e], G);
-          const float g2 = __shfl_down_sync(kFull, acc.a[k][e], 2 * G);
-          acc.a[k][e] = (acc.a[k][e] + g1) + g2;
-        }
-    }
-  } else {
-    // nonzeros whose gathers are in flight per lane: about 16 staged floats
-    constexpr int kStaged = 16 / (VPL * E);
-    constexpr int kUnroll = kStaged < 1 ? 1 : (kStaged > 4 ? 4 : kStaged);
-    for (int64_t base = j0; base < j1; base += 32) {
-      const int cnt = (int)((j1 - base) < 32 ? (j1 - base) : 32);
-      const uint32_t c = lane < cnt ? R.c(base + lane) : 0u;
-      const float v = Rows::kHasVal ? (lane < cnt ? R.v(base + lane) : 0.f) : 1.f;
-      for (int t0 = 0; t0 < cnt; t0 += P * kUnroll) {
-        uint32_t cc[kUnroll];
-        float vv[kUnroll];
-        float x[kUnroll][VPL][E];
-#pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-          const int t = t0 + u * P + grp;
-          cc[u] = __shfl_sync(kFull, c, t & 31);
-          vv[u] = Rows::kHasVal ? __shfl_sync(kFull, v, t & 31) : 1.f;
-          const XT* xr = X + (int64_t)cc[u] * ldx;
-#pragma unroll
-          for (int k = 0; k < VPL; ++k) {
-            const int ch = gl + G * k;
-            if (t < cnt && ch < C) {
-              Vec16<XT>::load(xr + ch * E, x[u][k]);
-            } else {
-#pragma unroll
-              for (int e = 0; e < E; ++e) x[u][k][e] = 0.f;
-            }
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kUnroll; ++u)
+        for (int o = G; o < 32; o <<= 1)
 #pragma unroll
           for (int k = 0; k < VPL; ++k)
 #pragma unroll
-            for (int e = 0; e < E; ++e) acc.a[k][e] = fmaf(vv[u], x[u][k][e], acc.a[k][e]);
-      }
-    }
+            for (int e = 0; e < E; ++e) acc[k][e] += __shfl_xor_sync(kFull, acc[k][e], o);
+      } else {
+        static_assert(P == 3, "non-power-of-two groups: three groups per warp");
 #pragma unroll
-    for (int o = G; o < 32; o <<= 1)
+        for (int k = 0; k < VPL; ++k)
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            const float g1 = __shfl_down_sync(kFull, acc[k][e], G);
+            const float g2 = __shfl_down_sync(kFull, acc[k][e], 2 * G);
+            acc[k][e] = (acc[k][e] + g1) + g2;
+          }
+      }
 #pragma unroll
       for (int k = 0; k < VPL; ++k)
 #pragma unroll
-        for (int e = 0; e < E; ++e) acc.a[k][e] += __shfl_xor_sync(kFull, acc.a[k][e], o);
-  }
-}
+        for (int e = 0; e < N; ++e) sum[k][e] = acc[k][e];
+    }
 
-// Main kernel: short rows call the epilogue directly; chunks of long rows
-// store partial sums (FP32, ld = ldp) for k_spmm_finish.
-template <typename XT, int G, int VPL, class Rows, class Epi>
-__global__ void __launch_bounds__(256, 4) k_spmm(Rows R, SpmmPlan plan, const XT* __restrict__ X, int64_t ldx, int C,
-                                              float* __restrict__ partial, int64_t ldp, int e_base, Epi epi) {
-  constexpr int E = Vec16<XT>::E;
-  const int lane = threadIdx.x & 31;
-  const int gl = lane % G;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t items = plan.n_short + plan.n_chunks;
-  for (int64_t it = warp; it < items; it += nwarps) {
-    Acc<XT, VPL> acc;
-    acc.zero();
-    if (it < plan.n_short) {
-      const uint32_t r = __ldg(plan.short_rows + it);
-      spmm_accumulate<XT, G, VPL>(R, R.begin(r), R.end(r), X, ldx, C, acc);
-      if (lane < G) {
+    if (!chunk) {
+      if (epi_lane) {
 #pragma unroll
         for (int k = 0; k < VPL; ++k) {
           const int ch = gl + G * k;
-          if (ch < C) epi(r, e_base + ch * E, acc.a[k]);
+          if (ch >= s.C) continue;
+          if (!kHoist) pre[k] = epi.template load<N>(r, s.e_base + ch * E + e_lane);
+          epi.template store<N>(r, s.e_base + ch * E + e_lane, sum[k], pre[k], state);
         }
       }
     } else {
-      const int64_t ci = it - plan.n_short;
-      const int64_t b = __ldg(plan.chunk_begin + ci);
-      const uint32_t r = __ldg(plan.chunk_row + ci);
-      int64_t e = R.end(r);
-      const int64_t lim = b + kChunkNnz;
-      e = e < lim ? e : lim;
-      spmm_accumulate<XT, G, VPL>(R, b, e, X, ldx, C, acc);
-      if (lane < G) {
+      if (epi_lane) {
 #pragma unroll
         for (int k = 0; k < VPL; ++k) {
           const int ch = gl + G * k;
-          if (ch < C) {
-            float* p = partial + ci * ldp + ch * E;
+          if (ch < s.C) {
+            float* p = s.partial + (int64_t)it * s.ldp + ch * E + e_lane;
 #pragma unroll
-            for (int q = 0; q < E; q += 4)
-              *reinterpret_cast<float4*>(p + q) = make_float4(acc.a[k][q], acc.a[k][q + 1], acc.a[k][q + 2],
-                                                             acc.a[k][q + 3]);
+            for (int q = 0; q < N; q += 4)
+              __stcg(reinterpret_cast<float4*>(p + q), make_float4(sum[k][q], sum[k][q + 1], sum[k][q + 2], sum[k][q + 3]));
           }
         }
       }
-    }
-  }
-}
-
-// Long rows: add the chunk partials in order and apply the epilogue.
-// One warp per long row; lanes cover the row in 16-byte (4-float) vectors.
-template <class Epi>
-__global__ void k_spmm_finish(SpmmPlan plan, const float* __restrict__ partial, int64_t ldp, int cols, int e_base,
-                              Epi epi) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t w = warp; w < plan.n_long; w += nwarps) {
-    const uint32_t r = plan.long_rows[w];
-    const int64_t c0 = plan.long_first[w], c1 = plan.long_first[w + 1];
-    for (int q = lane * 4; q < cols; q += 128) {
-      float s[4] = {0.f, 0.f, 0.f, 0.f};
-      for (int64_t ci = c0; ci < c1; ++ci) {
-        const float4 v = *reinterpret_cast<const float4*>(partial + ci * ldp + q);
-        s[0] += v.x; s[1] += v.y; s[2] += v.z; s[3] += v.w;
+      // the warp that completes the row's last chunk adds them all, in order
+      __threadfence();
+      __syncwarp();
+      unsigned before = 0;
+      if (lane == 0) before = atomicAdd(s.done + sp.x, 1u);
+      before = __shfl_sync(kFull, before, 0);
+      if (before + 1 == sp.y) {
+        __threadfence();
+        if (lane == 0) s.done[sp.x] = 0;  // ready for the next launch
+        const int cols = s.C * E;
+        for (int q = lane * 4; q < cols; q += 128) {
+          const auto fin = epi.template load<4>(r, s.e_base + q);
+          const float* p = s.partial + (int64_t)sp.x * s.ldp + q;
+          float t[4] = {0.f, 0.f, 0.f, 0.f};
+          constexpr int kD = 4;  // chunks in flight
+          for (unsigned i = 0; i < sp.y; i += kD) {
+            float4 w[kD];
+#pragma unroll
+            for (int d = 0; d < kD; ++d)
+              w[d] = i + d < sp.y ? __ldcg(reinterpret_cast<const float4*>(p + (int64_t)(i + d) * s.ldp))
+                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int d = 0; d < kD; ++d) {
+              if (i + d < sp.y) {
+                t[0] += w[d].x;
+                t[1] += w[d].y;
+                t[2] += w[d].z;
+                t[3] += w[d].w;
+              }
+            }
+          }
+          epi.template store<4>(r, s.e_base + q, t, fin, state);
+        }
+        __syncwarp();
       }
-      epi(r, e_base + q, s);
     }
   }
+  if constexpr (Epi::State::kSums)
+    state.put(epi.dot, s.n_heavy * HeavyTune<G>::kParts + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5));
+  // Launched beside k_spmm_heavy, whose blocks have all started by then:
+  // this launch ends after that one, so that what follows it on the stream
+  // sees the rows of both.
+  if constexpr (BAL) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 }  // namespace lne

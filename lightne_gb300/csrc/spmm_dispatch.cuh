@@ -10,18 +10,83 @@
 
 namespace lne {
 
-template <typename XT, int G, int VPL, class Rows, class Epi>
-static void spmm_launch(lne_ctx* ctx, Rows R, const SpmmPlan& plan, const XT* X, int64_t ldx, int C, float* partial,
-                        int64_t ldp, int e_base, const Epi& epi) {
-  const int64_t items = plan.n_short + plan.n_chunks;
-  int64_t blocks = (items + 7) / 8;
+template <typename XT, int G, int VPL, bool VAL, class Epi>
+static void spmm_launch(lne_ctx* ctx, const SpmmArgs<XT>& s, const Epi& epi, int* nl) {
+  int64_t blocks = ((int64_t)s.n_items + kSpmmWarps - 1) / kSpmmWarps;
   const int64_t cap = (int64_t)ctx->num_sms * 16;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
-  k_spmm<XT, G, VPL, Rows, Epi><<<(unsigned)blocks, 256, 0, ctx->stream>>>(R, plan, X, ldx, C, partial, ldp, e_base,
-                                                                          epi);
+  k_spmm<XT, G, VPL, VAL, false, Epi><<<(unsigned)blocks, kSpmmThreads, 0, ctx->stream>>>(s, epi);
+  *nl += 1;
 }
 
+static constexpr int kSpmmPartsMax = HeavyTune<32>::kParts;
+// Blocks of the light rows of the balanced form: persistent, four per SM.
+static inline int64_t spmm_bal_blocks(const lne_ctx* ctx, const SpmmPlan& plan) {
+  const int64_t want = (plan.n_items - plan.n_heavy + kSpmmWarps - 1) / kSpmmWarps;
+  return std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->num_sms * 4));
+}
+// Places of the sums an epilogue takes over the rows: one per part of a
+// heavy item, one per warp.
+static inline int64_t spmm_places(const lne_ctx* ctx, const SpmmPlan& plan) {
+  return plan.n_heavy * kSpmmPartsMax + spmm_bal_blocks(ctx, plan) * kSpmmWarps;
+}
+
+// The heavy rows, and the light rows beside them (programmatic dependent
+// launch: the second kernel starts once the first one's blocks all have, and
+// ends after it).  Adds the launches to *nl.
+template <typename XT, int G, bool VAL, class Epi>
+static void spmm_launch_bal(lne_ctx* ctx, const SpmmPlan& plan, const SpmmArgs<XT>& s, const Epi& epi, int* nl) {
+  const int64_t units = plan.n_heavy * HeavyTune<G>::kParts;
+  if (units > 0) {
+    k_spmm_heavy<XT, G, VAL, Epi>
+        <<<(unsigned)((units + kHeavyWarps - 1) / kHeavyWarps), kHeavyWarps * 32, 0, ctx->stream>>>(s, epi);
+    *nl += 1;
+  }
+  if (plan.n_items == plan.n_heavy) return;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3((unsigned)spmm_bal_blocks(ctx, plan), 1, 1);
+  cfg.blockDim = dim3(kSpmmThreads, 1, 1);
+  cfg.stream = ctx->stream;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = units > 0 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k_spmm<XT, G, 1, VAL, true, Epi>, s, epi);
+  *nl += 1;
+}
+
+// Scratch of the launches over a plan, owned by one call: partial sums of
+// the chunks up to `width` floats wide and their arrival counters (launches
+// on a stream follow one another and leave them at zero).
+struct SpmmWork {
+  float* partial = nullptr;
+  unsigned* done = nullptr;
+};
+static inline int spmm_work_alloc(lne_ctx* ctx, const SpmmPlan& plan, int64_t width, SpmmWork* w) {
+  *w = SpmmWork();
+  if (plan.n_big == 0) return LNE_OK;
+  const size_t pb = sizeof(float) * (size_t)plan.n_big * (size_t)width;  // width: a multiple of 4 floats
+  const size_t zb = sizeof(unsigned) * kSpmmPartsMax * (size_t)plan.n_big;
+  int rc = dalloc(ctx, (void**)&w->partial, pb + zb, "spmm partials");
+  if (rc) return rc;
+  w->done = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(w->partial) + pb);
+  LNE_CUDA_TRY(cudaMemsetAsync(w->done, 0, zb, ctx->stream));
+  return LNE_OK;
+}
+static inline void spmm_work_free(lne_ctx* ctx, SpmmWork* w) {
+  if (w->partial) dfree(ctx, w->partial);
+  *w = SpmmWork();
+}
+// Floats per chunk that a product with d columns needs (slabs of at most 128
+// vectors).
+template <typename XT>
+static inline int64_t spmm_work_width(int64_t d) {
+  constexpr int E = Vec16<XT>::E;
+  const int64_t vecs = (d + E - 1) / E;
+  return (vecs < 128 ? vecs : 128) * E;
+}
 // Copies columns [v0, v0 + C) (16-byte vectors) of the x_rows rows of X
 // into a dense x_rows x C array.
 static __global__ void k_slab_copy(const uint4* __restrict__ X, int64_t ldv, int64_t v0, int64_t x_rows, int C,
@@ -40,17 +105,25 @@ static __global__ void k_slab_copy(const uint4* __restrict__ X, int64_t ldv, int
 // per row of X, so the copy stays in L2 while the slab's gathers run.
 static constexpr int64_t kSlabCopyMaxBytes = (int64_t)96 << 20;
 
-// Runs Y-epilogue(A * X) over all rows.  X rows: ldx elements, 16-byte
+// Runs Y-epilogue(A * X) over all rows.  A: the work list `plan` over the
+// column ids `col` (and values, null: ones).  X rows: ldx elements, 16-byte
 // aligned; d columns are produced (the epilogue sees element offsets).
 // x_rows (the rows of X; 0 if unknown) enables the tail-slab copies.
-template <typename XT, class Rows, class Epi>
-static int spmm_run(lne_ctx* ctx, Rows R, const SpmmPlan& plan, const XT* X, int64_t ldx, int64_t d, const Epi& epi,
-                    int* launches = nullptr, int64_t x_rows = 0) {
+template <typename XT, bool VAL, class Epi>
+static int spmm_run(lne_ctx* ctx, const SpmmPlan& plan, const uint32_t* col, const float* val, const XT* X, int64_t ldx,
+                    int64_t d, const Epi& epi, int* launches = nullptr, int64_t x_rows = 0,
+                    const SpmmWork* work = nullptr) {
   constexpr int E = Vec16<XT>::E;
   const int64_t c_total = (d + E - 1) / E;
-  float* partial = nullptr;
   int rc;
   int nl = 0;
+  // graphs, and matrices too small for a warp to take every row alone
+  const bool bal = !VAL || plan.warp_max < kChunkNnz;
+  SpmmWork own;
+  if (!work) {
+    if ((rc = spmm_work_alloc(ctx, plan, spmm_work_width<XT>(d), &own))) return rc;
+    work = &own;
+  }
   // Column slabs of a power-of-two number of 16-byte vectors (at most 128),
   // largest first: each slab fills its lane layout exactly (a 144-wide FP32
   // row is a 32-vector slab and a 4-vector slab, not 36 vectors on 32 lanes).
@@ -63,18 +136,15 @@ static int spmm_run(lne_ctx* ctx, Rows R, const SpmmPlan& plan, const XT* X, int
     // its tail shares the gathers of the row instead of a second pass
     if (E == 16 && rem == 9) C2 = 9;
     if (E == 8 && rem == 18) C2 = 18;
+    // from 32 vectors on a row is one strand: narrower slabs, same sums
+    if (bal && C2 > 32) C2 = 32;
     const int C = (int)C2;
-    const int64_t ldp = (int64_t)C * E;
-    if (plan.n_chunks > 0 && partial == nullptr) {
-      const int64_t w = (c_total < 128 ? c_total : 128) * E;
-      if ((rc = dalloc(ctx, (void**)&partial, sizeof(float) * plan.n_chunks * w, "spmm partials"))) return rc;
-    }
     const XT* Xs = X + c_off * E;
     int64_t ldxs = ldx;
     XT* slab = nullptr;
-    if (c_off > 0 && x_rows > 0 && x_rows * C * 16 <= kSlabCopyMaxBytes) {
+    if (c_off > 0 && C < 32 && x_rows > 0 && x_rows * C * 16 <= kSlabCopyMaxBytes) {
       if ((rc = dalloc(ctx, (void**)&slab, (size_t)(x_rows * C * 16), "spmm slab copy"))) {
-        if (partial) dfree(ctx, partial);
+        spmm_work_free(ctx, &own);
         return rc;
       }
       const int64_t nv = x_rows * C;
@@ -86,43 +156,60 @@ static int spmm_run(lne_ctx* ctx, Rows R, const SpmmPlan& plan, const XT* X, int
       Xs = slab;
       ldxs = (int64_t)C * E;
     }
-    const int e_base = (int)(c_off * E);
-    if (E == 8 && C == 18) {
-      if constexpr (E == 8) spmm_launch<XT, 9, 2>(ctx, R, plan, Xs, ldxs, C, partial, ldp, e_base, epi);
-    } else if (E == 16 && (C == 1 || C == 9)) {
-      // FP8: one lane per nonzero for one vector, three 9-lane groups for a
-      // 144-element row (instantiated for FP8 only)
-      if constexpr (E == 16) {
-        if (C == 1)
-          spmm_launch<XT, 1, 1>(ctx, R, plan, Xs, ldxs, C, partial, ldp, e_base, epi);
-        else
-          spmm_launch<XT, 9, 1>(ctx, R, plan, Xs, ldxs, C, partial, ldp, e_base, epi);
-      }
-    } else if (C <= 2)
-      spmm_launch<XT, 2, 1>(ctx, R, plan, Xs, ldxs, C, partial, ldp, e_base, epi);
-    else if (C <= 4)
-      spmm_launch<XT, 4, 1>(ctx, R, plan, Xs, ldxs, C, partial, ldp, e_base, epi);
-    else if (C <= 8)
-      spmm_launch<XT, 8, 1>(ctx, R, plan, Xs, ldxs, C, partial, ldp, e_base, epi);
-    else if (C <= 16)
-      spmm_launch<XT, 16, 1>(ctx, R, plan, Xs, ldxs, C, partial, ldp, e_base, epi);
-    else if (C <= 32)
-      spmm_launch<XT, 32, 1>(ctx, R, plan, Xs, ldxs, C, partial, ldp, e_base, epi);
-    else if (C <= 64)
-      spmm_launch<XT, 32, 2>(ctx, R, plan, Xs, ldxs, C, partial, ldp, e_base, epi);
-    else
-      spmm_launch<XT, 32, 4>(ctx, R, plan, Xs, ldxs, C, partial, ldp, e_base, epi);
-    ++nl;
-    if (plan.n_long > 0) {
-      int64_t blocks = (plan.n_long + 7) / 8;
-      if (blocks > (int64_t)ctx->num_sms * 8) blocks = (int64_t)ctx->num_sms * 8;
-      k_spmm_finish<Epi><<<(unsigned)blocks, 256, 0, ctx->stream>>>(plan, partial, ldp, (int)ldp, e_base, epi);
-      ++nl;
+    SpmmArgs<XT> s;
+    s.items = plan.items;
+    s.n_items = (uint32_t)plan.n_items;
+    s.n_big = (uint32_t)plan.n_big;
+    s.n_heavy = (uint32_t)plan.n_heavy;
+    s.span = plan.span;
+    s.col = col;
+    s.val = val;
+    s.X = Xs;
+    s.ldx = ldxs;
+    s.C = C;
+    s.partial = work->partial;
+    s.ldp = (int64_t)C * E;
+    s.done = work->done;
+    s.e_base = (int)(c_off * E);
+    const bool nine = (E == 8 && C == 18) || (E == 16 && C == 9);
+    if (bal && !nine && !(E == 16 && C == 1)) {
+      if (C <= 2)
+        spmm_launch_bal<XT, 2, VAL>(ctx, plan, s, epi, &nl);
+      else if (C <= 4)
+        spmm_launch_bal<XT, 4, VAL>(ctx, plan, s, epi, &nl);
+      else if (C <= 8)
+        spmm_launch_bal<XT, 8, VAL>(ctx, plan, s, epi, &nl);
+      else if (C <= 16)
+        spmm_launch_bal<XT, 16, VAL>(ctx, plan, s, epi, &nl);
+      else
+        spmm_launch_bal<XT, 32, VAL>(ctx, plan, s, epi, &nl);
+    } else if (nine) {
+      // E == 4 rows have no 9-lane layout, and sums over rows none either
+      if constexpr (E == 8) spmm_launch<XT, 9, 2, VAL>(ctx, s, epi, &nl);
+      if constexpr (E == 16) spmm_launch<XT, 9, 1, VAL>(ctx, s, epi, &nl);
+    } else if (E == 16 && C == 1) {
+      // FP8: one lane per nonzero for one vector
+      if constexpr (E == 16) spmm_launch<XT, 1, 1, VAL>(ctx, s, epi, &nl);
+    } else if constexpr (VAL) {
+      if (C <= 2)
+        spmm_launch<XT, 2, 1, VAL>(ctx, s, epi, &nl);
+      else if (C <= 4)
+        spmm_launch<XT, 4, 1, VAL>(ctx, s, epi, &nl);
+      else if (C <= 8)
+        spmm_launch<XT, 8, 1, VAL>(ctx, s, epi, &nl);
+      else if (C <= 16)
+        spmm_launch<XT, 16, 1, VAL>(ctx, s, epi, &nl);
+      else if (C <= 32)
+        spmm_launch<XT, 32, 1, VAL>(ctx, s, epi, &nl);
+      else if (C <= 64)
+        spmm_launch<XT, 32, 2, VAL>(ctx, s, epi, &nl);
+      else
+        spmm_launch<XT, 32, 4, VAL>(ctx, s, epi, &nl);
     }
     if (slab) dfree(ctx, slab);
     c_off += C;
   }
-  if (partial) dfree(ctx, partial);
+  spmm_work_free(ctx, &own);
   if (launches) *launches += nl;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -159,9 +246,9 @@ static int spmm_csr_panels(lne_ctx* ctx, lne_csr* A, const XT* X, int64_t ldx, i
   if (budget == 0 || xbytes <= budget) {
     if (!A->plan_ready && launches) *launches += kPlanLaunches;
     if ((rc = build_plan_csr(ctx, A))) return rc;
-    CsrRows R{A->row_ptr, A->col, A->val};
     epi.add = false;
-    return spmm_run<XT>(ctx, R, A->plan, X, ldx, d, epi, launches, A->n);
+    return spmm_run<XT, true>(ctx, A->plan, reinterpret_cast<const uint32_t*>(A->col), A->val, X, ldx, d, epi, launches,
+                              A->n);
   }
   const int64_t pw = std::max<int64_t>(1, budget / row_bytes);
   std::vector<int64_t> bounds{0};
@@ -174,9 +261,10 @@ static int spmm_csr_panels(lne_ctx* ctx, lne_csr* A, const XT* X, int64_t ldx, i
   if (A->panel_bounds != bounds && launches) *launches += 1 + (int)(bounds.size() - 1) * kPlanLaunches;
   if ((rc = build_panels(ctx, A, bounds))) return rc;
   for (int p = 0; p < A->npanels; ++p) {
-    PanelRows R{A->row_ptr, A->seg, A->col, A->val, A->npanels + 1, p};
     epi.add = p > 0;
-    if ((rc = spmm_run<XT>(ctx, R, A->panel_plans[p], X, ldx, d, epi, launches))) return rc;
+    if ((rc = spmm_run<XT, true>(ctx, A->panel_plans[p], reinterpret_cast<const uint32_t*>(A->col), A->val, X, ldx, d,
+                                 epi, launches)))
+      return rc;
   }
   return LNE_OK;
 }

@@ -423,15 +423,15 @@ __global__ void __launch_bounds__(256) k_chol_inv_cluster(const double* __restri
       for (int k = k0; k < k1; ++k) {
         double* ck = col + (size_t)(qs * kCholPanel + (k - k0)) * r;
         // FP64 division and square root are long instruction sequences on
-        // this part: one square root and one reciprocal per pivot, then
-        // the column is scaled by multiplications spread over all warps
+        // this part: one reciprocal square root per pivot, then the column
+        // is scaled by multiplications spread over all warps
         if (warp == 0) {  // one warp evaluates the pivot
           const double d = ck[k];
           const bool ok = d > 0.0 && isfinite(d);
-          const double piv = ok ? sqrt(d) : 1.0;
+          const double rp = ok ? rsqrt(d) : 1.0;
           if (lane == 0) {
-            prcp = 1.0 / piv;
-            ck[k] = piv;
+            prcp = rp;
+            ck[k] = ok ? d * rp : 1.0;
             if (!ok) bad = 1;
           }
         }
@@ -520,9 +520,155 @@ static size_t chol_cluster_smem(int r, int csize) {
   return sizeof(double) * (nps * kCholPanel * r + (size_t)kCholPanel * r + (size_t)r * r + 9 * (size_t)r);
 }
 
-// Launches k_chol_inv_cluster on a 16- or 8-CTA cluster; false if neither
+// The factorisation above for 144 < r <= kCholWideMax, whose L does not fit
+// every CTA's shared memory beside the panels: L goes to global memory, column
+// by column, with the reciprocals of its diagonal, and k_tri_inv_cols solves
+// for the columns of L^-1 over the whole device, a warp each.  At r = 256 the
+// one-block factorisation in global memory and the one-thread-per-column
+// inverse (k_cholesky, k_tri_inv_t) took 2.4 + 2.8 ms per call.
+constexpr int kCholWideMax = 512;
+
+__global__ void __launch_bounds__(256) k_chol_cluster(const double* __restrict__ G, int r, double shift,
+                                                      double* __restrict__ Lc, double* __restrict__ idg,
+                                                      int* __restrict__ status) {
+  extern __shared__ double chs[];
+  __shared__ int bad;
+  __shared__ double prcp;
+  const int csize = gridDim.x;
+  const int rank = (int)cluster_rank();
+  const int npan = (r + kCholPanel - 1) / kCholPanel;
+  const int nps = (npan + csize - 1) / csize;  // panel slots per CTA
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  double* col = chs;                               // [nps * 8][r]: my columns
+  double* pan = col + (size_t)nps * kCholPanel * r;  // [8][r]: the panel of this step
+  auto j_of = [&](int c) { return ((c / kCholPanel) * csize + rank) * kCholPanel + (c % kCholPanel); };
+  const int ncols = nps * kCholPanel;
+  for (int c = 0; c < ncols; ++c) {
+    const int j = j_of(c);
+    if (j < r)
+      for (int i = tid; i < r; i += blockDim.x) col[(size_t)c * r + i] = G[(size_t)j * r + i] + (i == j ? shift : 0.0);
+  }
+  if (tid == 0) bad = 0;
+  const uint32_t col_s = (uint32_t)__cvta_generic_to_shared(col);
+  const uint32_t bad_s = (uint32_t)__cvta_generic_to_shared(&bad);
+  cluster_barrier();
+  bool failed = false;
+  for (int q = 0; q < npan; ++q) {
+    const int own = q % csize, qs = q / csize;
+    const int k0 = q * kCholPanel, k1 = min(k0 + kCholPanel, r);
+    if (rank == own) {
+      for (int k = k0; k < k1; ++k) {
+        double* ck = col + (size_t)(qs * kCholPanel + (k - k0)) * r;
+        if (warp == 0) {
+          const double d = ck[k];
+          const bool ok = d > 0.0 && isfinite(d);
+          const double rp = ok ? rsqrt(d) : 1.0;
+          if (lane == 0) {
+            prcp = rp;
+            ck[k] = ok ? d * rp : 1.0;
+            idg[k] = rp;
+            if (!ok) bad = 1;
+          }
+        }
+        __syncthreads();
+        if (bad) break;
+        const double rp = prcp;
+        for (int i = k + 1 + tid; i < r; i += blockDim.x) ck[i] *= rp;
+        __syncthreads();
+        for (int j = k + 1 + warp; j < k1; j += nw) {
+          double* cj = col + (size_t)(qs * kCholPanel + (j - k0)) * r;
+          const double ljk = ck[j];
+          for (int i = j + lane; i < r; i += 32) cj[i] -= ck[i] * ljk;
+        }
+        __syncthreads();
+      }
+    }
+    cluster_barrier();
+    if (dsmem_ld32(dsmem_map(bad_s, (uint32_t)own))) {
+      failed = true;
+      break;
+    }
+    if (k1 < r) {
+      // the panel's rows k0.. into pan (column t of the panel at pan + t r)
+      const uint32_t src = dsmem_map(col_s + (uint32_t)(qs * kCholPanel * r) * 8u, (uint32_t)own);
+      for (int t = warp; t < kCholPanel; t += nw)
+        for (int i = k0 + lane; i < r; i += 32) pan[(size_t)t * r + i] = dsmem_ld(src + 8u * (uint32_t)(t * r + i));
+      __syncthreads();
+      // rank-8 update of my columns after the panel
+      for (int c = warp; c < ncols; c += nw) {
+        const int j = j_of(c);
+        if (j < k1 || j >= r) continue;
+        double lj[kCholPanel];
+#pragma unroll
+        for (int t = 0; t < kCholPanel; ++t) lj[t] = pan[(size_t)t * r + j];
+        double* cj = col + (size_t)c * r;
+        for (int i = j + lane; i < r; i += 32) {
+          double v = cj[i];
+#pragma unroll
+          for (int t = 0; t < kCholPanel; ++t) v -= pan[(size_t)t * r + i] * lj[t];
+          cj[i] = v;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  if (!failed) {
+    for (int c = warp; c < ncols; c += nw) {
+      const int j = j_of(c);
+      if (j >= r) continue;
+      for (int i = j + lane; i < r; i += 32) Lc[(size_t)j * r + i] = col[(size_t)c * r + i];
+    }
+  }
+  if (rank == 0 && tid == 0) *status = failed ? 1 : 0;
+  cluster_barrier();  // no CTA leaves while another may still read its shared memory
+}
+
+// Column j of X = L^-1 by column-oriented forward substitution, one warp (and
+// CTA) each: x_j = 1 / L_jj, x_i = -(sum_{k=j}^{i-1} L_ik x_k) / L_ii, the
+// sums of rows lane, lane + 32, ... in registers; row j of W = X^T.
+template <int PER>
+__global__ void __launch_bounds__(32) k_tri_inv_cols(const double* __restrict__ Lc, const double* __restrict__ idg,
+                                                     const int* __restrict__ status, int r, float* __restrict__ W) {
+  if (*status) return;
+  const int lane = threadIdx.x, j = blockIdx.x;
+  double s[PER], dg[PER];  // sums, then the solution; reciprocal diagonals
+#pragma unroll
+  for (int m = 0; m < PER; ++m) {
+    s[m] = 0.0;
+    dg[m] = 32 * m + lane < r ? idg[32 * m + lane] : 0.0;
+  }
+#pragma unroll
+  for (int m = 0; m < PER; ++m) {
+    if (32 * m + 31 < j || 32 * m >= r) continue;  // the same for the warp
+    const int k1 = min(32 * m + 32, r);
+    for (int k = max(32 * m, j); k < k1; ++k) {
+      const double* lk = Lc + (size_t)k * r;
+      double l[PER];
+#pragma unroll
+      for (int b = m; b < PER; ++b) {
+        const int i = 32 * b + lane;
+        l[b] = i > k && i < r ? lk[i] : 0.0;
+      }
+      // every lane has its own row's candidate; the one of row k counts
+      const double cand = k == j ? dg[m] : -s[m] * dg[m];
+      const double xk = __shfl_sync(0xffffffffu, cand, k - 32 * m);
+#pragma unroll
+      for (int b = m; b < PER; ++b) s[b] = fma(l[b], xk, s[b]);
+      if (lane == k - 32 * m) s[m] = xk;
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < PER; ++m) {
+    const int i = 32 * m + lane;
+    if (i < r) W[(size_t)j * r + i] = i < j ? 0.0f : (float)s[m];
+  }
+}
+
+// Launches `kern` (arguments args...) on one thread-block cluster of 16, else
+// 8 CTAs of 256 threads; smem(size) is its shared memory.  False if neither
 // size can be launched.
-static bool chol_inv_cluster_launch(lne_ctx* ctx, const double* G, int r, double shift, float* W, int* status) {
+template <class Kern, class Smem, class... Args>
+static bool cluster_launch(lne_ctx* ctx, Kern kern, Smem smem_of, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   cfg.blockDim = dim3(256, 1, 1);
@@ -531,15 +677,13 @@ static bool chol_inv_cluster_launch(lne_ctx* ctx, const double* G, int r, double
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   for (int cl : {16, 8}) {
-    const size_t smem = chol_cluster_smem(r, cl);
-    if (smem > ctx->smem_optin) continue;
-    if (cl == 16 &&
-        cudaFuncSetAttribute(k_chol_inv_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    const size_t smem = smem_of(cl);
+    if (smem + 1024 > ctx->smem_optin) continue;
+    if (cl == 16 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
       cudaGetLastError();
       continue;
     }
-    if (cudaFuncSetAttribute(k_chol_inv_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
       cudaGetLastError();
       continue;
     }
@@ -549,18 +693,35 @@ static bool chol_inv_cluster_launch(lne_ctx* ctx, const double* G, int r, double
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, k_chol_inv_cluster, &cfg) != cudaSuccess || nclusters < 1) {
+    if (cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) != cudaSuccess || nclusters < 1) {
       cudaGetLastError();
       continue;
     }
-    if (cudaLaunchKernelEx(&cfg, k_chol_inv_cluster, G, r, shift, W, status) == cudaSuccess) return true;
+    if (cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess) return true;
     cudaGetLastError();
   }
   return false;
 }
 
+static bool chol_wide_launch(lne_ctx* ctx, const double* G, int r, double shift, double* Lc, double* idg, int* status,
+                             float* W) {
+  auto smem = [r](int cl) {
+    const size_t npan = (size_t)(r + kCholPanel - 1) / kCholPanel;
+    return sizeof(double) * ((npan + cl - 1) / cl + 1) * kCholPanel * (size_t)r;
+  };
+  if (!cluster_launch(ctx, k_chol_cluster, smem, G, r, shift, Lc, idg, status)) return false;
+  if (r <= 160)
+    k_tri_inv_cols<5><<<(unsigned)r, 32, 0, ctx->stream>>>(Lc, idg, status, r, W);
+  else if (r <= 256)
+    k_tri_inv_cols<8><<<(unsigned)r, 32, 0, ctx->stream>>>(Lc, idg, status, r, W);
+  else
+    k_tri_inv_cols<16><<<(unsigned)r, 32, 0, ctx->stream>>>(Lc, idg, status, r, W);
+  return true;
+}
+
 int cholesky_inv_launches(lne_ctx* ctx, int r) {
   if (r <= kCholClusterMax) return 1;
+  if (r <= kCholWideMax) return 2;
   return (r <= kCholSmemMax && sizeof(double) * ((size_t)r * r + r) <= ctx->smem_optin) ? 1 : 2;
 }
 
@@ -568,11 +729,15 @@ int cholesky_inv(lne_ctx* ctx, double* G, int r, double shift, float* W) {
   double* X = nullptr;
   int* status = nullptr;
   int rc;
-  if ((rc = dalloc(ctx, (void**)&X, sizeof(double) * r * r + 16, "triangular inverse"))) return rc;
-  status = (int*)(X + (int64_t)r * r);
+  if ((rc = dalloc(ctx, (void**)&X, sizeof(double) * ((size_t)r * r + r) + 16, "triangular inverse"))) return rc;
+  double* idg = X + (int64_t)r * r;  // reciprocal diagonal (wide form)
+  status = (int*)(idg + r);
   const size_t csmem = sizeof(double) * ((size_t)r * r + r);
-  if (r <= kCholClusterMax && chol_inv_cluster_launch(ctx, G, r, shift, W, status)) {
+  if (r <= kCholClusterMax &&
+      cluster_launch(ctx, k_chol_inv_cluster, [r](int cl) { return chol_cluster_smem(r, cl); }, G, r, shift, W, status)) {
     // done on the cluster
+  } else if (r > kCholClusterMax && r <= kCholWideMax && chol_wide_launch(ctx, G, r, shift, X, idg, status, W)) {
+    // factored on the cluster, inverted over the device
   } else if (r <= kCholSmemMax && csmem <= ctx->smem_optin) {
     cudaFuncSetAttribute(k_chol_inv_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem);
     k_chol_inv_smem<<<1, 1024, csmem, ctx->stream>>>(G, r, shift, W, status);
@@ -829,6 +994,253 @@ __global__ void __launch_bounds__(256) k_jacobi_sweeps_dsmem(int r, double* __re
   if (blockIdx.x == 0 && threadIdx.x == 0) *sweeps_out = sweep < max_sweeps ? sweep + 1 : max_sweeps;
 }
 
+// The sweeps of k_jacobi_sweeps for 160 < r <= 32 PER with the columns in
+// distributed shared memory, arranged around the FP64 units, which are what
+// bounds it (two FP64 FMAs per clock and SM):
+//   - the squared norms are tracked as above, so a pair needs one dot
+//     product instead of three;
+//   - columns are kept scaled, column = scale * stored (fast rotations:
+//     x - t y, y + t x, both scales times c): two FMAs per element pair
+//     instead of four operations; the scales are folded in every sweep;
+//   - the rotations of a CTA's pairs are evaluated together by one warp, a
+//     pair per lane, instead of 32 times over by each pair's warp.
+// The rotations are those of k_jacobi_sweeps to FP64 rounding (same pairs,
+// same order, smaller angle), so the columns come out with the same signs.
+// At r = 256 the global-memory form took 28 ms.
+constexpr int kJacobiWideWarps = 8;
+
+// 1 / sqrt(x) for x in [2^-4, 2^4]: FP32 seed, two Newton steps.
+__device__ __forceinline__ double rsqrt_newton(double x) {
+  double y = (double)rsqrtf((float)x);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) y = y * fma(-0.5 * x * y, y, 1.5);
+  return y;
+}
+
+template <int PER>
+__global__ void __launch_bounds__(kJacobiWideWarps * 32) k_jacobi_sweeps_wide(int r, double* __restrict__ Wc,
+                                                                              int max_sweeps,
+                                                                              int* __restrict__ sweeps_out) {
+  extern __shared__ double jcols[];  // nslots columns (slot s: column s * csize + rank), then nslots {norm, scale}
+  __shared__ int rot_flag[kJacobiMaxSweeps];
+  __shared__ double part[kJacobiWideWarps][33];  // a pair's partial dot products
+  __shared__ double pa[kJacobiWideWarps][4];     // {norm p, scale p, norm q, scale q}
+  // {t q/p, t p/q, norm p, norm q, scale p, scale q, stored factors of p, q}
+  __shared__ double rot[kJacobiWideWarps][8];
+  __shared__ int act[kJacobiWideWarps];
+  __shared__ unsigned long long cmax;
+  __shared__ double csum;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int k = tid; k < kJacobiMaxSweeps; k += blockDim.x) rot_flag[k] = 0;
+  const int csize = gridDim.x;
+  const int rank = (int)cluster_rank();
+  const int cshift = __ffs(csize) - 1;  // csize is a power of two
+  const int nslots = (r + csize - 1) / csize;
+  double* ns = jcols + (size_t)nslots * r;  // {norm, scale} of slot s at 2 s
+  if (tid == 0) cmax = 0;
+  __syncthreads();
+  unsigned long long mx = 0;  // largest |entry|, as bits
+  for (int s = warp; s < nslots; s += kJacobiWideWarps) {
+    const int c = s * csize + rank;
+    for (int i = lane; i < r; i += 32) {
+      const double v = c < r ? Wc[(size_t)c * r + i] : 0.0;
+      jcols[(size_t)s * r + i] = v;
+      mx = max(mx, (unsigned long long)__double_as_longlong(fabs(v)));
+    }
+  }
+  atomicMax(&cmax, mx);
+  cluster_barrier();
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(jcols);
+  const uint32_t nbase = (uint32_t)__cvta_generic_to_shared(ns);
+  {
+    const uint32_t ma = (uint32_t)__cvta_generic_to_shared(&cmax);
+    for (int c = 0; c < csize; ++c) {
+      const unsigned long long v = (unsigned long long)__double_as_longlong(dsmem_ld(dsmem_map(ma, (uint32_t)c)));
+      mx = c == 0 ? v : max(mx, v);
+    }
+  }
+  // the sweeps run on the matrix scaled by a power of two to entries below 2
+  const int ex = (int)(mx >> 52);
+  const bool scaled = ex >= 1 && ex <= 2045;
+  const double down = scaled ? __longlong_as_double((long long)(2046 - ex) << 52) : 1.0;
+  const double up = scaled ? __longlong_as_double((long long)ex << 52) : 1.0;
+  for (int s = tid; s < nslots; s += blockDim.x) ns[2 * s + 1] = down;
+  const int rp = (r + 1) & ~1;
+  const int m = rp - 1;
+  const double tol2 = fmax(1e-30, 4.930380657631324e-32 * r);  // max(1e-15, sqrt(r) 2^-52)^2
+  double tiny = 0.0;
+  int sweep = 0;
+  for (; sweep < max_sweeps; ++sweep) {
+    // fold the scales in; fresh squared norms
+    __syncthreads();
+    for (int s = warp; s < nslots; s += kJacobiWideWarps) {
+      const double sc = ns[2 * s + 1];
+      double a = 0.0;
+      double* col = jcols + (size_t)s * r;
+      for (int i = lane; i < r; i += 32) {
+        const double v = sc * col[i];
+        col[i] = v;
+        a = fma(v, v, a);
+      }
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (lane == 0) {
+        ns[2 * s] = a;
+        ns[2 * s + 1] = 1.0;
+      }
+    }
+    __syncthreads();
+    if (sweep == 0) {
+      // A sweep leaves rounding noise of about eps |C|_F in a column (eps
+      // |x| of each partner x).  A column below 8 eps |C|_F is that noise:
+      // it is not rotated, or noise would rotate forever on a rank-deficient
+      // matrix.
+      if (tid == 0) {
+        double t = 0.0;
+        for (int s = 0; s < nslots; ++s) t += ns[2 * s];
+        csum = t;
+      }
+      cluster_barrier();
+      double fro2 = 0.0;
+      const uint32_t ca = (uint32_t)__cvta_generic_to_shared(&csum);
+      for (int c = 0; c < csize; ++c) fro2 += dsmem_ld(dsmem_map(ca, (uint32_t)c));
+      tiny = fro2 * 3.1554436208840472e-30;  // fro2 (8 2^-52)^2
+    } else {
+      cluster_barrier();
+    }
+    for (int s = 0; s < m; ++s) {
+      for (int pk0 = 0; pk0 < rp / 2; pk0 += kJacobiWideWarps * csize) {  // the same for the whole cluster
+        // the round-robin pairs of step s: (s + pk, s - pk) mod m, and (m, s)
+        const int pk = pk0 + warp * csize + rank;
+        int p = 0, q = 0;
+        bool live = pk < rp / 2;
+        if (live) {
+          if (pk == 0) {
+            p = m;
+            q = s;
+          } else {
+            p = s + pk;
+            if (p >= m) p -= m;
+            q = s - pk;
+            if (q < 0) q += m;
+          }
+          if (p >= r || q >= r) live = false;
+          if (p > q) { const int t = p; p = q; q = t; }
+        }
+        const uint32_t pc = (uint32_t)(p & (csize - 1)), qc = (uint32_t)(q & (csize - 1));
+        const uint32_t ap = dsmem_map(base + (uint32_t)((p >> cshift) * r) * 8u, pc);
+        const uint32_t aq = dsmem_map(base + (uint32_t)((q >> cshift) * r) * 8u, qc);
+        const uint32_t np_ = dsmem_map(nbase + (uint32_t)(p >> cshift) * 16u, pc);
+        const uint32_t nq_ = dsmem_map(nbase + (uint32_t)(q >> cshift) * 16u, qc);
+        double x[PER], y[PER];
+        if (live) {
+          if (lane < 4) pa[warp][lane] = dsmem_ld((lane < 2 ? np_ : nq_) + 8u * (lane & 1));
+#pragma unroll
+          for (int k = 0; k < PER; ++k) {
+            const int i = lane + 32 * k;
+            x[k] = i < r ? dsmem_ld(ap + 8u * i) : 0.0;
+            y[k] = i < r ? dsmem_ld(aq + 8u * i) : 0.0;
+          }
+          double g = 0.0;
+#pragma unroll
+          for (int k = 0; k < PER; ++k) g = fma(x[k], y[k], g);
+          part[warp][lane] = g;
+        }
+        if (lane == 0) act[warp] = live;
+        __syncthreads();
+        if (warp == 0) {
+          // four lanes add a pair's partial products, then one evaluates
+          // its rotation: t = tan of the smaller angle that makes the
+          // columns orthogonal, from d = b - a and h = 2 g scaled to [1, 2)
+          const int w = lane >> 2;
+          double g = 0.0;
+          const bool on = act[w] != 0;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) g += part[w][(lane & 3) + 4 * k];
+          g += __shfl_xor_sync(0xffffffffu, g, 1);
+          g += __shfl_xor_sync(0xffffffffu, g, 2);
+          if ((lane & 3) == 0) {
+            const double a = pa[w][0], dp = pa[w][1], b = pa[w][2], dq = pa[w][3];
+            g *= dp * dq;
+            bool go = on && g != 0.0 && a > tiny && b > tiny && g * g > tol2 * (a * b);
+            if (go) {
+              double d = b - a, h = 2.0 * g;
+              const double big = fmax(fabs(d), fabs(h));
+              // 2^-exponent of the larger
+              const double sc = __longlong_as_double((2046LL - ((__double_as_longlong(big) >> 52) & 0x7ff)) << 52);
+              d *= sc;
+              h *= sc;
+              const double root2 = fma(d, d, h * h);
+              const double ir = rsqrt_newton(root2);           // 1 / sqrt(d^2 + h^2)
+              const double c2 = fma(0.5 * fabs(d), ir, 0.5);   // cos^2, in [1/2, 1]
+              const double ic = rsqrt_newton(c2);              // 1 / cos
+              const double c = c2 * ic;
+              const double sn = 0.5 * fabs(h) * ir * ic * (d * h >= 0.0 ? 1.0 : -1.0);
+              const double t = sn * ic;
+              // scales dq / dp and its inverse, by FP32 seeds and Newton
+              double ip = (double)(1.0f / (float)dp), iq = (double)(1.0f / (float)dq);
+#pragma unroll
+              for (int i = 0; i < 2; ++i) {
+                ip = ip * fma(-dp, ip, 2.0);
+                iq = iq * fma(-dq, iq, 2.0);
+              }
+              const double cc = c * c, ss = sn * sn, cs2 = 2.0 * c * sn * g;
+              rot[w][0] = t * dq * ip;
+              rot[w][1] = t * dp * iq;
+              rot[w][2] = fmax(fma(cc, a, fma(ss, b, -cs2)), 0.0);
+              rot[w][3] = fmax(fma(ss, a, fma(cc, b, cs2)), 0.0);
+              // a scale that has shrunk far is raised by 2^30 (exact)
+              const bool up = dp * c < 9.3132257461547852e-10, uq = dq * c < 9.3132257461547852e-10;
+              rot[w][4] = dp * c * (up ? 1073741824.0 : 1.0);
+              rot[w][5] = dq * c * (uq ? 1073741824.0 : 1.0);
+              rot[w][6] = up ? 9.3132257461547852e-10 : 1.0;
+              rot[w][7] = uq ? 9.3132257461547852e-10 : 1.0;
+              rot_flag[sweep] = 1;
+            }
+            act[w] = go;
+          }
+        }
+        __syncthreads();
+        if (act[warp]) {
+          const double t1 = rot[warp][0], t2 = rot[warp][1], f1 = rot[warp][6], f2 = rot[warp][7];
+          const bool plain = f1 == 1.0 && f2 == 1.0;
+#pragma unroll
+          for (int k = 0; k < PER; ++k) {
+            const int i = lane + 32 * k;
+            if (i < r) {
+              double u = fma(-t1, y[k], x[k]), v = fma(t2, x[k], y[k]);
+              if (!plain) {
+                u *= f1;
+                v *= f2;
+              }
+              dsmem_st(ap + 8u * i, u);
+              dsmem_st(aq + 8u * i, v);
+            }
+          }
+          if (lane < 4) {
+            // {norm, scale} of p, then of q
+            const double v = rot[warp][lane < 2 ? 2 + 2 * lane : 3 + 2 * (lane - 2)];
+            dsmem_st((lane < 2 ? np_ : nq_) + 8u * (lane & 1), v);
+          }
+        }
+        __syncthreads();  // act, part and rot are rewritten
+      }
+      cluster_barrier();
+    }
+    int any = 0;
+    const uint32_t fa = (uint32_t)__cvta_generic_to_shared(&rot_flag[sweep]);
+    for (int c = 0; c < csize; ++c) any |= dsmem_ld32(dsmem_map(fa, (uint32_t)c));
+    if (!any) break;
+  }
+  cluster_barrier();  // no CTA leaves while another may still read its flags
+  for (int s = warp; s < nslots; s += kJacobiWideWarps) {
+    const int c = s * csize + rank;
+    const double sc = up * ns[2 * s + 1];
+    if (c < r)
+      for (int i = lane; i < r; i += 32) Wc[(size_t)c * r + i] = sc * jcols[(size_t)s * r + i];
+  }
+  if (blockIdx.x == 0 && tid == 0) *sweeps_out = sweep < max_sweeps ? sweep + 1 : max_sweeps;
+}
+
 // FP32 preconditioning of the FP64 sweeps (r <= 32 * kJacobiPer, one CTA):
 // one-sided Jacobi on an FP32 copy of C (scaled to unit largest entry), the
 // rotations accumulated in V from I, until no pair has |x.y| > kJacobiTol32
@@ -1036,29 +1448,34 @@ __global__ void __launch_bounds__(256) k_jacobi_ns(const double* __restrict__ X1
   if (i < r && j < r) Y[(int64_t)j * r + i] = fma(1.5, X[(int64_t)j * r + i], -0.5 * acc);
 }
 
-__global__ void k_jacobi_finish(int r, const double* __restrict__ Wc, double* __restrict__ U,
-                                double* __restrict__ S) {
-  __shared__ int order[1024];
-  __shared__ double norms[1024];
-  for (int j = threadIdx.x; j < r; j += blockDim.x) {
-    double s2 = 0.0;
-    for (int i = 0; i < r; ++i) s2 = fma(Wc[(int64_t)j * r + i], Wc[(int64_t)j * r + i], s2);
-    norms[j] = sqrt(s2);
-  }
+// Singular values: the column norms (a warp each).
+__global__ void k_jacobi_norms(int r, const double* __restrict__ Wc, double* __restrict__ norms) {
+  const int lane = threadIdx.x & 31, j = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (j >= r) return;
+  double s2 = 0.0;
+  for (int i = lane; i < r; i += 32) s2 = fma(Wc[(size_t)j * r + i], Wc[(size_t)j * r + i], s2);
+  for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  if (lane == 0) norms[j] = sqrt(s2);
+}
+
+// Block j writes column j, normalised, at its place in descending order (ties
+// by index).
+__global__ void k_jacobi_finish(int r, const double* __restrict__ Wc, const double* __restrict__ norms,
+                                double* __restrict__ U, double* __restrict__ S) {
+  __shared__ int place;
+  const int j = blockIdx.x;
+  if (threadIdx.x == 0) place = 0;
   __syncthreads();
-  for (int j = threadIdx.x; j < r; j += blockDim.x) {
-    int rank = 0;
-    for (int k = 0; k < r; ++k) rank += (norms[k] > norms[j]) || (norms[k] == norms[j] && k < j);
-    order[rank] = j;
-  }
+  const double nrm = norms[j];
+  int before = 0;
+  for (int k = threadIdx.x; k < r; k += blockDim.x) before += (norms[k] > nrm) || (norms[k] == nrm && k < j);
+  before = __reduce_add_sync(0xffffffffu, before);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&place, before);
   __syncthreads();
-  for (int64_t t = threadIdx.x; t < (int64_t)r * r; t += blockDim.x) {
-    const int i = (int)(t / r), jn = (int)(t % r);
-    const int j = order[jn];
-    const double nrm = norms[j];
-    U[t] = nrm > 0.0 ? Wc[(int64_t)j * r + i] / nrm : 0.0;
-  }
-  for (int jn = threadIdx.x; jn < r; jn += blockDim.x) S[jn] = norms[order[jn]];
+  const int jn = place;
+  for (int i = threadIdx.x; i < r; i += blockDim.x)
+    U[(size_t)i * r + jn] = nrm > 0.0 ? Wc[(size_t)j * r + i] / nrm : 0.0;
+  if (threadIdx.x == 0) S[jn] = nrm;
 }
 
 static size_t jacobi_precond_smem(int r) { return sizeof(float) * 2 * (size_t)r * jacobi32_stride(r); }
@@ -1067,7 +1484,7 @@ static bool jacobi_precond_applies(lne_ctx* ctx, int r) {
   return r <= 32 * kJacobi32Vec && jacobi_precond_smem(r) + 1024 <= ctx->smem_optin;
 }
 
-int jacobi_svd_launches(lne_ctx* ctx, int r) { return jacobi_precond_applies(ctx, r) ? 7 : 3; }
+int jacobi_svd_launches(lne_ctx* ctx, int r) { return jacobi_precond_applies(ctx, r) ? 8 : 4; }
 
 int jacobi_svd(lne_ctx* ctx, double* C, int r, double* U, double* S, int* sweeps_out, int* sweeps32_out,
                int fp64_sweep_cap) {
@@ -1083,14 +1500,15 @@ int jacobi_svd(lne_ctx* ctx, double* C, int r, double* U, double* S, int* sweeps
   double* Wc = nullptr;
   int rc;
   // Wc, then (preconditioned) V, P, M, V1, P1 (FP64 r x r each)
-  const size_t bytes = sizeof(double) * rr * (pre ? 6 : 1) + sizeof(int) * (kMaxSweeps + 4);
+  const size_t bytes = sizeof(double) * (rr * (pre ? 6 : 1) + r) + sizeof(int) * (kMaxSweeps + 4);
   if ((rc = dalloc(ctx, (void**)&Wc, bytes, "jacobi work"))) return rc;
   double* Vd = Wc + rr;
   double* Pc = Vd + rr;
   double* M = Pc + rr;
   double* V1 = M + rr;
   double* P1 = V1 + rr;
-  int* rotated = (int*)(Wc + rr * (pre ? 6 : 1));
+  double* norms = Wc + rr * (pre ? 6 : 1);
+  int* rotated = (int*)(norms + r);
   int* d_sw = rotated + kMaxSweeps;  // [0]: FP64 sweeps, [1]: FP32 sweeps
   LNE_CUDA_TRY(cudaMemsetAsync(d_sw + 1, 0, sizeof(int), ctx->stream));
   if (pre) {
@@ -1108,43 +1526,23 @@ int jacobi_svd(lne_ctx* ctx, double* C, int r, double* U, double* S, int* sweeps
   } else {
     k_jacobi_init<<<64, 256, 0, ctx->stream>>>(C, r, Wc, rotated, kMaxSweeps);
   }
-  // one cluster: 16 CTAs if the device accepts that (non-portable) size
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  cfg.blockDim = dim3(256, 1, 1);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = ctx->stream;
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaErrorUnknown;
-  const bool dsmem = r <= 32 * kJacobiPer;
-  auto kern = dsmem ? k_jacobi_sweeps_dsmem : k_jacobi_sweeps;
-  for (int cl : {16, 8}) {
-    if (cl == 16 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-      cudaGetLastError();
-      continue;
-    }
-    cfg.gridDim = dim3(cl, 1, 1);
-    cfg.dynamicSmemBytes = dsmem ? sizeof(double) * (size_t)((r + cl - 1) / cl) * (r + 1) : 0;
-    attr[0].val.clusterDim.x = cl;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) != cudaSuccess || nclusters < 1) {
-      cudaGetLastError();
-      continue;
-    }
-    e = cudaLaunchKernelEx(&cfg, kern, r, Wc, rotated, max_sweeps, d_sw);
-    if (e == cudaSuccess) break;
-    cudaGetLastError();
-  }
-  if (e != cudaSuccess) {
+  // one cluster (16 CTAs if the device accepts that size), the columns in
+  // its shared memory where they fit
+  auto dsmem_bytes = [r](int cl) { return sizeof(double) * (size_t)((r + cl - 1) / cl) * (r + 2); };
+  bool ok;
+  if (r <= 32 * kJacobiPer)
+    ok = cluster_launch(ctx, k_jacobi_sweeps_dsmem, dsmem_bytes, r, Wc, rotated, max_sweeps, d_sw);
+  else
+    ok = (r <= 256 && cluster_launch(ctx, k_jacobi_sweeps_wide<8>, dsmem_bytes, r, Wc, max_sweeps, d_sw)) ||
+         (r > 256 && r <= 512 && cluster_launch(ctx, k_jacobi_sweeps_wide<16>, dsmem_bytes, r, Wc, max_sweeps, d_sw)) ||
+         cluster_launch(ctx, k_jacobi_sweeps, [](int) { return (size_t)0; }, r, Wc, rotated, max_sweeps, d_sw);
+  if (!ok) {
     dfree(ctx, Wc);
-    set_error(std::string("jacobi_svd: cluster launch failed: ") + cudaGetErrorString(e));
+    set_error("jacobi_svd: no thread-block cluster can be launched");
     return LNE_ERR_CUDA;
   }
-  k_jacobi_finish<<<1, 1024, 0, ctx->stream>>>(r, Wc, U, S);
+  k_jacobi_norms<<<(unsigned)((r + 7) / 8), 256, 0, ctx->stream>>>(r, Wc, norms);
+  k_jacobi_finish<<<(unsigned)r, 128, 0, ctx->stream>>>(r, Wc, norms, U, S);
   int h[2] = {0, 0};
   LNE_CUDA_TRY(cudaMemcpyAsync(h, d_sw, sizeof(int) * 2, cudaMemcpyDeviceToHost, ctx->stream));
   LNE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
@@ -1193,23 +1591,23 @@ int normalize_rows(lne_ctx* ctx, float* X, int64_t n, int d, int64_t ld, float e
   return LNE_OK;
 }
 
-__global__ void k_trace(const double* G, int r, double* out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < r; ++i) s += G[(int64_t)i * r + i];
-    *out = s;
-  }
+// Trace (one warp).
+__global__ void k_trace(const double* __restrict__ G, int r, double* __restrict__ out) {
+  double s = 0.0;
+  for (int i = threadIdx.x; i < r; i += 32) s += G[(int64_t)i * r + i];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (threadIdx.x == 0) *out = s;
 }
 
 // ||G - I||_F in FP64 (one block; r x r row-major).
 __global__ void k_identity_distance(const double* __restrict__ G, int r, double* __restrict__ out) {
   __shared__ double part[32];
   double s = 0.0;
-  for (int64_t t = threadIdx.x; t < (int64_t)r * r; t += blockDim.x) {
-    const int64_t i = t / r, j = t - i * r;
-    const double e = G[t] - (i == j ? 1.0 : 0.0);
-    s = fma(e, e, s);
-  }
+  for (int i = threadIdx.x >> 5; i < r; i += blockDim.x >> 5)
+    for (int j = threadIdx.x & 31; j < r; j += 32) {
+      const double e = G[(int64_t)i * r + j] - (i == j ? 1.0 : 0.0);
+      s = fma(e, e, s);
+    }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
   __syncthreads();
@@ -1224,7 +1622,7 @@ int identity_distance_host(lne_ctx* ctx, const double* G, int r, double* out) {
   double* d = nullptr;
   int rc;
   if ((rc = dalloc(ctx, (void**)&d, sizeof(double), "identity distance"))) return rc;
-  k_identity_distance<<<1, 256, 0, ctx->stream>>>(G, r, d);
+  k_identity_distance<<<1, 1024, 0, ctx->stream>>>(G, r, d);
   LNE_CUDA_TRY(cudaMemcpyAsync(out, d, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   LNE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   dfree(ctx, d);

@@ -423,15 +423,15 @@ __global__ void __launch_bounds__(256) k_chol_inv_cluster(const double* __restri
       for (int k = k0; k < k1; ++k) {
         double* ck = col + (size_t)(qs * kCholPanel + (k - k0)) * r;
         // FP64 division and square root are long instruction sequences on
-        // this part: one reciprocal square root per pivot, then the column
-        // is scaled by multiplications spread over all warps
+        // this part: one square root and one reciprocal per pivot, then
+        // the column is scaled by multiplications spread over all warps
         if (warp == 0) {  // one warp evaluates the pivot
           const double d = ck[k];
           const bool ok = d > 0.0 && isfinite(d);
-          const double rp = ok ? rsqrt(d) : 1.0;
+          const double piv = ok ? sqrt(d) : 1.0;
           if (lane == 0) {
-            prcp = rp;
-            ck[k] = ok ? d * rp : 1.0;
+            prcp = 1.0 / piv;
+            ck[k] = piv;
             if (!ok) bad = 1;
           }
         }
@@ -522,18 +522,18 @@ static size_t chol_cluster_smem(int r, int csize) {
 
 // The factorisation above for 144 < r <= kCholWideMax, whose L does not fit
 // every CTA's shared memory beside the panels: L goes to global memory, column
-// by column, with the reciprocals of its diagonal, and k_tri_inv_cols solves
-// for the columns of L^-1 over the whole device, a warp each.  At r = 256 the
-// one-block factorisation in global memory and the one-thread-per-column
-// inverse (k_cholesky, k_tri_inv_t) took 2.4 + 2.8 ms per call.
+// by column, and k_tri_inv_cols solves for the columns of L^-1 over the whole
+// device, a warp each.  The operations and their order are those of
+// k_cholesky and k_tri_inv_t (divisions by the pivot included), bit for bit:
+// what follows them in an SVD is sensitive enough for one rounding to change
+// a vector's sign.  At r = 256 those two took 2.4 + 2.8 ms per call.
 constexpr int kCholWideMax = 512;
 
 __global__ void __launch_bounds__(256) k_chol_cluster(const double* __restrict__ G, int r, double shift,
-                                                      double* __restrict__ Lc, double* __restrict__ idg,
-                                                      int* __restrict__ status) {
+                                                      double* __restrict__ Lc, int* __restrict__ status) {
   extern __shared__ double chs[];
   __shared__ int bad;
-  __shared__ double prcp;
+  __shared__ double pivot;
   const int csize = gridDim.x;
   const int rank = (int)cluster_rank();
   const int npan = (r + kCholPanel - 1) / kCholPanel;
@@ -562,18 +562,17 @@ __global__ void __launch_bounds__(256) k_chol_cluster(const double* __restrict__
         if (warp == 0) {
           const double d = ck[k];
           const bool ok = d > 0.0 && isfinite(d);
-          const double rp = ok ? rsqrt(d) : 1.0;
+          const double piv = ok ? sqrt(d) : 1.0;
           if (lane == 0) {
-            prcp = rp;
-            ck[k] = ok ? d * rp : 1.0;
-            idg[k] = rp;
+            pivot = piv;
+            ck[k] = piv;
             if (!ok) bad = 1;
           }
         }
         __syncthreads();
         if (bad) break;
-        const double rp = prcp;
-        for (int i = k + 1 + tid; i < r; i += blockDim.x) ck[i] *= rp;
+        const double piv = pivot;
+        for (int i = k + 1 + tid; i < r; i += blockDim.x) ck[i] /= piv;
         __syncthreads();
         for (int j = k + 1 + warp; j < k1; j += nw) {
           double* cj = col + (size_t)(qs * kCholPanel + (j - k0)) * r;
@@ -627,15 +626,15 @@ __global__ void __launch_bounds__(256) k_chol_cluster(const double* __restrict__
 // CTA) each: x_j = 1 / L_jj, x_i = -(sum_{k=j}^{i-1} L_ik x_k) / L_ii, the
 // sums of rows lane, lane + 32, ... in registers; row j of W = X^T.
 template <int PER>
-__global__ void __launch_bounds__(32) k_tri_inv_cols(const double* __restrict__ Lc, const double* __restrict__ idg,
-                                                     const int* __restrict__ status, int r, float* __restrict__ W) {
+__global__ void __launch_bounds__(32) k_tri_inv_cols(const double* __restrict__ Lc, const int* __restrict__ status, int r,
+                                                     float* __restrict__ W) {
   if (*status) return;
   const int lane = threadIdx.x, j = blockIdx.x;
-  double s[PER], dg[PER];  // sums, then the solution; reciprocal diagonals
+  double s[PER], dg[PER];  // sums, then the solution; L's diagonal
 #pragma unroll
   for (int m = 0; m < PER; ++m) {
     s[m] = 0.0;
-    dg[m] = 32 * m + lane < r ? idg[32 * m + lane] : 0.0;
+    dg[m] = 32 * m + lane < r ? Lc[(size_t)(32 * m + lane) * r + 32 * m + lane] : 1.0;
   }
 #pragma unroll
   for (int m = 0; m < PER; ++m) {
@@ -650,7 +649,7 @@ __global__ void __launch_bounds__(32) k_tri_inv_cols(const double* __restrict__ 
         l[b] = i > k && i < r ? lk[i] : 0.0;
       }
       // every lane has its own row's candidate; the one of row k counts
-      const double cand = k == j ? dg[m] : -s[m] * dg[m];
+      const double cand = (k == j ? 1.0 : -s[m]) / dg[m];
       const double xk = __shfl_sync(0xffffffffu, cand, k - 32 * m);
 #pragma unroll
       for (int b = m; b < PER; ++b) s[b] = fma(l[b], xk, s[b]);
@@ -665,13 +664,13 @@ __global__ void __launch_bounds__(32) k_tri_inv_cols(const double* __restrict__ 
 }
 
 // Launches `kern` (arguments args...) on one thread-block cluster of 16, else
-// 8 CTAs of 256 threads; smem(size) is its shared memory.  False if neither
+// 8 CTAs; smem(size) is its shared memory.  False if neither
 // size can be launched.
 template <class Kern, class Smem, class... Args>
-static bool cluster_launch(lne_ctx* ctx, Kern kern, Smem smem_of, Args... args) {
+static bool cluster_launch(lne_ctx* ctx, Kern kern, int threads, Smem smem_of, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
-  cfg.blockDim = dim3(256, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
   cfg.stream = ctx->stream;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   cfg.attrs = attr;
@@ -703,19 +702,18 @@ static bool cluster_launch(lne_ctx* ctx, Kern kern, Smem smem_of, Args... args) 
   return false;
 }
 
-static bool chol_wide_launch(lne_ctx* ctx, const double* G, int r, double shift, double* Lc, double* idg, int* status,
-                             float* W) {
+static bool chol_wide_launch(lne_ctx* ctx, const double* G, int r, double shift, double* Lc, int* status, float* W) {
   auto smem = [r](int cl) {
     const size_t npan = (size_t)(r + kCholPanel - 1) / kCholPanel;
     return sizeof(double) * ((npan + cl - 1) / cl + 1) * kCholPanel * (size_t)r;
   };
-  if (!cluster_launch(ctx, k_chol_cluster, smem, G, r, shift, Lc, idg, status)) return false;
+  if (!cluster_launch(ctx, k_chol_cluster, 256, smem, G, r, shift, Lc, status)) return false;
   if (r <= 160)
-    k_tri_inv_cols<5><<<(unsigned)r, 32, 0, ctx->stream>>>(Lc, idg, status, r, W);
+    k_tri_inv_cols<5><<<(unsigned)r, 32, 0, ctx->stream>>>(Lc, status, r, W);
   else if (r <= 256)
-    k_tri_inv_cols<8><<<(unsigned)r, 32, 0, ctx->stream>>>(Lc, idg, status, r, W);
+    k_tri_inv_cols<8><<<(unsigned)r, 32, 0, ctx->stream>>>(Lc, status, r, W);
   else
-    k_tri_inv_cols<16><<<(unsigned)r, 32, 0, ctx->stream>>>(Lc, idg, status, r, W);
+    k_tri_inv_cols<16><<<(unsigned)r, 32, 0, ctx->stream>>>(Lc, status, r, W);
   return true;
 }
 
@@ -729,14 +727,13 @@ int cholesky_inv(lne_ctx* ctx, double* G, int r, double shift, float* W) {
   double* X = nullptr;
   int* status = nullptr;
   int rc;
-  if ((rc = dalloc(ctx, (void**)&X, sizeof(double) * ((size_t)r * r + r) + 16, "triangular inverse"))) return rc;
-  double* idg = X + (int64_t)r * r;  // reciprocal diagonal (wide form)
-  status = (int*)(idg + r);
+  if ((rc = dalloc(ctx, (void**)&X, sizeof(double) * r * r + 16, "triangular inverse"))) return rc;
+  status = (int*)(X + (int64_t)r * r);
   const size_t csmem = sizeof(double) * ((size_t)r * r + r);
   if (r <= kCholClusterMax &&
-      cluster_launch(ctx, k_chol_inv_cluster, [r](int cl) { return chol_cluster_smem(r, cl); }, G, r, shift, W, status)) {
+      cluster_launch(ctx, k_chol_inv_cluster, 256, [r](int cl) { return chol_cluster_smem(r, cl); }, G, r, shift, W, status)) {
     // done on the cluster
-  } else if (r > kCholClusterMax && r <= kCholWideMax && chol_wide_launch(ctx, G, r, shift, X, idg, status, W)) {
+  } else if (r > kCholClusterMax && r <= kCholWideMax && chol_wide_launch(ctx, G, r, shift, X, status, W)) {
     // factored on the cluster, inverted over the device
   } else if (r <= kCholSmemMax && csmem <= ctx->smem_optin) {
     cudaFuncSetAttribute(k_chol_inv_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem);
@@ -994,251 +991,201 @@ __global__ void __launch_bounds__(256) k_jacobi_sweeps_dsmem(int r, double* __re
   if (blockIdx.x == 0 && threadIdx.x == 0) *sweeps_out = sweep < max_sweeps ? sweep + 1 : max_sweeps;
 }
 
-// The sweeps of k_jacobi_sweeps for 160 < r <= 32 PER with the columns in
-// distributed shared memory, arranged around the FP64 units, which are what
-// bounds it (two FP64 FMAs per clock and SM):
-//   - the squared norms are tracked as above, so a pair needs one dot
-//     product instead of three;
-//   - columns are kept scaled, column = scale * stored (fast rotations:
-//     x - t y, y + t x, both scales times c): two FMAs per element pair
-//     instead of four operations; the scales are folded in every sweep;
-//   - the rotations of a CTA's pairs are evaluated together by one warp, a
-//     pair per lane, instead of 32 times over by each pair's warp.
-// The rotations are those of k_jacobi_sweeps to FP64 rounding (same pairs,
-// same order, smaller angle), so the columns come out with the same signs.
-// At r = 256 the global-memory form took 28 ms.
-constexpr int kJacobiWideWarps = 8;
+// The sweeps of k_jacobi_sweeps for 160 < r <= 32 PER, a CTA of four warps per
+// pair of the current step over the whole device instead of eight pairs to an
+// SM of one cluster.  What bounds a step is FP64: a warp instruction takes 64
+// cycles of its quarter of the SM (69 measured, dependent or not; a division
+// or a root 670), so the pair's three dot products go to three warps, the
+// columns' rotation to four, and only the rotation's own divisions and roots
+// are one chain.  The columns lie in global memory (L2); a column's version
+// counts the steps it has been through, and a pair starts when both of its
+// columns have the version of its step, so nothing waits for a whole step but
+// the end of a sweep.  Same pairs, same order and the same operations as
+// k_jacobi_sweeps: the columns are bit for bit the same, signs included (the
+// path is sensitive: tangents good to one unit in the last place changed
+// signs).  At r = 256, 13 sweeps: 28 ms by the cluster form, 25 with a warp
+// per pair, 18.5 so.
+//
+// Launched cooperatively (the CTAs wait on one another).  Every wait gives up
+// after kFlowSpins polls, raises *abort and lets the others leave too.
+constexpr int kFlowSpins = 1 << 20;
+constexpr int kFlowMax = 512;
 
-// 1 / sqrt(x) for x in [2^-4, 2^4]: FP32 seed, two Newton steps.
-__device__ __forceinline__ double rsqrt_newton(double x) {
-  double y = (double)rsqrtf((float)x);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) y = y * fma(-0.5 * x * y, y, 1.5);
-  return y;
+__device__ __forceinline__ int ld_relaxed(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
 }
-
+__device__ __forceinline__ void st_relaxed(int* p, int v) {
+  asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 template <int PER>
-__global__ void __launch_bounds__(kJacobiWideWarps * 32) k_jacobi_sweeps_wide(int r, double* __restrict__ Wc,
-                                                                              int max_sweeps,
-                                                                              int* __restrict__ sweeps_out) {
-  extern __shared__ double jcols[];  // nslots columns (slot s: column s * csize + rank), then nslots {norm, scale}
-  __shared__ int rot_flag[kJacobiMaxSweeps];
-  __shared__ double part[kJacobiWideWarps][33];  // a pair's partial dot products
-  __shared__ double pa[kJacobiWideWarps][4];     // {norm p, scale p, norm q, scale q}
-  // {t q/p, t p/q, norm p, norm q, scale p, scale q, stored factors of p, q}
-  __shared__ double rot[kJacobiWideWarps][8];
-  __shared__ int act[kJacobiWideWarps];
-  __shared__ unsigned long long cmax;
-  __shared__ double csum;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int k = tid; k < kJacobiMaxSweeps; k += blockDim.x) rot_flag[k] = 0;
-  const int csize = gridDim.x;
-  const int rank = (int)cluster_rank();
-  const int cshift = __ffs(csize) - 1;  // csize is a power of two
-  const int nslots = (r + csize - 1) / csize;
-  double* ns = jcols + (size_t)nslots * r;  // {norm, scale} of slot s at 2 s
-  if (tid == 0) cmax = 0;
-  __syncthreads();
-  unsigned long long mx = 0;  // largest |entry|, as bits
-  for (int s = warp; s < nslots; s += kJacobiWideWarps) {
-    const int c = s * csize + rank;
-    for (int i = lane; i < r; i += 32) {
-      const double v = c < r ? Wc[(size_t)c * r + i] : 0.0;
-      jcols[(size_t)s * r + i] = v;
-      mx = max(mx, (unsigned long long)__double_as_longlong(fabs(v)));
-    }
-  }
-  atomicMax(&cmax, mx);
-  cluster_barrier();
-  const uint32_t base = (uint32_t)__cvta_generic_to_shared(jcols);
-  const uint32_t nbase = (uint32_t)__cvta_generic_to_shared(ns);
-  {
-    const uint32_t ma = (uint32_t)__cvta_generic_to_shared(&cmax);
-    for (int c = 0; c < csize; ++c) {
-      const unsigned long long v = (unsigned long long)__double_as_longlong(dsmem_ld(dsmem_map(ma, (uint32_t)c)));
-      mx = c == 0 ? v : max(mx, v);
-    }
-  }
-  // the sweeps run on the matrix scaled by a power of two to entries below 2
-  const int ex = (int)(mx >> 52);
-  const bool scaled = ex >= 1 && ex <= 2045;
-  const double down = scaled ? __longlong_as_double((long long)(2046 - ex) << 52) : 1.0;
-  const double up = scaled ? __longlong_as_double((long long)ex << 52) : 1.0;
-  for (int s = tid; s < nslots; s += blockDim.x) ns[2 * s + 1] = down;
-  const int rp = (r + 1) & ~1;
+__global__ void __launch_bounds__(128) k_jacobi_sweeps_flow(int r, double* __restrict__ Wc, int* __restrict__ rotated,
+                                                            int* __restrict__ version, int* __restrict__ arrived,
+                                                            int* __restrict__ abort, int max_sweeps,
+                                                            int* __restrict__ sweeps_out) {
+  __shared__ double sum[3], root[2], rotn[2];
+  __shared__ int state;  // of the step: 0 no rotation, 1 rotation, 2 given up; at a sweep's end: 2 go on
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pk = blockIdx.x;
+  const int rp = (r + 1) & ~1;  // even number of players (index r is a dummy when r is odd)
   const int m = rp - 1;
-  const double tol2 = fmax(1e-30, 4.930380657631324e-32 * r);  // max(1e-15, sqrt(r) 2^-52)^2
-  double tiny = 0.0;
+  // below sqrt(r) eps a rotation only chases the rounding of the dot product
+  const double tol = fmax(1e-15, 2.220446049250313e-16 * sqrt((double)r));
+  bool failed = false;  // the same for the whole block
   int sweep = 0;
   for (; sweep < max_sweeps; ++sweep) {
-    // fold the scales in; fresh squared norms
-    __syncthreads();
-    for (int s = warp; s < nslots; s += kJacobiWideWarps) {
-      const double sc = ns[2 * s + 1];
-      double a = 0.0;
-      double* col = jcols + (size_t)s * r;
-      for (int i = lane; i < r; i += 32) {
-        const double v = sc * col[i];
-        col[i] = v;
-        a = fma(v, v, a);
-      }
-      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (lane == 0) {
-        ns[2 * s] = a;
-        ns[2 * s + 1] = 1.0;
-      }
-    }
-    __syncthreads();
-    if (sweep == 0) {
-      // A sweep leaves rounding noise of about eps |C|_F in a column (eps
-      // |x| of each partner x).  A column below 8 eps |C|_F is that noise:
-      // it is not rotated, or noise would rotate forever on a rank-deficient
-      // matrix.
-      if (tid == 0) {
-        double t = 0.0;
-        for (int s = 0; s < nslots; ++s) t += ns[2 * s];
-        csum = t;
-      }
-      cluster_barrier();
-      double fro2 = 0.0;
-      const uint32_t ca = (uint32_t)__cvta_generic_to_shared(&csum);
-      for (int c = 0; c < csize; ++c) fro2 += dsmem_ld(dsmem_map(ca, (uint32_t)c));
-      tiny = fro2 * 3.1554436208840472e-30;  // fro2 (8 2^-52)^2
-    } else {
-      cluster_barrier();
-    }
+    bool any = false;
     for (int s = 0; s < m; ++s) {
-      for (int pk0 = 0; pk0 < rp / 2; pk0 += kJacobiWideWarps * csize) {  // the same for the whole cluster
-        // the round-robin pairs of step s: (s + pk, s - pk) mod m, and (m, s)
-        const int pk = pk0 + warp * csize + rank;
-        int p = 0, q = 0;
-        bool live = pk < rp / 2;
-        if (live) {
-          if (pk == 0) {
-            p = m;
-            q = s;
-          } else {
-            p = s + pk;
-            if (p >= m) p -= m;
-            q = s - pk;
-            if (q < 0) q += m;
-          }
-          if (p >= r || q >= r) live = false;
-          if (p > q) { const int t = p; p = q; q = t; }
-        }
-        const uint32_t pc = (uint32_t)(p & (csize - 1)), qc = (uint32_t)(q & (csize - 1));
-        const uint32_t ap = dsmem_map(base + (uint32_t)((p >> cshift) * r) * 8u, pc);
-        const uint32_t aq = dsmem_map(base + (uint32_t)((q >> cshift) * r) * 8u, qc);
-        const uint32_t np_ = dsmem_map(nbase + (uint32_t)(p >> cshift) * 16u, pc);
-        const uint32_t nq_ = dsmem_map(nbase + (uint32_t)(q >> cshift) * 16u, qc);
-        double x[PER], y[PER];
-        if (live) {
-          if (lane < 4) pa[warp][lane] = dsmem_ld((lane < 2 ? np_ : nq_) + 8u * (lane & 1));
-#pragma unroll
-          for (int k = 0; k < PER; ++k) {
-            const int i = lane + 32 * k;
-            x[k] = i < r ? dsmem_ld(ap + 8u * i) : 0.0;
-            y[k] = i < r ? dsmem_ld(aq + 8u * i) : 0.0;
-          }
-          double g = 0.0;
-#pragma unroll
-          for (int k = 0; k < PER; ++k) g = fma(x[k], y[k], g);
-          part[warp][lane] = g;
-        }
-        if (lane == 0) act[warp] = live;
-        __syncthreads();
-        if (warp == 0) {
-          // four lanes add a pair's partial products, then one evaluates
-          // its rotation: t = tan of the smaller angle that makes the
-          // columns orthogonal, from d = b - a and h = 2 g scaled to [1, 2)
-          const int w = lane >> 2;
-          double g = 0.0;
-          const bool on = act[w] != 0;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) g += part[w][(lane & 3) + 4 * k];
-          g += __shfl_xor_sync(0xffffffffu, g, 1);
-          g += __shfl_xor_sync(0xffffffffu, g, 2);
-          if ((lane & 3) == 0) {
-            const double a = pa[w][0], dp = pa[w][1], b = pa[w][2], dq = pa[w][3];
-            g *= dp * dq;
-            bool go = on && g != 0.0 && a > tiny && b > tiny && g * g > tol2 * (a * b);
-            if (go) {
-              double d = b - a, h = 2.0 * g;
-              const double big = fmax(fabs(d), fabs(h));
-              // 2^-exponent of the larger
-              const double sc = __longlong_as_double((2046LL - ((__double_as_longlong(big) >> 52) & 0x7ff)) << 52);
-              d *= sc;
-              h *= sc;
-              const double root2 = fma(d, d, h * h);
-              const double ir = rsqrt_newton(root2);           // 1 / sqrt(d^2 + h^2)
-              const double c2 = fma(0.5 * fabs(d), ir, 0.5);   // cos^2, in [1/2, 1]
-              const double ic = rsqrt_newton(c2);              // 1 / cos
-              const double c = c2 * ic;
-              const double sn = 0.5 * fabs(h) * ir * ic * (d * h >= 0.0 ? 1.0 : -1.0);
-              const double t = sn * ic;
-              // scales dq / dp and its inverse, by FP32 seeds and Newton
-              double ip = (double)(1.0f / (float)dp), iq = (double)(1.0f / (float)dq);
-#pragma unroll
-              for (int i = 0; i < 2; ++i) {
-                ip = ip * fma(-dp, ip, 2.0);
-                iq = iq * fma(-dq, iq, 2.0);
-              }
-              const double cc = c * c, ss = sn * sn, cs2 = 2.0 * c * sn * g;
-              rot[w][0] = t * dq * ip;
-              rot[w][1] = t * dp * iq;
-              rot[w][2] = fmax(fma(cc, a, fma(ss, b, -cs2)), 0.0);
-              rot[w][3] = fmax(fma(ss, a, fma(cc, b, cs2)), 0.0);
-              // a scale that has shrunk far is raised by 2^30 (exact)
-              const bool up = dp * c < 9.3132257461547852e-10, uq = dq * c < 9.3132257461547852e-10;
-              rot[w][4] = dp * c * (up ? 1073741824.0 : 1.0);
-              rot[w][5] = dq * c * (uq ? 1073741824.0 : 1.0);
-              rot[w][6] = up ? 9.3132257461547852e-10 : 1.0;
-              rot[w][7] = uq ? 9.3132257461547852e-10 : 1.0;
-              rot_flag[sweep] = 1;
-            }
-            act[w] = go;
-          }
-        }
-        __syncthreads();
-        if (act[warp]) {
-          const double t1 = rot[warp][0], t2 = rot[warp][1], f1 = rot[warp][6], f2 = rot[warp][7];
-          const bool plain = f1 == 1.0 && f2 == 1.0;
-#pragma unroll
-          for (int k = 0; k < PER; ++k) {
-            const int i = lane + 32 * k;
-            if (i < r) {
-              double u = fma(-t1, y[k], x[k]), v = fma(t2, x[k], y[k]);
-              if (!plain) {
-                u *= f1;
-                v *= f2;
-              }
-              dsmem_st(ap + 8u * i, u);
-              dsmem_st(aq + 8u * i, v);
-            }
-          }
-          if (lane < 4) {
-            // {norm, scale} of p, then of q
-            const double v = rot[warp][lane < 2 ? 2 + 2 * lane : 3 + 2 * (lane - 2)];
-            dsmem_st((lane < 2 ? np_ : nq_) + 8u * (lane & 1), v);
-          }
-        }
-        __syncthreads();  // act, part and rot are rewritten
+      int p, q;
+      if (pk == 0) {
+        p = rp - 1;
+        q = s;
+      } else {
+        p = s + pk;
+        if (p >= m) p -= m;
+        q = s - pk;
+        if (q < 0) q += m;
       }
-      cluster_barrier();
+      if (p > q) { const int t = p; p = q; q = t; }
+      const bool two = q < r;  // else p's column sits this step out
+      const int step = sweep * m + s;
+      if (warp == 0) {
+        // lanes 0 and 1 watch a column each
+        const bool watch = lane == 0 || (lane == 1 && two);
+        const int mine = lane == 0 ? p : q;
+        bool ok = true;
+        for (int tries = 0;; ++tries) {
+          if (__all_sync(0xffffffffu, !watch || ld_relaxed(version + mine) == step)) break;
+          if (tries >= kFlowSpins || ((tries & 255) == 255 && __any_sync(0xffffffffu, ld_relaxed(abort) != 0))) {
+            ok = false;
+            break;
+          }
+        }
+        __threadfence();  // the columns' elements are read after their versions
+        if (lane == 0) {
+          if (!ok) atomicExch(abort, 1);
+          state = ok ? 0 : 2;
+        }
+      }
+      __syncthreads();
+      if (state == 2) {
+        failed = true;
+        break;
+      }
+      if (two) {
+        double* wp = Wc + (size_t)p * r;
+        double* wq = Wc + (size_t)q * r;
+        double xs[PER], ys[PER];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+          const int i = lane + 32 * k;
+          xs[k] = i < r ? __ldcg(wp + i) : 0.0;
+          ys[k] = i < r ? __ldcg(wq + i) : 0.0;
+        }
+        // x.x, y.y and x.y by warps 0, 1 and 2
+        double d = 0.0;
+        if (warp < 3) {
+#pragma unroll
+          for (int k = 0; k < PER; ++k)
+            if (lane + 32 * k < r) d = fma(warp == 1 ? ys[k] : xs[k], warp == 0 ? xs[k] : ys[k], d);
+          for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+          if (lane == 0) sum[warp] = d;
+        }
+        __syncthreads();
+        // the limit's roots (warps 0 and 1) beside the rotation (warp 2)
+        double c = 1.0, sn = 0.0, g = 0.0;
+        if (warp < 2) {
+          const double rt = sqrt(d);
+          if (lane == 0) root[warp] = rt;
+        } else if (warp == 2) {
+          const double a = sum[0], b = sum[1];
+          g = d;
+          const double zeta = (b - a) / (2.0 * g);
+          const double t = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+          c = 1.0 / sqrt(1.0 + t * t);
+          sn = c * t;
+          if (lane == 0) {
+            rotn[0] = c;
+            rotn[1] = sn;
+          }
+        }
+        __syncthreads();
+        g = sum[2];
+        const bool rot = fabs(g) > tol * root[0] * root[1] && g != 0.0;
+        any = any || rot;
+        if (rot) {
+          c = rotn[0];
+          sn = rotn[1];
+          // each warp a quarter of the elements
+#pragma unroll
+          for (int k = 0; k < PER; ++k) {
+            const int i = lane + 32 * k;
+            if ((k & 3) == warp && i < r) {
+              const double x = xs[k], y = ys[k];
+              __stcg(wp + i, c * x - sn * y);
+              __stcg(wq + i, sn * x + c * y);
+            }
+          }
+          __threadfence();
+        }
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) st_relaxed(version + p, step + 1);
+      if (threadIdx.x == 1 && two) st_relaxed(version + q, step + 1);
     }
-    int any = 0;
-    const uint32_t fa = (uint32_t)__cvta_generic_to_shared(&rot_flag[sweep]);
-    for (int c = 0; c < csize; ++c) any |= dsmem_ld32(dsmem_map(fa, (uint32_t)c));
-    if (!any) break;
+    // the end of the sweep: did any pair rotate?
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int go = 0;
+      if (any) atomicExch(rotated + sweep, 1);
+      __threadfence();
+      atomicAdd(arrived, 1);
+      if (!failed) {
+        const int all = (sweep + 1) * (int)gridDim.x;
+        int k = 0;
+        while (ld_relaxed(arrived) < all && k < kFlowSpins && !((k & 255) == 255 && ld_relaxed(abort))) ++k;
+        __threadfence();
+        if (ld_relaxed(arrived) >= all)
+          go = ld_relaxed(rotated + sweep) ? 2 : 1;
+        else
+          atomicExch(abort, 1);
+      }
+      state = go;
+    }
+    __syncthreads();
+    const int go = state;
+    __syncthreads();
+    if (go != 2) break;  // converged, or given up
   }
-  cluster_barrier();  // no CTA leaves while another may still read its flags
-  for (int s = warp; s < nslots; s += kJacobiWideWarps) {
-    const int c = s * csize + rank;
-    const double sc = up * ns[2 * s + 1];
-    if (c < r)
-      for (int i = lane; i < r; i += 32) Wc[(size_t)c * r + i] = sc * jcols[(size_t)s * r + i];
+  if (pk == 0 && threadIdx.x == 0) *sweeps_out = sweep < max_sweeps ? sweep + 1 : max_sweeps;
+}
+
+// Launches the dataflow sweeps on the columns Wc; false if they cannot run
+// here (the caller takes the cluster form).  `words`: kFlowMax + 2 ints, zero.
+template <int PER>
+static bool jacobi_flow_launch(lne_ctx* ctx, int r, double* Wc, int* rotated, int* words, int max_sweeps, int* d_sw) {
+  int per_sm = 0, coop = 0;
+  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device) != cudaSuccess || !coop ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_jacobi_sweeps_flow<PER>, 128, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
   }
-  if (blockIdx.x == 0 && tid == 0) *sweeps_out = sweep < max_sweeps ? sweep + 1 : max_sweeps;
+  const int pairs = ((r + 1) & ~1) / 2;
+  if (pairs > per_sm * ctx->num_sms) return false;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3((unsigned)pairs, 1, 1);
+  cfg.blockDim = dim3(128, 1, 1);
+  cfg.stream = ctx->stream;
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, k_jacobi_sweeps_flow<PER>, r, Wc, rotated, words + 2, words, words + 1, max_sweeps,
+                         d_sw) == cudaSuccess)
+    return true;
+  cudaGetLastError();
+  return false;
 }
 
 // FP32 preconditioning of the FP64 sweeps (r <= 32 * kJacobiPer, one CTA):
@@ -1484,7 +1431,9 @@ static bool jacobi_precond_applies(lne_ctx* ctx, int r) {
   return r <= 32 * kJacobi32Vec && jacobi_precond_smem(r) + 1024 <= ctx->smem_optin;
 }
 
-int jacobi_svd_launches(lne_ctx* ctx, int r) { return jacobi_precond_applies(ctx, r) ? 8 : 4; }
+int jacobi_svd_launches(lne_ctx* ctx, int r) {
+  return jacobi_precond_applies(ctx, r) ? 8 : 4;
+}
 
 int jacobi_svd(lne_ctx* ctx, double* C, int r, double* U, double* S, int* sweeps_out, int* sweeps32_out,
                int fp64_sweep_cap) {
@@ -1500,7 +1449,7 @@ int jacobi_svd(lne_ctx* ctx, double* C, int r, double* U, double* S, int* sweeps
   double* Wc = nullptr;
   int rc;
   // Wc, then (preconditioned) V, P, M, V1, P1 (FP64 r x r each)
-  const size_t bytes = sizeof(double) * (rr * (pre ? 6 : 1) + r) + sizeof(int) * (kMaxSweeps + 4);
+  const size_t bytes = sizeof(double) * (rr * (pre ? 6 : 1) + r) + sizeof(int) * (kMaxSweeps + 4 + 2 + kFlowMax);
   if ((rc = dalloc(ctx, (void**)&Wc, bytes, "jacobi work"))) return rc;
   double* Vd = Wc + rr;
   double* Pc = Vd + rr;
@@ -1510,7 +1459,8 @@ int jacobi_svd(lne_ctx* ctx, double* C, int r, double* U, double* S, int* sweeps
   double* norms = Wc + rr * (pre ? 6 : 1);
   int* rotated = (int*)(norms + r);
   int* d_sw = rotated + kMaxSweeps;  // [0]: FP64 sweeps, [1]: FP32 sweeps
-  LNE_CUDA_TRY(cudaMemsetAsync(d_sw + 1, 0, sizeof(int), ctx->stream));
+  int* words = d_sw + 4;              // arrivals, abort, column versions (dataflow form)
+  LNE_CUDA_TRY(cudaMemsetAsync(d_sw, 0, sizeof(int) * (4 + 2 + kFlowMax), ctx->stream));
   if (pre) {
     // FP32 sweeps give V; two Newton-Schulz steps make it orthogonal to
     // FP64 precision (V^T V - I: about 1e-5 -> 1e-10 -> 1e-16); W = C V
@@ -1531,11 +1481,11 @@ int jacobi_svd(lne_ctx* ctx, double* C, int r, double* U, double* S, int* sweeps
   auto dsmem_bytes = [r](int cl) { return sizeof(double) * (size_t)((r + cl - 1) / cl) * (r + 2); };
   bool ok;
   if (r <= 32 * kJacobiPer)
-    ok = cluster_launch(ctx, k_jacobi_sweeps_dsmem, dsmem_bytes, r, Wc, rotated, max_sweeps, d_sw);
+    ok = cluster_launch(ctx, k_jacobi_sweeps_dsmem, 256, dsmem_bytes, r, Wc, rotated, max_sweeps, d_sw);
   else
-    ok = (r <= 256 && cluster_launch(ctx, k_jacobi_sweeps_wide<8>, dsmem_bytes, r, Wc, max_sweeps, d_sw)) ||
-         (r > 256 && r <= 512 && cluster_launch(ctx, k_jacobi_sweeps_wide<16>, dsmem_bytes, r, Wc, max_sweeps, d_sw)) ||
-         cluster_launch(ctx, k_jacobi_sweeps, [](int) { return (size_t)0; }, r, Wc, rotated, max_sweeps, d_sw);
+    ok = (r <= 256 && jacobi_flow_launch<8>(ctx, r, Wc, rotated, words, max_sweeps, d_sw)) ||
+         (r > 256 && r <= kFlowMax && jacobi_flow_launch<16>(ctx, r, Wc, rotated, words, max_sweeps, d_sw)) ||
+         cluster_launch(ctx, k_jacobi_sweeps, 256, [](int) { return (size_t)0; }, r, Wc, rotated, max_sweeps, d_sw);
   if (!ok) {
     dfree(ctx, Wc);
     set_error("jacobi_svd: no thread-block cluster can be launched");
@@ -1543,11 +1493,16 @@ int jacobi_svd(lne_ctx* ctx, double* C, int r, double* U, double* S, int* sweeps
   }
   k_jacobi_norms<<<(unsigned)((r + 7) / 8), 256, 0, ctx->stream>>>(r, Wc, norms);
   k_jacobi_finish<<<(unsigned)r, 128, 0, ctx->stream>>>(r, Wc, norms, U, S);
-  int h[2] = {0, 0};
+  int h[2] = {0, 0}, gave_up = 0;
   LNE_CUDA_TRY(cudaMemcpyAsync(h, d_sw, sizeof(int) * 2, cudaMemcpyDeviceToHost, ctx->stream));
+  LNE_CUDA_TRY(cudaMemcpyAsync(&gave_up, words + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   LNE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   dfree(ctx, Wc);
   LNE_CUDA_TRY(cudaGetLastError());
+  if (gave_up) {
+    set_error("jacobi_svd: a wait of the sweeps timed out");
+    return LNE_ERR_CUDA;
+  }
   if (sweeps_out) *sweeps_out = h[0];
   if (sweeps32_out) *sweeps32_out = h[1];
   return LNE_OK;
@@ -1591,11 +1546,14 @@ int normalize_rows(lne_ctx* ctx, float* X, int64_t n, int d, int64_t ld, float e
   return LNE_OK;
 }
 
-// Trace (one warp).
+// Trace, added in index order (one warp fetches, one lane adds).
 __global__ void k_trace(const double* __restrict__ G, int r, double* __restrict__ out) {
   double s = 0.0;
-  for (int i = threadIdx.x; i < r; i += 32) s += G[(int64_t)i * r + i];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  for (int i0 = 0; i0 < r; i0 += 32) {
+    const int i = i0 + (int)threadIdx.x;
+    const double v = i < r ? G[(int64_t)i * r + i] : 0.0;
+    for (int k = 0; k < 32 && i0 + k < r; ++k) s += __shfl_sync(0xffffffffu, v, k);
+  }
   if (threadIdx.x == 0) *out = s;
 }
 

@@ -48,6 +48,7 @@ struct __align__(16) SpmmItem {
 };
 struct SpmmPlan {
   int64_t n_items = 0, n_big = 0, n_heavy = 0;
+  int64_t nnz = 0;
   int warp_max = kChunkNnz;   // a power of two in [kWarpNnzMin, kChunkNnz]
   SpmmItem* items = nullptr;  // [n_items]
   uint2* span = nullptr;      // [n_big] {first item of its row, items of its row}

@@ -72,6 +72,7 @@ static int build_plan(lne_ctx* ctx, Rows R, int64_t n, int64_t nnz, SpmmPlan& pl
   LNE_CUDA_TRY(cudaMemcpyAsync(&tot[0], pos_heavy + n, 8, cudaMemcpyDeviceToHost, st));
   LNE_CUDA_TRY(cudaMemcpyAsync(&tot[1], pos_light + n, 8, cudaMemcpyDeviceToHost, st));
   LNE_CUDA_TRY(cudaStreamSynchronize(st));
+  plan.nnz = nnz;
   plan.n_big = tot[0] >> 32;
   plan.n_heavy = plan.n_big + (tot[0] & 0xffffffffLL);
   plan.n_items = plan.n_heavy + tot[1];

@@ -117,8 +117,12 @@ static int spmm_run(lne_ctx* ctx, const SpmmPlan& plan, const uint32_t* col, con
   const int64_t c_total = (d + E - 1) / E;
   int rc;
   int nl = 0;
-  // graphs, and matrices too small for a warp to take every row alone
-  const bool bal = !VAL || plan.warp_max < kChunkNnz;
+  // graphs, and matrices so small that a warp walking a 2048-entry row (some
+  // 250 us) would outlast the rest: below 4 GB of gathers (about 0.4 ms).
+  // Above, the 16-byte gathers of a warp per row take fewer instructions: a
+  // 10,312-row matrix with 33M entries and 256 FP32 columns, 34 GB, takes
+  // 1.4 ms that way and 2.3 ms balanced.
+  const bool bal = !VAL || (plan.warp_max < kChunkNnz && (double)plan.nnz * d * sizeof(XT) < 4e9);
   SpmmWork own;
   if (!work) {
     if ((rc = spmm_work_alloc(ctx, plan, spmm_work_width<XT>(d), &own))) return rc;

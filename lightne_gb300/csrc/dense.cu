@@ -1466,7 +1466,9 @@ int jacobi_svd(lne_ctx* ctx, double* C, int r, double* U, double* S, int* sweeps
     // FP64 precision (V^T V - I: about 1e-5 -> 1e-10 -> 1e-16); W = C V
     const size_t psmem = jacobi_precond_smem(r);
     cudaFuncSetAttribute(k_jacobi_precond32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem);
-    k_jacobi_precond32<<<1, 1024, psmem, ctx->stream>>>(C, r, Vd, d_sw + 1);
+    // four pairs per warp; warps without a pair would only meet the barriers
+    const int pwarps = ((r + 1) / 2 + 3) / 4;
+    k_jacobi_precond32<<<1, 32 * pwarps, psmem, ctx->stream>>>(C, r, Vd, d_sw + 1);
     const int nt = (r + 15) / 16;
     const size_t msmem = sizeof(double) * 32 * (size_t)(r + 1);
     k_jacobi_pm<<<2 * nt * nt, 256, msmem, ctx->stream>>>(C, Vd, r, Pc, M);              // M = V^T V, P = C V

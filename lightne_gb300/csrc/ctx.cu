@@ -43,6 +43,7 @@ void dfree(lne_ctx* ctx, void* p) {
 static constexpr int kScanThreads = 1024;
 static constexpr int kScanItems = 4;
 static constexpr int kScanTile = kScanThreads * kScanItems;
+static constexpr int64_t kScanSmall = 4 * kScanTile;  // one block scans these
 
 __device__ __forceinline__ long long warp_incl_scan(long long v) {
   const int lane = threadIdx.x & 31;
@@ -117,6 +118,34 @@ __global__ void k_scan_add(int64_t* out, int64_t n, const int64_t* tile_tot) {
     if (base + i < n) out[base + i] += add;
 }
 
+// The whole scan by one block, tile after tile, for a few tiles: the three
+// launches above are 10 us however small n is.
+__global__ void __launch_bounds__(kScanThreads) k_scan_small(const int64_t* __restrict__ in, int64_t* __restrict__ out,
+                                                             int64_t n) {
+  long long carry = 0;
+  for (int64_t t0 = 0; t0 < n; t0 += kScanTile) {
+    const int64_t base = t0 + (int64_t)threadIdx.x * kScanItems;
+    long long v[kScanItems];
+    long long s = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+      v[i] = base + i < n ? in[base + i] : 0;
+      s += v[i];
+    }
+    long long tot;
+    long long pre = carry + block_excl_scan(s, &tot);
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+      if (base + i < n) out[base + i] = pre;
+      pre += v[i];
+    }
+    carry += tot;
+  }
+  if (threadIdx.x == 0) out[n] = carry;
+}
+
+int scan_launches(int64_t n) { return n <= kScanSmall ? 1 : 3; }
+
 size_t scan_tmp_bytes(int64_t n) {
   int64_t ntiles = (n + kScanTile - 1) / kScanTile;
   return (size_t)(ntiles + 1) * sizeof(int64_t);
@@ -124,6 +153,10 @@ size_t scan_tmp_bytes(int64_t n) {
 
 void scan_exclusive_i64(const int64_t* counts, int64_t* out, int64_t n, void* tmp,
                         cudaStream_t stream) {
+  if (n <= kScanSmall) {
+    k_scan_small<<<1, kScanThreads, 0, stream>>>(counts, out, n);
+    return;
+  }
   int64_t ntiles = (n + kScanTile - 1) / kScanTile;
   int64_t* tile_tot = (int64_t*)tmp;
   if (ntiles > 0) k_scan_tiles<<<(unsigned)ntiles, kScanThreads, 0, stream>>>(counts, out, n, tile_tot);

@@ -163,12 +163,13 @@ void dfree(lne_ctx* ctx, void* p);
 // Exclusive scan of int64 counts[0..n) into out[0..n] (out[n] = total),
 // on ctx->stream.  tmp must hold scan_tmp_bytes(n).
 size_t scan_tmp_bytes(int64_t n);
+int scan_launches(int64_t n);  // kernels of one scan
 void scan_exclusive_i64(const int64_t* counts, int64_t* out, int64_t n, void* tmp,
                         cudaStream_t stream);
 
 // SpMM work lists (built on ctx->stream; synchronises once): a count
-// kernel, two exclusive scans of three launches each, a fill kernel.
-static constexpr int kPlanLaunches = 8;
+// kernel, two exclusive scans, a fill kernel.
+inline int plan_launches(int64_t rows) { return 2 + 2 * scan_launches(rows); }
 int build_plan_csr(lne_ctx* ctx, lne_csr* c);
 int build_plan_graph(lne_ctx* ctx, lne_graph* g);
 void free_plan(SpmmPlan& p);

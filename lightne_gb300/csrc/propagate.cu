@@ -964,7 +964,7 @@ extern "C" int lne_propagate(lne_ctx* ctx, const lne_graph* g, const lne_propaga
                 "lne_propagate: bad precision");
   LNE_CUDA_TRY(cudaSetDevice(ctx->device));
   lne_graph* gm = const_cast<lne_graph*>(g);
-  if (!gm->plan_ready) ctx->launch_count += kPlanLaunches;
+  if (!gm->plan_ready) ctx->launch_count += plan_launches(gm->n);
   int rc = build_plan_graph(ctx, gm);
   if (rc) return rc;
   if (p->precision == LNE_PREC_BF16) return propagate_impl<__nv_bfloat16>(ctx, gm, p, d_a, d_y, d_a_out, stats);
@@ -982,7 +982,7 @@ extern "C" int lne_propagate_adjoint(lne_ctx* ctx, const lne_graph* g, const lne
                 "lne_propagate_adjoint: bad precision");
   LNE_CUDA_TRY(cudaSetDevice(ctx->device));
   lne_graph* gm = const_cast<lne_graph*>(g);
-  if (!gm->plan_ready) ctx->launch_count += kPlanLaunches;
+  if (!gm->plan_ready) ctx->launch_count += plan_launches(gm->n);
   int rc = build_plan_graph(ctx, gm);
   if (rc) return rc;
   if (p->precision == LNE_PREC_BF16)

@@ -98,6 +98,46 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const unsigned lon
   for (int d = lane; d < bins; d += 32) hist[(int64_t)d * ntiles + tile] = my[d];
 }
 
+// The same with a block per tile, for inputs whose tiles do not fill the
+// device as warps: a warp's 64 dependent rounds took 19 us however few tiles
+// there were.
+template <int MODE>
+__global__ void __launch_bounds__(kRadixThreads) k_radix_hist_block(const unsigned long long* __restrict__ keys,
+                                                                     int64_t count, int shift, int dbits,
+                                                                     int64_t ntiles, int64_t* __restrict__ hist,
+                                                                     unsigned long long hmask) {
+  const int bins = 1 << dbits;
+  __shared__ unsigned int h[kMaxBins];
+  const int64_t base = (int64_t)blockIdx.x * kRadixTile;
+  unsigned long long key[kRadixItems];
+#pragma unroll
+  for (int r = 0; r < kRadixItems; ++r) {
+    const int64_t i = base + r * kRadixThreads + threadIdx.x;
+    key[r] = i < count ? keys[i] : 0ULL;
+  }
+  if (threadIdx.x < bins) h[threadIdx.x] = 0;
+  __syncthreads();
+  const unsigned long long mask = (unsigned long long)(bins - 1);
+#pragma unroll
+  for (int r = 0; r < kRadixItems; ++r)
+    if (base + r * kRadixThreads + threadIdx.x < count) atomicAdd(&h[digit_of<MODE>(key[r], shift, mask, hmask)], 1u);
+  __syncthreads();
+  if (threadIdx.x < bins) hist[(int64_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
+}
+
+// Counts the digits of every tile: a warp per tile once those fill half the
+// device's 64 warps per SM, else a block per tile.
+template <int MODE>
+static void radix_hist(lne_ctx* ctx, const unsigned long long* keys, int64_t count, int shift, int dbits, int64_t ntiles,
+                       int64_t* hist, unsigned long long hmask) {
+  if (ntiles < (int64_t)ctx->num_sms * 32)
+    k_radix_hist_block<MODE>
+        <<<(unsigned)ntiles, kRadixThreads, 0, ctx->stream>>>(keys, count, shift, dbits, ntiles, hist, hmask);
+  else
+    k_radix_hist<MODE>
+        <<<hist_grid(ntiles), kRadixThreads, 0, ctx->stream>>>(keys, count, shift, dbits, ntiles, hist, hmask);
+}
+
 // Exclusive scan of v over the block's threads (kRadixThreads); returns the
 // prefix of this thread.  `warp_tot` is kRadixWarps words of shared memory.
 __device__ __forceinline__ unsigned block_excl_scan_u32(unsigned v, unsigned* warp_tot) {
@@ -306,7 +346,7 @@ int radix_sort_pairs_to_csr(lne_ctx* ctx, unsigned long long* keys, uint32_t* va
   uint32_t *src_v = vals, *dst_v = vals_tmp;
   for (int p = 0; p < passes; ++p) {
     const int shift = p * dbits;
-    k_radix_hist<kDigitKey><<<hist_grid(ntiles), kRadixThreads, 0, st>>>(src_k, count, shift, dbits, ntiles, hist, 0);
+    radix_hist<kDigitKey>(ctx, src_k, count, shift, dbits, ntiles, hist, 0);
     scan_exclusive_i64(hist, offs, cells, scan_tmp, st);
     if (p == passes - 1) {
       k_radix_scatter<kOutCsr, kDigitKey, true><<<(unsigned)ntiles, kRadixThreads, kScatterSmem, st>>>(
@@ -317,7 +357,7 @@ int radix_sort_pairs_to_csr(lne_ctx* ctx, unsigned long long* keys, uint32_t* va
       std::swap(src_k, dst_k);
       std::swap(src_v, dst_v);
     }
-    if (launches) *launches += 5;  // histogram, 3-launch scan, scatter
+    if (launches) *launches += 2 + scan_launches(cells);  // histogram, scan, scatter
   }
   dfree(ctx, mem);
   cudaError_t e = cudaGetLastError();
@@ -366,7 +406,7 @@ int radix_sort_sym_csr(lne_ctx* ctx, unsigned long long* keys, uint32_t* vals, u
   for (int p = 0; p < passes1; ++p) {
     const int shift = p * dbits1, dbits = dbits1;
     const int64_t c = (int64_t)(1 << dbits) * ntiles;
-    k_radix_hist<kDigitKey><<<hist_grid(ntiles), kRadixThreads, 0, st>>>(src_k, count, shift, dbits, ntiles, hist, 0);
+    radix_hist<kDigitKey>(ctx, src_k, count, shift, dbits, ntiles, hist, 0);
     scan_exclusive_i64(hist, offs, c, scan_tmp, st);
     if (p == passes1 - 1)
       k_radix_scatter<kOutUpper, kDigitKey, true><<<(unsigned)ntiles, kRadixThreads, kScatterSmem, st>>>(
@@ -377,13 +417,13 @@ int radix_sort_sym_csr(lne_ctx* ctx, unsigned long long* keys, uint32_t* vals, u
           src_k, src_v, count, shift, dbits, ntiles, offs, dst_k, dst_v, nullptr, nullptr, 0, 0);
     std::swap(src_k, dst_k);
     std::swap(src_v, dst_v);
-    if (launches) *launches += 5;
+    if (launches) *launches += 2 + scan_launches(c);
   }
   // the transposes, already ordered by u, stably by v: the lower triangle
   for (int p = 0; p < passes2; ++p) {
     const int shift = cbits + p * dbits2, dbits = dbits2;
     const int64_t c = (int64_t)(1 << dbits) * ntiles;
-    k_radix_hist<kDigitKey><<<hist_grid(ntiles), kRadixThreads, 0, st>>>(src_k, count, shift, dbits, ntiles, hist, 0);
+    radix_hist<kDigitKey>(ctx, src_k, count, shift, dbits, ntiles, hist, 0);
     scan_exclusive_i64(hist, offs, c, scan_tmp, st);
     if (p == passes2 - 1)
       k_radix_scatter<kOutLower, kDigitKey, true><<<(unsigned)ntiles, kRadixThreads, kScatterSmem, st>>>(
@@ -394,7 +434,7 @@ int radix_sort_sym_csr(lne_ctx* ctx, unsigned long long* keys, uint32_t* vals, u
           src_k, src_v, count, shift, dbits, ntiles, offs, dst_k, dst_v, nullptr, nullptr, 0, 0);
     std::swap(src_k, dst_k);
     std::swap(src_v, dst_v);
-    if (launches) *launches += 5;
+    if (launches) *launches += 2 + scan_launches(c);
   }
   dfree(ctx, mem);
   cudaError_t e = cudaGetLastError();
@@ -428,12 +468,11 @@ int partition_by_slot(lne_ctx* ctx, const unsigned long long* keys, unsigned lon
   cudaStream_t st = ctx->stream;
   cudaFuncSetAttribute(k_radix_scatter<kOutNext, kDigitSlot, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)kScatterSmem);
-  k_radix_hist<kDigitSlot><<<hist_grid(ntiles), kRadixThreads, 0, st>>>(keys, count, shift, dbits, ntiles, hist,
-                                                                       hmask);
+  radix_hist<kDigitSlot>(ctx, keys, count, shift, dbits, ntiles, hist, hmask);
   scan_exclusive_i64(hist, offs, cells, scan_tmp, st);
   k_radix_scatter<kOutNext, kDigitSlot, false><<<(unsigned)ntiles, kRadixThreads, kScatterSmem, st>>>(
       keys, nullptr, count, shift, dbits, ntiles, offs, out, nullptr, nullptr, nullptr, 0, hmask);
-  if (launches) *launches += 5;
+  if (launches) *launches += 2 + scan_launches(cells);
   dfree(ctx, mem);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -475,12 +514,12 @@ int partition_by_top_bits(lne_ctx* ctx, unsigned long long* keys, unsigned long 
     // digits from the least significant of the top bits up; the last digit
     // may extend past bit 63, where the shifted word is zero
     const int shift = 64 - top_bits + p * dbits;
-    k_radix_hist<kDigitKey><<<hist_grid(ntiles), kRadixThreads, 0, st>>>(src, count, shift, dbits, ntiles, hist, 0);
+    radix_hist<kDigitKey>(ctx, src, count, shift, dbits, ntiles, hist, 0);
     scan_exclusive_i64(hist, offs, cells, scan_tmp, st);
     k_radix_scatter<kOutNext, kDigitKey, false><<<(unsigned)ntiles, kRadixThreads, kScatterSmem, st>>>(
         src, nullptr, count, shift, dbits, ntiles, offs, dst, nullptr, nullptr, nullptr, 0, 0);
     std::swap(src, dst);
-    if (launches) *launches += 5;
+    if (launches) *launches += 2 + scan_launches(cells);
   }
   *result = src;
   dfree(ctx, mem);

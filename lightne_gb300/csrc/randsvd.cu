@@ -201,7 +201,7 @@ extern "C" int lne_randsvd(lne_ctx* ctx, const lne_csr* Acsr, const lne_randsvd_
   const bool low = p->precision != LNE_PREC_FP32;  // a 16-bit form
   cudaStream_t st = ctx->stream;
   int launches = 0;
-  if (!A->plan_ready) launches += kPlanLaunches;
+  if (!A->plan_ready) launches += plan_launches(A->n);
   int rc = build_plan_csr(ctx, A);
   if (rc) return rc;
 

@@ -183,7 +183,7 @@ int sparse_projection_build(lne_ctx* ctx, int64_t n, int rank, uint64_t seed, do
       (rc = dalloc(ctx, (void**)&O->val, sizeof(float) * (nnz > 0 ? nnz : 1), "sparse projection val")))
     return rc;
   if (n > 0) k_sp_fill<<<grid, 256, 0, st>>>(n, rank, seed, density, value, O->rp, O->col, O->val);
-  if (launches) *launches += 5;  // count, 3-launch scan, fill
+  if (launches) *launches += 2 + scan_launches(n);  // count, scan, fill
   LNE_CUDA_TRY(cudaGetLastError());
   return LNE_OK;
 }

@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdio.h>
+#include <string.h>
 
 #include <algorithm>
 #include <string>
@@ -427,6 +428,85 @@ __global__ void __launch_bounds__(kWalkThreads, 6) k_walk_counts(
       else
         atomicExch(flags + kFlagSortOverflow, 1);
     }
+  }
+}
+
+// The same sampler in two kernels for graphs with few directed entries.  An
+// entry's generator state is a chain, but how far a sample moves it depends
+// on the sample's r alone, not on the walk (one draw for r, one for k, one
+// per step), so k_walk_states runs ahead of the walks: a lane per entry
+// writes down the state at the start of each of its samples.  Then every
+// sample is a lane of k_walk_samples.  k_walk_counts hides the latency of a
+// walk's dependent loads behind other entries' walks; with fewer entries than
+// lanes a sample waited for the one before it (8,000 edges x 20 samples
+// took 101 us), while a full device is bound by the draws, of which this form
+// makes each one twice.
+__global__ void __launch_bounds__(kWalkThreads) k_walk_states(const uint32_t* __restrict__ nbrs,
+                                                              const uint32_t* __restrict__ src, int64_t m_dir,
+                                                              SampleArgs a, uint64_t* __restrict__ states,
+                                                              uint8_t* __restrict__ extra) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= m_dir) return;
+  uint64_t s = rng_fork(a.seed, ((uint64_t)__ldg(src + e) << 32) | (uint64_t)__ldg(nbrs + e));
+  uint64_t todo = a.exp_rv;
+  if (a.use_frac) todo += (map_uint64(rng_draw(s)) < a.frac) ? 1u : 0u;
+  extra[e] = todo > a.exp_rv;
+  for (uint64_t i = 0; i < todo; ++i) {
+    states[i * (uint64_t)m_dir + (uint64_t)e] = s;
+    // k and the r - 1 steps: r draws after r's own
+    const uint32_t r = gm_mod(rng_draw(s), (uint32_t)a.walk_len, a.walk_magic) + 1u;
+    for (uint32_t d = 0; d < r; ++d) s = rng_next(s);
+  }
+}
+
+__global__ void __launch_bounds__(kWalkThreads) k_walk_samples(const Vertex* __restrict__ vd,
+                                                               const uint32_t* __restrict__ nbrs,
+                                                               const uint32_t* __restrict__ src, int64_t m_dir,
+                                                               SampleArgs a, const uint64_t* __restrict__ states,
+                                                               const uint8_t* __restrict__ extra, int64_t samples,
+                                                               unsigned long long* __restrict__ out_keys,
+                                                               unsigned long long* __restrict__ out_count,
+                                                               uint64_t out_cap, int* flags) {
+  __shared__ unsigned long long rmag[kMaxRMagic + 1];
+  for (int i = threadIdx.x; i <= kMaxRMagic; i += blockDim.x) rmag[i] = gm_magic(i > 0 ? (uint32_t)i : 1u);
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t i = t / m_dir, e = t - i * m_dir;
+  const bool on = t < samples && ((uint64_t)i < a.exp_rv || extra[e]);
+  unsigned long long key = 0;
+  if (on) {
+    uint64_t s = states[t];
+    const uint32_t u = __ldg(src + e), v = __ldg(nbrs + e);
+    const uint32_t r = gm_mod(rng_draw(s), (uint32_t)a.walk_len, a.walk_magic) + 1u;
+    const uint32_t k = gm_mod(rng_draw(s), r, r <= kMaxRMagic ? rmag[r] : gm_magic(r)) + 1u;
+    // k - 1 steps from u, then r - k from v
+    uint32_t end[2] = {u, v};
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      uint32_t cur = end[side];
+      const uint32_t steps = side == 0 ? k - 1u : r - k;
+      for (uint32_t d = 0; d < steps; ++d) {
+        const uint4 rec = __ldg(reinterpret_cast<const uint4*>(vd + cur));
+        const uint32_t deg = rec.y > 0 ? rec.y : 1u;  // (a validated graph has no walk through degree 0)
+        cur = __ldg(nbrs + rec.x + gm_mod(rng_draw(s), deg, ((uint64_t)rec.w << 32) | rec.z));
+      }
+      end[side] = cur;
+    }
+    const uint32_t lo = end[0] < end[1] ? end[0] : end[1], hi = end[0] < end[1] ? end[1] : end[0];
+    key = hash64_2(((uint64_t)lo << 32) + (uint64_t)hi);
+  }
+  // (the keys' order does not show in the output)
+  const unsigned em = __ballot_sync(kFullMask, on);
+  unsigned long long base = 0;
+  if (lane == 0 && em) base = atomicAdd(out_count, (unsigned long long)__popc(em));
+  base = __shfl_sync(kFullMask, base, 0);
+  if (on) {
+    const uint64_t pos = base + __popc(em & ((1u << lane) - 1));
+    if (pos < out_cap)
+      out_keys[pos] = key;
+    else
+      atomicExch(flags + kFlagSortOverflow, 1);
   }
 }
 
@@ -1146,7 +1226,7 @@ static int sparsify_rounds(lne_ctx* ctx, const lne_graph* g, const lne_sparsify_
       }
       if ((rc = dalloc(ctx, (void**)&row_ptr, sizeof(int64_t) * (n + 1), "row_ptr"))) return rc;
       scan_exclusive_i64((const int64_t*)rowcnt, row_ptr, n, scan_tmp, st);
-      launches += 3;
+      launches += scan_launches(n);
       LNE_CUDA_TRY(cudaMemcpyAsync(&nnz, row_ptr + n, 8, cudaMemcpyDeviceToHost, st));
       LNE_CUDA_TRY(cudaStreamSynchronize(st));
       if ((rc = dalloc(ctx, (void**)&col, sizeof(int32_t) * (nnz > 0 ? nnz : 1), "csr col")) ||
@@ -1394,13 +1474,30 @@ extern "C" int lne_sparsify(lne_ctx* ctx, const lne_graph* g, const lne_sparsify
   const size_t slice_smem = (size_t)slots_max * (sizeof(unsigned long long) + sizeof(unsigned));
   const bool sliced_try = !p->sample && slots_max > 0 && want_keys <= max_keys && slice_smem + 1024 <= ctx->smem_optin;
   bool sliced = false;
+  unsigned long long sliced_cnt[2] = {0, 0};  // samples counted, distinct pairs
+  int sliced_flags[kFlagWords] = {};
   unsigned long long emitted_total = 0;
   if (sliced_try) {
     const unsigned wblocks = (unsigned)std::min<int64_t>((m_dir + kWalkThreads - 1) / kWalkThreads,
                                                          (int64_t)ctx->num_sms * 6);
-    LNE_CUDA_TRY(cudaMemsetAsync(counters + 6, 0, 8, st));
-    k_walk_counts<true><<<wblocks, kWalkThreads, 0, st>>>(g->vdata, g->nbrs, g->src, 0, m_dir, a, keys, counters,
-                                                          buf_keys, ctx->d_flags, counters + 6);
+    // Few entries: the states ahead of the walks (in the buffer the partition
+    // uses afterwards).  At a third of the lanes of the other form's grid the
+    // two take the same time.
+    if (3 * m_dir <= (int64_t)ctx->num_sms * 6 * kWalkThreads) {
+      uint8_t* extra = nullptr;
+      if ((rc = S.get((void**)&extra, (size_t)m_dir, "extra samples"))) return rc;
+      k_walk_states<<<(unsigned)((m_dir + kWalkThreads - 1) / kWalkThreads), kWalkThreads, 0, st>>>(
+          g->nbrs, g->src, m_dir, a, reinterpret_cast<uint64_t*>(keys2), extra);
+      k_walk_samples<<<(unsigned)((want_keys + kWalkThreads - 1) / kWalkThreads), kWalkThreads, 0, st>>>(
+          g->vdata, g->nbrs, g->src, m_dir, a, reinterpret_cast<const uint64_t*>(keys2), extra, (int64_t)want_keys,
+          keys, counters, buf_keys, ctx->d_flags);
+      S.release(extra);
+      launches_sample += 1;
+    } else {
+      LNE_CUDA_TRY(cudaMemsetAsync(counters + 6, 0, 8, st));
+      k_walk_counts<true><<<wblocks, kWalkThreads, 0, st>>>(g->vdata, g->nbrs, g->src, 0, m_dir, a, keys, counters,
+                                                            buf_keys, ctx->d_flags, counters + 6);
+    }
     ++launches_sample;
     unsigned long long got = 0;
     LNE_CUDA_TRY(cudaMemcpyAsync(&got, counters, 8, cudaMemcpyDeviceToHost, st));
@@ -1444,6 +1541,9 @@ extern "C" int lne_sparsify(lne_ctx* ctx, const lne_graph* g, const lne_sparsify
       // Above 90% of the pair table's capacity the table decides whether
       // the reference's table would fill: rerun through it.
       sliced = !fl[kFlagSliceOverflow] && sc[1] * 10 <= (unsigned long long)cap * 9;
+      sliced_cnt[0] = sc[0];
+      sliced_cnt[1] = sc[1];
+      memcpy(sliced_flags, fl, sizeof(fl));
       if (!sliced) {
         S.release(uniq);
         uniq = nullptr;
@@ -1499,14 +1599,16 @@ extern "C" int lne_sparsify(lne_ctx* ctx, const lne_graph* g, const lne_sparsify
       k_table_sum<false><<<sgrid, 256, 0, st>>>(table, cap, counters + 1, counters + 2, wsum);
     k_sum_blocks<<<1, 32, 0, st>>>(wsum, sgrid, wsum + sum_blocks);
   }
-  unsigned long long h_cnt[3] = {0, 0, 0};
-  LNE_CUDA_TRY(cudaMemsetAsync(counters, 0, 8, st));
+  unsigned long long h_cnt[3] = {0, sliced_cnt[0], sliced_cnt[1]};
   double h_w = 0.0;
   int h_flags[kFlagWords];
-  LNE_CUDA_TRY(cudaMemcpyAsync(h_cnt, counters, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
-  LNE_CUDA_TRY(cudaMemcpyAsync(&h_w, wsum + sum_blocks, sizeof(double), cudaMemcpyDeviceToHost, st));
-  LNE_CUDA_TRY(cudaMemcpyAsync(h_flags, ctx->d_flags, sizeof(h_flags), cudaMemcpyDeviceToHost, st));
-  LNE_CUDA_TRY(cudaStreamSynchronize(st));
+  memcpy(h_flags, sliced_flags, sizeof(h_flags));
+  if (!sliced) {  // (the sliced aggregation has read them back)
+    LNE_CUDA_TRY(cudaMemcpyAsync(h_cnt, counters, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
+    LNE_CUDA_TRY(cudaMemcpyAsync(&h_w, wsum + sum_blocks, sizeof(double), cudaMemcpyDeviceToHost, st));
+    LNE_CUDA_TRY(cudaMemcpyAsync(h_flags, ctx->d_flags, sizeof(h_flags), cudaMemcpyDeviceToHost, st));
+    LNE_CUDA_TRY(cudaStreamSynchronize(st));
+  }
   LNE_CUDA_TRY(cudaGetLastError());
   h_cnt[0] = emitted_total;
   if (h_flags[kFlagSortOverflow]) {
@@ -1571,7 +1673,7 @@ extern "C" int lne_sparsify(lne_ctx* ctx, const lne_graph* g, const lne_sparsify
   // sorts: [full | tcnt | upstart | tstart | upoff | looff]
   int64_t* offs = nullptr;
   int64_t *upoff = nullptr, *looff = nullptr;
-  int extra_launches = 3;  // the row pointer scan
+  int extra_launches = scan_launches(n);  // the row pointer scan
   if (!p->upper) {
     if ((rc = dalloc(ctx, (void**)&offs, sizeof(int64_t) * (6 * (size_t)n + 2), "csr offsets"))) {
       dfree(ctx, row_ptr);
@@ -1589,7 +1691,7 @@ extern "C" int lne_sparsify(lne_ctx* ctx, const lne_graph* g, const lne_sparsify
     scan_exclusive_i64((const int64_t*)rowcnt, upstart, n, scan_tmp, st);
     scan_exclusive_i64(tcnt, tstart, n, scan_tmp, st);
     k_sym_offsets<<<og, 256, 0, st>>>(row_ptr, lowcnt, upstart, tstart, n, upoff, looff);
-    extra_launches += 2 + 6;
+    extra_launches += 2 + 2 * scan_launches(n);
   } else {
     scan_exclusive_i64((const int64_t*)rowcnt, row_ptr, n, scan_tmp, st);
   }

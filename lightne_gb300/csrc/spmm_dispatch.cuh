@@ -248,7 +248,7 @@ static int spmm_csr_panels(lne_ctx* ctx, lne_csr* A, const XT* X, int64_t ldx, i
     if (A->hub_share < 0.5) budget = 0;
   }
   if (budget == 0 || xbytes <= budget) {
-    if (!A->plan_ready && launches) *launches += kPlanLaunches;
+    if (!A->plan_ready && launches) *launches += plan_launches(A->n);
     if ((rc = build_plan_csr(ctx, A))) return rc;
     epi.add = false;
     return spmm_run<XT, true>(ctx, A->plan, reinterpret_cast<const uint32_t*>(A->col), A->val, X, ldx, d, epi, launches,
@@ -262,7 +262,7 @@ static int spmm_csr_panels(lne_ctx* ctx, lne_csr* A, const XT* X, int64_t ldx, i
     for (int64_t b = pw; b < A->n; b += pw) bounds.push_back(b);
   }
   bounds.push_back(A->n);
-  if (A->panel_bounds != bounds && launches) *launches += 1 + (int)(bounds.size() - 1) * kPlanLaunches;
+  if (A->panel_bounds != bounds && launches) *launches += 1 + (int)(bounds.size() - 1) * plan_launches(A->n);
   if ((rc = build_panels(ctx, A, bounds))) return rc;
   for (int p = 0; p < A->npanels; ++p) {
     epi.add = p > 0;

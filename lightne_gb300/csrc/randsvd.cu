@@ -93,9 +93,10 @@ __global__ void k_copy_cols(const float* __restrict__ X, int64_t ldx, int64_t n,
 
 }  // namespace
 
-// CholeskyQR on X (n x ld FP32, r columns) with tmp as the ping-pong
-// partner; the two pointers are swapped so that the result ends in X.  Xb
-// (optional) receives a 16-bit copy of the result from the last GEMM.
+// CholeskyQR of `in` (n x ld FP32, r columns): the passes write to `a`, then
+// to `b` and `a` in turn (b may be `in`); *Q gets the one that holds the
+// result, *spare the other.  Xb (optional) receives a 16-bit copy of the
+// result from the last GEMM.
 //
 // The first pass is shifted (Fukaya et al. 2020: G + s I with s = 64 u tr G,
 // the shift growing x10 while a pivot fails), then plain passes follow.
@@ -105,15 +106,15 @@ __global__ void k_copy_cols(const float* __restrict__ X, int64_t ldx, int64_t n,
 // third pass follows (shifted CholeskyQR3), as for the second QR of the
 // randomized SVD, whose Z = B P has kappa ~ 5e3.
 static constexpr double kCholQR2Tol = 0.5;
-static int cholqr3(lne_ctx* ctx, float*& X, float*& tmp, int64_t n, int64_t ld, int r, Copy16 Xb,
-                   int* launches) {
+static int cholqr3(lne_ctx* ctx, const float* in, float* a, float* b, float** Q, float** spare, int64_t n, int64_t ld,
+                   int r, Copy16 Xb, int* launches) {
   Buf B(ctx);
   double* G = nullptr;
   float* W = nullptr;
   int rc;
   if ((rc = B.get(&G, (size_t)r * r, "gram")) || (rc = B.get(&W, (size_t)r * r, "R^-1"))) return rc;
-  float* src = X;
-  float* dst = tmp;
+  const float* src = in;
+  float* dst = a;
   const double u32 = 5.9604644775390625e-08;
   for (int pass = 0; pass < 3; ++pass) {
     double shift = 0.0;
@@ -140,15 +141,12 @@ static int cholqr3(lne_ctx* ctx, float*& X, float*& tmp, int64_t n, int64_t ld, 
     }
     if ((rc = gemm_tall(ctx, src, ld, r, W, r, n, dst, ld, last ? Xb : Copy16()))) return rc;
     *launches += 1;
-    float* t = src;
     src = dst;
-    dst = t;
+    dst = dst == a ? b : a;
     if (last) break;
   }
-  // the result is in src: the buffer X came in after two passes, tmp's
-  // after three
-  X = src;
-  tmp = dst;
+  *spare = dst;
+  *Q = dst == a ? b : a;
   return LNE_OK;
 }
 
@@ -269,7 +267,7 @@ extern "C" int lne_randsvd(lne_ctx* ctx, const lne_csr* Acsr, const lne_randsvd_
     q16.kind = f16 ? 2 : 1;
     q16.scale = f16 ? kQHalfScale : 1.0f;
   }
-  if ((rc = cholqr3(ctx, Y, T, n, ld, r, q16, &launches))) return rc;
+  if ((rc = cholqr3(ctx, Y, T, Y, &Y, &T, n, ld, r, q16, &launches))) return rc;
   cudaEventRecord(ev[2], st);
   // B = A * Q
   if ((rc = B.get(&Bm, (size_t)n * ld, "B"))) return rc;
@@ -288,7 +286,7 @@ extern "C" int lne_randsvd(lne_ctx* ctx, const lne_csr* Acsr, const lne_randsvd_
   if ((rc = gaussian_fill_f32(ctx, p->seed, 1, r, r, P, r))) return rc;
   if ((rc = gemm_tall(ctx, Bm, ld, r, P, r, n, Y, ld))) return rc;
   launches += 2;
-  if ((rc = cholqr3(ctx, Y, T, n, ld, r, Copy16(), &launches))) return rc;
+  if ((rc = cholqr3(ctx, Y, T, Y, &Y, &T, n, ld, r, Copy16(), &launches))) return rc;
   cudaEventRecord(ev[4], st);
   // C = Z^T B, C = U_C S V^T
   if ((rc = B.get(&C, (size_t)r * r, "C")) || (rc = B.get(&U, (size_t)r * r, "U_C")) ||
@@ -376,19 +374,23 @@ extern "C" int lne_dense_embed(lne_ctx* ctx, const float* d_x, int64_t n, int64_
   float *X = nullptr, *Q = nullptr, *T = nullptr, *W = nullptr;
   double *C = nullptr, *U = nullptr, *S = nullptr;
   int rc, launches = 0;
-  if ((rc = B.get(&X, (size_t)n * ld, "X")) || (rc = B.get(&Q, (size_t)n * ld, "Q")) ||
+  // x is read in place where its rows are whole 16-byte vectors, else a
+  // zero-padded copy
+  const bool direct = ld == d && ((uintptr_t)d_x & 15) == 0;
+  if ((!direct && (rc = B.get(&X, (size_t)n * ld, "X"))) || (rc = B.get(&Q, (size_t)n * ld, "Q")) ||
       (rc = B.get(&T, (size_t)n * ld, "QR scratch")) || (rc = B.get(&C, (size_t)d * d, "R")) ||
       (rc = B.get(&U, (size_t)d * d, "U_R")) || (rc = B.get(&S, (size_t)d, "S")) ||
       (rc = B.get(&W, (size_t)d * d, "U sqrt(S)")))
     return rc;
-  // padded copy (the pad columns are zero)
-  LNE_CUDA_TRY(cudaMemsetAsync(X, 0, sizeof(float) * n * ld, st));
-  LNE_CUDA_TRY(cudaMemcpy2DAsync(X, sizeof(float) * ld, d_x, sizeof(float) * d, sizeof(float) * d, n,
-                                 cudaMemcpyDeviceToDevice, st));
-  LNE_CUDA_TRY(cudaMemcpyAsync(Q, X, sizeof(float) * n * ld, cudaMemcpyDeviceToDevice, st));
+  if (!direct) {
+    LNE_CUDA_TRY(cudaMemsetAsync(X, 0, sizeof(float) * n * ld, st));
+    LNE_CUDA_TRY(cudaMemcpy2DAsync(X, sizeof(float) * ld, d_x, sizeof(float) * d, sizeof(float) * d, n,
+                                   cudaMemcpyDeviceToDevice, st));
+  }
+  const float* Xin = direct ? d_x : X;
   // X = Q R with Q from CholeskyQR; R = Q^T X; R = U_R S V^T; U = Q U_R
-  if ((rc = cholqr3(ctx, Q, T, n, ld, d, Copy16(), &launches))) return rc;
-  if ((rc = gram(ctx, Q, ld, d, X, ld, d, n, C))) return rc;
+  if ((rc = cholqr3(ctx, Xin, Q, T, &Q, &T, n, ld, d, Copy16(), &launches))) return rc;
+  if ((rc = gram(ctx, Q, ld, d, Xin, ld, d, n, C))) return rc;
   int sweeps = 0;
   if ((rc = jacobi_svd(ctx, C, d, U, S, &sweeps, nullptr, core_svd_sweep_cap(ctx, true)))) return rc;
   k_scale_cols<<<(d * d + 255) / 256, 256, 0, st>>>(U, S, d, d, W);

@@ -118,6 +118,28 @@ __device__ __forceinline__ void copy16_put(const Copy16& c, int64_t idx, float v
     reinterpret_cast<__half*>(c.p)[idx] = __float2half_rn(v * c.scale);
 }
 
+// Four consecutive elements from index idx (a multiple of 4).
+__device__ __forceinline__ void copy16_put4(const Copy16& c, int64_t idx, const float4 v) {
+  if (c.kind == 0) return;
+  uint2 q;
+  if (c.kind == 1) {
+    q.x = pack2_16<__nv_bfloat16>(v.x, v.y);
+    q.y = pack2_16<__nv_bfloat16>(v.z, v.w);
+  } else {
+    q.x = pack2_16<__half>(c.scale * v.x, c.scale * v.y);
+    q.y = pack2_16<__half>(c.scale * v.z, c.scale * v.w);
+  }
+  uint16_t* p = reinterpret_cast<uint16_t*>(c.p) + idx;
+  if ((reinterpret_cast<uintptr_t>(c.p) & 7) == 0) {
+    *reinterpret_cast<uint2*>(p) = q;
+  } else {
+    copy16_put(c, idx, v.x);
+    copy16_put(c, idx + 1, v.y);
+    copy16_put(c, idx + 2, v.z);
+    copy16_put(c, idx + 3, v.w);
+  }
+}
+
 // Elements [col0, col0 + 16) of row `row` (leading dimension ld), of which
 // the first `valid` are in the row: 16-byte stores where ld is a multiple
 // of 8 and the copy is 16-byte aligned, element stores otherwise.

@@ -433,6 +433,27 @@ __global__ void __launch_bounds__(kSThreads, 1) k_tc_gemm_stream(const float* __
   stream_finish(sh, tmem, 256, ok, last_commit, flags);
 }
 
+// Piece q (4 floats) of each of a lane group's four rows to lane q: on entry a
+// lane holds the four pieces of its row, on return piece (lane & 3) of rows
+// 0..3 of the group.
+__device__ __forceinline__ void transpose4(float (&v)[16], int lane) {
+#pragma unroll
+  for (int s = 1; s <= 2; s <<= 1) {
+    const bool up = lane & s;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int a = s == 1 ? 2 * h : h, b = a + s;  // the pieces that change places
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float give = up ? v[4 * a + e] : v[4 * b + e];
+        const float got = __shfl_xor_sync(0xffffffffu, give, s);
+        v[4 * a + e] = up ? got : v[4 * a + e];
+        v[4 * b + e] = up ? v[4 * b + e] : got;
+      }
+    }
+  }
+}
+
 // Warp-specialised form of the update GEMM (same operands, layouts and
 // MMAs as k_tc_gemm_stream), for W of at most kWsMaxCols columns:
 //   warps 8-9 (loaders)  cp.async of raw 16-K slices of In into a ring of
@@ -655,20 +676,31 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_tc_gemm_ws(const __grid_const
       for (int cg = 0; cg * 16 < nmma; ++cg) {
         float v[16];
         tc::tmem_ld16(tmem + (uint32_t)(b * kWsMaxCols) + ((uint32_t)(32 * lg) << 16) + (uint32_t)(cg * 16), v);
-        if (row < n) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (cg * 16 + i >= c2) v[i] = 0.0f;
+        if (vec) {
+          // Four lanes exchange the 16-byte pieces of their four rows, so
+          // that they store 64 consecutive bytes of a row together: a store
+          // touches 8 rows instead of 32 rows' half sectors.
+          transpose4(v, lane);
+          const int col = cg * 16 + 4 * (lane & 3);
+          const int64_t row0 = tile * 128 + 32 * lg + (lane & ~3);
+          if (col < ldo) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              if (row0 + k < n) {
+                const float4 o = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                *reinterpret_cast<float4*>(Out + (row0 + k) * ldo + col) = o;
+                copy16_put4(OutB, (row0 + k) * ldo + col, o);
+              }
+            }
+          }
+        } else if (row < n) {
+          float* orow = Out + row * ldo + cg * 16;
 #pragma unroll
           for (int i = 0; i < 16; ++i)
-            if (cg * 16 + i >= c2) v[i] = 0.0f;
-          float* orow = Out + row * ldo + cg * 16;
-          if (vec && cg * 16 + 16 <= ldo) {
-#pragma unroll
-            for (int i = 0; i < 16; i += 4)
-              *reinterpret_cast<float4*>(orow + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-              if (cg * 16 + i < ldo) orow[i] = v[i];
-          }
+            if (cg * 16 + i < ldo) orow[i] = v[i];
           copy16_put_row16(OutB, row, ldo, cg * 16, v, (int)std::min<int64_t>(16, ldo - cg * 16));
         }
       }

@@ -132,12 +132,21 @@ struct RawRow {
     }
   }
 };
+// FP32 state of the recursion: read and written once per product, with the
+// streaming policy, so that it does not push the gathered operand out of L2.
 template <int N>
 __device__ __forceinline__ void load_f32(const float* __restrict__ X, int64_t ld, int64_t r, int e0, float (&o)[N]) {
-  uint32_t w[N];
-  load_words<N>(reinterpret_cast<const uint32_t*>(X + r * ld + e0), w);
+  const float* p = X + r * ld + e0;
+  if constexpr (N % 4 == 0) {
 #pragma unroll
-  for (int i = 0; i < N; ++i) o[i] = __uint_as_float(w[i]);
+    for (int i = 0; i < N; i += 4) {
+      const float4 v = __ldcs(reinterpret_cast<const float4*>(p + i));
+      o[i] = v.x; o[i + 1] = v.y; o[i + 2] = v.z; o[i + 3] = v.w;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) o[i] = __ldcs(p + i);
+  }
 }
 template <int N>
 __device__ __forceinline__ void store_f32(float* __restrict__ X, int64_t ld, int64_t r, int e0, const float (&o)[N]) {
@@ -145,6 +154,29 @@ __device__ __forceinline__ void store_f32(float* __restrict__ X, int64_t ld, int
 #pragma unroll
   for (int i = 0; i < N; ++i) w[i] = __float_as_uint(o[i]);
   store_words<N>(reinterpret_cast<uint32_t*>(X + r * ld + e0), w);
+}
+template <int N>
+__device__ __forceinline__ void store_f32_cs(float* __restrict__ X, int64_t ld, int64_t r, int e0,
+                                             const float (&o)[N]) {
+  float* p = X + r * ld + e0;
+  if constexpr (N % 4 == 0) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4)
+      __stcs(reinterpret_cast<float4*>(p + i), make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]));
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) __stcs(p + i, o[i]);
+  }
+}
+// A Chebyshev vector's FP32 copy: gathered by the next product in the FP32
+// form only.
+template <typename XT, int N>
+__device__ __forceinline__ void store_state(float* __restrict__ X, int64_t ld, int64_t r, int e0,
+                                            const float (&o)[N]) {
+  if constexpr (sizeof(XT) == 4)
+    store_f32<N>(X, ld, r, e0, o);
+  else
+    store_f32_cs<N>(X, ld, r, e0, o);
 }
 template <typename HT, int N>
 __device__ __forceinline__ void store_16(HT* __restrict__ X, int64_t ld, int64_t r, int e0, const float (&o)[N]) {
@@ -323,12 +355,12 @@ struct EpiFirst {
       cv[i] = fmaf(c1, l1[i], c0 * a);
     }
     if constexpr (DOTS) dot_v<N>(dot, coef, r, e0, l1, st);
-    if (L1) store_f32<N>(L1, ld, r, e0, l1);
+    if (L1) store_state<XT, N>(L1, ld, r, e0, l1);
     if (L1b) store_16<HT, N>(L1b, ld, r, e0, l1);
     if (fin.base)
       fin.template apply<N>(r, e0, ld, coef, cv);
     else if (conv)
-      store_f32<N>(conv, ld, r, e0, cv);
+      store_f32_cs<N>(conv, ld, r, e0, cv);
   }
 };
 
@@ -385,9 +417,9 @@ struct EpiStep {
     if (fin.base) {
       fin.template apply<N>(r, e0, ld, coef, cv);
     } else {
-      if (L2) store_f32<N>(L2, ld, r, e0, l2);
+      if (L2) store_state<XT, N>(L2, ld, r, e0, l2);
       if (L2b) store_16<HT, N>(L2b, ld, r, e0, l2);
-      if (sum) store_f32<N>(conv, ld, r, e0, cv);
+      if (sum) store_f32_cs<N>(conv, ld, r, e0, cv);
     }
   }
 };
@@ -471,7 +503,7 @@ struct EpiAdjInit {
 };
 
 // dst (n x ld, zero padding; may be null) = scale * src (n x d) and its
-// 16-bit copy.
+// 16-bit copy (may be null).
 template <typename HT>
 __global__ void k_pad_copy(const float* __restrict__ src, int64_t n, int d, float scale, float* __restrict__ dst,
                            int64_t ld, HT* __restrict__ dstb) {
@@ -489,6 +521,17 @@ __global__ void k_pad_copy(const float* __restrict__ src, int64_t n, int d, floa
   }
 }
 
+// dst = the 16-bit copy of scale * src, total a multiple of 8 values, both
+// 16-byte aligned.
+template <typename HT>
+__global__ void k_shadow_copy(const float4* __restrict__ src, int64_t total8, float scale, uint4* __restrict__ dst) {
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total8; t += (int64_t)gridDim.x * blockDim.x) {
+    const float4 a = __ldcs(src + 2 * t), b = __ldcs(src + 2 * t + 1);
+    dst[t] = make_uint4(pack2_16<HT>(scale * a.x, scale * a.y), pack2_16<HT>(scale * a.z, scale * a.w),
+                        pack2_16<HT>(scale * b.x, scale * b.y), pack2_16<HT>(scale * b.z, scale * b.w));
+  }
+}
+
 // dst (n x d) = scale * src (n x ld).
 __global__ void k_unpad_copy(const float* __restrict__ src, int64_t ld, int64_t n, int d, float scale,
                              float* __restrict__ dst) {
@@ -500,13 +543,23 @@ __global__ void k_unpad_copy(const float* __restrict__ src, int64_t ld, int64_t 
 
 // Largest |x| over an n x d FP32 matrix (row stride d): one float per
 // block; non-finite values count as +inf.
-static constexpr int kAmaxBlocks = 512;
+static constexpr int kAmaxBlocks = 1216;
 __global__ void k_amax_partial(const float* __restrict__ x, int64_t total, float* __restrict__ out) {
   float m = 0.0f;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const float a = fabsf(x[t]);
+  auto take = [&](float v) {
+    const float a = fabsf(v);
     m = (a <= m) ? m : (isfinite(a) ? a : INFINITY);
+  };
+  // 16-byte loads where x allows, two in flight; then the rest
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
+  const int64_t n4 = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? total / 4 : 0;
+  const float4* x4 = reinterpret_cast<const float4*>(x);
+  for (int64_t t = tid; t < n4; t += 2 * nth) {
+    const float4 a = x4[t], b = t + nth < n4 ? x4[t + nth] : make_float4(0.f, 0.f, 0.f, 0.f);
+    take(a.x); take(a.y); take(a.z); take(a.w);
+    take(b.x); take(b.y); take(b.z); take(b.w);
   }
+  for (int64_t t = 4 * n4 + tid; t < total; t += nth) take(x[t]);
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
   __shared__ float ws[32];
   if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = m;
@@ -758,7 +811,11 @@ int propagate_impl(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, co
   if (!direct && (rc = B.get(&Acopy, sz, "a"))) return rc;
   if (k16 && ((rc = B.get(&Ab, sz, "a 16-bit")) || (rc = B.get(&Afb, sz, "a - conv 16-bit")))) return rc;
   const unsigned pg = (unsigned)std::min<int64_t>((n * ld + 255) / 256, (int64_t)ctx->num_sms * 32);
-  if (!direct || k16) {
+  if (direct && k16) {
+    k_shadow_copy<HT><<<pg, 256, 0, st>>>(reinterpret_cast<const float4*>(d_a), (int64_t)sz / 8, sc,
+                                          reinterpret_cast<uint4*>(Ab));
+    launches += 1;
+  } else if (!direct) {
     k_pad_copy<HT><<<pg, 256, 0, st>>>(d_a, n, d, sc, Acopy, ld, Ab);
     launches += 1;
   }
@@ -881,7 +938,11 @@ int adjoint_impl(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, cons
     return rc;
   if (k16 && ((rc = B.get(&Gb, sz, "g 16-bit")) || (rc = B.get(&Bb, sz, "b 16-bit")))) return rc;
   const unsigned pg = (unsigned)std::min<int64_t>(((int64_t)sz + 255) / 256, (int64_t)ctx->num_sms * 32);
-  if (k16 || !g_direct) {
+  if (g_direct && k16) {
+    k_shadow_copy<HT><<<pg, 256, 0, st>>>(reinterpret_cast<const float4*>(d_gy), (int64_t)sz / 8, sg,
+                                          reinterpret_cast<uint4*>(Gb));
+    launches += 1;
+  } else if (!g_direct) {
     k_pad_copy<HT><<<pg, 256, 0, st>>>(d_gy, n, d, sg, Gcopy, ld, Gb);
     launches += 1;
   }

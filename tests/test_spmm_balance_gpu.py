@@ -110,3 +110,20 @@ def test_parameter_gradients(ctx, precision, order, dim):
     assert abs(dmu - mu.grad.item()) <= 1e-4 * abs(mu.grad.item()) + 1e-6 * scale, (dmu, mu.grad.item())
     assert abs(ds - s.grad.item()) <= 1e-4 * abs(s.grad.item()) + 1e-6 * scale, (ds, s.grad.item())
     g.free()
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp16"])
+def test_unaligned_input(ctx, precision):
+    """Rows that are not on 16-byte boundaries take the padded copies: the
+    same bits."""
+    off, nbrs = hub_graph(900, [800, 100], 5)
+    g = Graph.from_numpy(ctx, off, nbrs)
+    buf = torch.randn(900 * 16 + 1, generator=torch.Generator().manual_seed(1)).cuda()
+    a = buf[1:].view(900, 16)
+    y, a_out, _ = chebyshev_expansion(ctx, g, a, 16, order=4, precision=precision, return_a=True)
+    y2, a2, _ = chebyshev_expansion(ctx, g, a.clone(), 16, order=4, precision=precision, return_a=True)
+    assert a.data_ptr() % 16 and torch.equal(y, y2) and torch.equal(a_out, a2)
+    ga = propagate_adjoint(ctx, g, a, a, 16, order=4, precision=precision)
+    ga2 = propagate_adjoint(ctx, g, a.clone(), a.clone(), 16, order=4, precision=precision)
+    assert torch.equal(ga[0], ga2[0]) and ga[1:] == ga2[1:]
+    g.free()

@@ -37,10 +37,8 @@ static inline int64_t spmm_places(const lne_ctx* ctx, const SpmmPlan& plan) {
 // ends after it).  Adds the launches to *nl.
 template <typename XT, int G, bool VAL, class Epi>
 static void spmm_launch_bal(lne_ctx* ctx, const SpmmPlan& plan, const SpmmArgs<XT>& s, const Epi& epi, int* nl) {
-  const int64_t units = plan.n_heavy * HeavyTune<G>::kParts;
-  if (units > 0) {
-    k_spmm_heavy<XT, G, VAL, Epi>
-        <<<(unsigned)((units + kHeavyWarps - 1) / kHeavyWarps), kHeavyWarps * 32, 0, ctx->stream>>>(s, epi);
+  if (plan.n_heavy > 0) {
+    k_spmm_heavy<XT, G, VAL, Epi><<<(unsigned)plan.n_heavy, kHeavyWarps * 32, 0, ctx->stream>>>(s, epi);
     *nl += 1;
   }
   if (plan.n_items == plan.n_heavy) return;
@@ -52,7 +50,7 @@ static void spmm_launch_bal(lne_ctx* ctx, const SpmmPlan& plan, const SpmmArgs<X
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = units > 0 ? 1 : 0;
+  cfg.numAttrs = plan.n_heavy > 0 ? 1 : 0;
   cudaLaunchKernelEx(&cfg, k_spmm<XT, G, 1, VAL, true, Epi>, s, epi);
   *nl += 1;
 }

@@ -121,11 +121,10 @@ static constexpr int kSpmmWarps = kSpmmThreads / 32;
 
 // ---------------------------------------------------------------------------
 // Balanced form (one 16-byte vector per lane, G a power of two): the rows
-// above warp_max go to k_spmm_heavy, a block of four warps per item: with one
-// 32-bit column word per lane instead of one 16-byte vector, and a strand per
-// warp (and lane group) where a row is narrower than 512 bytes, every lane
-// adds one strand of one word, with 64 rows in flight instead of four, in
-// order; so the sums are those of k_spmm.  The rest go
+// above warp_max go to k_spmm_heavy, with one 32-bit column word per lane
+// instead of one 16-byte vector, so that a 512-byte row is the work of four
+// warps and each lane has 64 rows in flight instead of four; a lane adds its
+// strands' rows in order, so the sums are those of k_spmm.  The rest go
 // to k_spmm (BAL), which starts beside it.  On a graph of 10,312 vertices
 // and 668K entries (128 FP32 columns) one product took 200 us with a warp
 // per row: a 2048-entry row is a chain of gathers that four rows in flight
@@ -134,15 +133,20 @@ static constexpr int kSpmmWarps = kSpmmThreads / 32;
 // 110 us (about 1 us per 32 rows).
 // ---------------------------------------------------------------------------
 static constexpr int kHeavyWarps = 4;
-template <int G>
+template <int G, bool VAL>
 struct HeavyTune {
   static constexpr int P = 32 / G;
   static constexpr int W = G * 4 < 32 ? G * 4 : 32;  // lanes of one row
   static constexpr int LG = 32 / W;                  // rows side by side in a warp
   static constexpr int kParts = G * 4 / W;           // warps side by side on one row
-  static constexpr int NS = kHeavyWarps / kParts;    // warps on strands of their own
+  // warps on strands of their own: an item of a graph, whose products wait
+  // for their longest rows, has the block (see k_spmm_heavy); the rows of a
+  // matrix are enough to fill the device without
+  static constexpr int NS = VAL ? 1 : kHeavyWarps / kParts;
+  static constexpr int A = P / (LG * NS);            // strands per lane
+  static constexpr int kWarps = kParts * NS;         // warps of one item
   static constexpr int kSets = 2;                    // sets of 32 rows in flight per lane
-  static_assert(LG * NS == P, "a strand per lane group and warp");
+  static_assert(A >= 1 && A * LG * NS == P && (A == 1 || NS == 1), "strands of the lanes, groups and warps");
 };
 
 // Elements of one 32-bit word of a dense row, widened.
@@ -184,23 +188,28 @@ struct Word32<__nv_fp8_e4m3> {
   }
 };
 
-// One block per heavy item: warp (part, ws) has the words 32 part .. of the
-// rows, its lane group lg the strand lg + LG ws.  The hardware hands out the
-// blocks in order, so the longest items start first.
+// kWarps warps per heavy item: warp (part, ws) has the words 32 part .. of
+// the rows, its lane group lg the strands lg + LG ws, and A - 1 more.  The
+// hardware hands out the blocks in order, so the longest items start first.
+// Spreading the strands of rows narrower than 512 bytes over a block's warps
+// took 19 products of a 2,001-vertex graph at 33 columns from 513 to 348 us;
+// on a matrix (12K rows of 250, 42 columns) it made a randomized SVD of
+// 1454 us 55 us longer, so its items have kParts warps.
 template <typename XT, int G, bool VAL, class Epi>
 __global__ void __launch_bounds__(kHeavyWarps * 32, 4) k_spmm_heavy(const SpmmArgs<XT> s, const Epi epi) {
-  using Tune = HeavyTune<G>;
-  constexpr int W = Tune::W, LG = Tune::LG, P = Tune::P, NS = Tune::NS, kSets = Tune::kSets, EW = Word32<XT>::E;
-  constexpr int kStep = 32 * P;  // nonzeros of a set of the block
+  using Tune = HeavyTune<G, VAL>;
+  constexpr int W = Tune::W, LG = Tune::LG, A = Tune::A, NS = Tune::NS, kSets = Tune::kSets, EW = Word32<XT>::E;
+  constexpr int kGap = LG * NS;     // from a lane's nonzero to its next
+  constexpr int kStep = 32 * kGap;  // nonzeros of a set
   // the light rows' kernel may start: it does not read what this one writes
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // the item from the warp's number, not the block's: 32.4 us per product of
   // that graph against 35.8 us with the item in uniform registers
   const uint32_t unit = blockIdx.x * kHeavyWarps + (threadIdx.x >> 5);
-  if (unit >= s.n_heavy * kHeavyWarps) return;
-  const uint32_t it = unit / kHeavyWarps;
+  if (unit >= s.n_heavy * Tune::kWarps) return;  // (an item's warps in one block, all or none)
+  const uint32_t it = unit / Tune::kWarps;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lg = lane / W;
-  const int part = NS == 1 ? warp : warp % Tune::kParts, ws = NS == 1 ? 0 : warp / Tune::kParts;
+  const int part = (int)(unit % Tune::kParts), ws = NS == 1 ? 0 : warp / Tune::kParts;
   const int q = part * 32 + lane % W;
   const bool on = q < s.C * 4;
   const uint4 rec = __ldg(reinterpret_cast<const uint4*>(s.items) + it);
@@ -210,9 +219,11 @@ __global__ void __launch_bounds__(kHeavyWarps * 32, 4) k_spmm_heavy(const SpmmAr
   const float* val = VAL ? s.val + item_begin(rec) : nullptr;
   const uint32_t* X = reinterpret_cast<const uint32_t*>(s.X) + (on ? q : 0);
   const uint32_t ldw = (uint32_t)(s.ldx * (int64_t)sizeof(XT) / 4);
-  float acc[EW];
+  float acc[A][EW];
 #pragma unroll
-  for (int e = 0; e < EW; ++e) acc[e] = 0.0f;
+  for (int a = 0; a < A; ++a)
+#pragma unroll
+    for (int e = 0; e < EW; ++e) acc[a][e] = 0.0f;
   // Ids and values pass through shared memory, each lane group's together,
   // so that one 16-byte broadcast serves four rows (a shuffle per row made
   // a chain of 30 cycles each); 36 words apart the groups meet no bank twice.
@@ -223,7 +234,7 @@ __global__ void __launch_bounds__(kHeavyWarps * 32, 4) k_spmm_heavy(const SpmmAr
   uint32_t c[LG];         // ids (and values) of the set after those
   float v[LG];
   // entry `at` of this warp's 32 LG ids of a set: group at % LG, its at / LG-th
-  auto nz = [&](int base, int at) { return base + P * (at / LG) + LG * ws + at % LG; };
+  auto nz = [&](int base, int at) { return NS == 1 ? base + at : base + kGap * (at / LG) + LG * ws + at % LG; };
   auto load_ids = [&](int base) {
 #pragma unroll
     for (int i = 0; i < LG; ++i) {
@@ -260,7 +271,7 @@ __global__ void __launch_bounds__(kHeavyWarps * 32, 4) k_spmm_heavy(const SpmmAr
         const uint32_t id[4] = {cc.x, cc.y, cc.z, cc.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          o[u + i] = base + (u + i) * P + LG * ws + lg < len ? __ldg(X + (uint64_t)id[i] * ldw) : 0u;
+          o[u + i] = base + (u + i) * kGap + LG * ws + lg < len ? __ldg(X + (uint64_t)id[i] * ldw) : 0u;
       }
     }
   };
@@ -273,9 +284,9 @@ __global__ void __launch_bounds__(kHeavyWarps * 32, 4) k_spmm_heavy(const SpmmAr
       for (int i = 0; i < 4; ++i) {
         float x[EW];
         Word32<XT>::unpack(o[u + i], x);
-        if (decltype(whole)::value || base + (u + i) * P + LG * ws + lg < len) {
+        if (decltype(whole)::value || base + (u + i) * kGap + LG * ws + lg < len) {
 #pragma unroll
-          for (int e = 0; e < EW; ++e) acc[e] = fmaf(m[i], x[e], acc[e]);
+          for (int e = 0; e < EW; ++e) acc[(u + i) % A][e] = fmaf(m[i], x[e], acc[(u + i) % A][e]);
         }
       }
     };
@@ -298,25 +309,34 @@ __global__ void __launch_bounds__(kHeavyWarps * 32, 4) k_spmm_heavy(const SpmmAr
       gather(base + (k + kSets) * kStep, k, w[k]);
     }
   }
-  // the strands in a balanced tree: the lane groups', then the warps'
+  // the strands in a balanced tree: the lane groups', then the lane's own or
+  // the warps'
 #pragma unroll
   for (int o = W; o < 32; o <<= 1)
 #pragma unroll
-    for (int e = 0; e < EW; ++e) acc[e] += __shfl_xor_sync(kFull, acc[e], o);
+    for (int a = 0; a < A; ++a)
+#pragma unroll
+      for (int e = 0; e < EW; ++e) acc[a][e] += __shfl_xor_sync(kFull, acc[a][e], o);
+#pragma unroll
+  for (int o = 1; o < A; o <<= 1)
+#pragma unroll
+    for (int a = 0; a + o < A; a += 2 * o)
+#pragma unroll
+      for (int e = 0; e < EW; ++e) acc[a][e] += acc[a + o][e];
   if constexpr (NS > 1) {
     __shared__ float red[kHeavyWarps][32][EW];
     if (ws > 0) {
 #pragma unroll
-      for (int e = 0; e < EW; ++e) red[warp][lane][e] = acc[e];
+      for (int e = 0; e < EW; ++e) red[warp][lane][e] = acc[0][e];
     }
     __syncthreads();
     if (ws > 0) return;
 #pragma unroll
     for (int e = 0; e < EW; ++e) {
       if constexpr (NS == 2)
-        acc[e] += red[warp + Tune::kParts][lane][e];
+        acc[0][e] += red[warp + Tune::kParts][lane][e];
       else
-        acc[e] = (acc[e] + red[1][lane][e]) + (red[2][lane][e] + red[3][lane][e]);
+        acc[0][e] = (acc[0][e] + red[1][lane][e]) + (red[2][lane][e] + red[3][lane][e]);
     }
   }
   const bool out = on && lane < W;
@@ -328,7 +348,7 @@ __global__ void __launch_bounds__(kHeavyWarps * 32, 4) k_spmm_heavy(const SpmmAr
     place = sp.x;
     if (out) {
 #pragma unroll
-      for (int e = 0; e < EW; ++e) __stcg(s.partial + (int64_t)it * s.ldp + e0 + e, acc[e]);
+      for (int e = 0; e < EW; ++e) __stcg(s.partial + (int64_t)it * s.ldp + e0 + e, acc[0][e]);
     }
     __threadfence();
     __syncwarp();
@@ -342,7 +362,7 @@ __global__ void __launch_bounds__(kHeavyWarps * 32, 4) k_spmm_heavy(const SpmmAr
     if (out) {
       const float* p = s.partial + (int64_t)sp.x * s.ldp + e0;
 #pragma unroll
-      for (int e = 0; e < EW; ++e) acc[e] = 0.0f;
+      for (int e = 0; e < EW; ++e) acc[0][e] = 0.0f;
       constexpr int kD = 8;  // chunks in flight
       for (unsigned i = 0; i < sp.y; i += kD) {
         float t[kD][EW];
@@ -354,14 +374,14 @@ __global__ void __launch_bounds__(kHeavyWarps * 32, 4) k_spmm_heavy(const SpmmAr
         for (int d = 0; d < kD; ++d)
           if (i + d < sp.y)
 #pragma unroll
-            for (int e = 0; e < EW; ++e) acc[e] += t[d][e];
+            for (int e = 0; e < EW; ++e) acc[0][e] += t[d][e];
       }
     }
   }
   typename Epi::State state;
   if (out) {
     const auto pre = epi.template load<EW>(r, s.e_base + e0);
-    epi.template store<EW>(r, s.e_base + e0, acc, pre, state);
+    epi.template store<EW>(r, s.e_base + e0, acc[0], pre, state);
   }
   if constexpr (Epi::State::kSums) state.put(epi.dot, place * Tune::kParts + part);
 }
@@ -606,7 +626,7 @@ __global__ void __launch_bounds__(kSpmmThreads, 4) k_spmm(const SpmmArgs<XT> s, 
     }
   }
   if constexpr (Epi::State::kSums)
-    state.put(epi.dot, s.n_heavy * HeavyTune<G>::kParts + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5));
+    state.put(epi.dot, s.n_heavy * HeavyTune<G, VAL>::kParts + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5));
   // Launched beside k_spmm_heavy, whose blocks have all started by then:
   // this launch ends after that one, so that what follows it on the stream
   // sees the rows of both.

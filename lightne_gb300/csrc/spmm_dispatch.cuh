@@ -20,7 +20,7 @@ static void spmm_launch(lne_ctx* ctx, const SpmmArgs<XT>& s, const Epi& epi, int
   *nl += 1;
 }
 
-static constexpr int kSpmmPartsMax = HeavyTune<32>::kParts;
+static constexpr int kSpmmPartsMax = HeavyTune<32, false>::kParts;
 // Blocks of the light rows of the balanced form: persistent, four per SM.
 static inline int64_t spmm_bal_blocks(const lne_ctx* ctx, const SpmmPlan& plan) {
   const int64_t want = (plan.n_items - plan.n_heavy + kSpmmWarps - 1) / kSpmmWarps;
@@ -38,7 +38,9 @@ static inline int64_t spmm_places(const lne_ctx* ctx, const SpmmPlan& plan) {
 template <typename XT, int G, bool VAL, class Epi>
 static void spmm_launch_bal(lne_ctx* ctx, const SpmmPlan& plan, const SpmmArgs<XT>& s, const Epi& epi, int* nl) {
   if (plan.n_heavy > 0) {
-    k_spmm_heavy<XT, G, VAL, Epi><<<(unsigned)plan.n_heavy, kHeavyWarps * 32, 0, ctx->stream>>>(s, epi);
+    const int64_t units = plan.n_heavy * HeavyTune<G, VAL>::kWarps;
+    k_spmm_heavy<XT, G, VAL, Epi>
+        <<<(unsigned)((units + kHeavyWarps - 1) / kHeavyWarps), kHeavyWarps * 32, 0, ctx->stream>>>(s, epi);
     *nl += 1;
   }
   if (plan.n_items == plan.n_heavy) return;

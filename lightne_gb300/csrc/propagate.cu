@@ -11,8 +11,9 @@
 // (float)(1 - mu - 1/d~_i) on the diagonal and (float)(-1/d~_i) on each
 // neighbour (the reference stores these floats in a CSR, :59-75), so
 // (M x)_i = m_i x_i + o_i * sum_{j in N(i)} x_j with the neighbour sum
-// gathered by the SpMM core.  Every half-step is one kernel whose epilogue
-// applies the recursion's axpbys while the row is in registers.
+// gathered by the SpMM core.  Every half-step is one product whose epilogue
+// applies the recursion's axpbys while the row is in registers (one kernel,
+// and a second beside it for the long rows of a graph that has some).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>

@@ -792,8 +792,16 @@ __global__ void k_trunc_log_values(const double* __restrict__ x, int64_t n, doub
 // The slots of a warp's stretch of the table are compacted into a per-warp
 // queue first (about a third of the slots are occupied), so that the
 // log evaluation runs with all 32 lanes busy.  On the dense distinct pairs
-// each thread evaluates kTruncLogPer pairs per round.
-static constexpr int kTruncLogPer = 4;
+// each thread evaluates kTruncLogPer pairs per round, and the block counts
+// rows in two tables of shared memory (a vertex's slot goes to the first
+// that asks, which a hub almost always is; the others count in global
+// memory): the hubs' global counters serialise in L2.  177M pairs of a
+// power-law graph: 9.5 ms with global counters alone (4.9 with none, 3.2 of
+// them the gathers and the logarithm), 5.7 with 2^10 slots and two pairs a
+// round, 6.1 with four; 2^12 slots take 6.4 (fewer blocks per SM, and every
+// block adds its table to the global counters at its end).
+static constexpr int kTruncLogPer = 2;
+static constexpr int kHotBits = 10;
 
 template <bool WEIGHTED>
 struct TruncLogOut {
@@ -833,7 +841,7 @@ __device__ __forceinline__ TruncLogOut<WEIGHTED> trunclog_entry(unsigned long lo
 }
 
 template <bool WEIGHTED, bool DENSE>
-__global__ void __launch_bounds__(256) k_trunclog(const Slot* __restrict__ T, uint64_t cap,
+__global__ void __launch_bounds__(256, 4) k_trunclog(const Slot* __restrict__ T, uint64_t cap,
                                                   const Vertex* __restrict__ vd, double factor, int upper,
                                                   const LogTable* __restrict__ ltab,
                                                   unsigned long long* __restrict__ rowcnt,
@@ -914,6 +922,34 @@ __global__ void __launch_bounds__(256) k_trunclog(const Slot* __restrict__ T, ui
     __shared__ unsigned wsum[8];
     __shared__ unsigned long long bbase;
     constexpr int kPer = kTruncLogPer;
+    constexpr uint32_t kFree = ~0u;  // no vertex
+    __shared__ uint32_t hot_id[2][1 << kHotBits], hot_n[2][1 << kHotBits];
+    // fewer pairs than twice the slots in a block: the tables would cost
+    // more than they save (20 us of 790 on 700K pairs)
+    const bool hot = cap >= ((uint64_t)gridDim.x << (kHotBits + 1));
+    if (hot) {
+      for (int i = threadIdx.x; i < 2 << kHotBits; i += blockDim.x) {
+        hot_id[0][i] = kFree;
+        hot_n[0][i] = 0;
+      }
+      __syncthreads();
+    }
+    auto bump = [&](int t, uint32_t id, unsigned long long* cnt) {
+      if (!hot) {
+        atomicAdd(&cnt[id], 1ULL);
+        return;
+      }
+      const uint32_t at = (id * 2654435761u) >> (32 - kHotBits);  // Fibonacci hashing
+      uint32_t who = *(volatile uint32_t*)&hot_id[t][at];
+      if (who == kFree) {
+        who = atomicCAS(&hot_id[t][at], kFree, id);
+        if (who == kFree) who = id;
+      }
+      if (who == id)
+        atomicAdd(&hot_n[t][at], 1u);
+      else
+        atomicAdd(&cnt[id], 1ULL);
+    };
     const uint64_t span = (uint64_t)blockDim.x * kPer;
     for (uint64_t b0 = (uint64_t)blockIdx.x * span; b0 < cap; b0 += (uint64_t)gridDim.x * span) {
       TruncLogOut<WEIGHTED> o[kPer];
@@ -930,8 +966,8 @@ __global__ void __launch_bounds__(256) k_trunclog(const Slot* __restrict__ T, ui
 #pragma unroll
       for (int q = 0; q < kPer; ++q) {
         if (o[q].nitem) {
-          atomicAdd(&rowcnt[o[q].u], 1ULL);
-          if (o[q].nitem == 2) atomicAdd(&lowcnt[o[q].v], 1ULL);
+          bump(0, o[q].u, rowcnt);
+          if (o[q].nitem == 2) bump(1, o[q].v, lowcnt);
           if (o[q].u == o[q].v) diag[o[q].u] = 1;
           ++kept;
           ++mine;
@@ -967,6 +1003,10 @@ __global__ void __launch_bounds__(256) k_trunclog(const Slot* __restrict__ T, ui
         }
       }
       __syncthreads();  // wsum and bbase are rewritten in the next round
+    }
+    for (int i = threadIdx.x; hot && i < 1 << kHotBits; i += blockDim.x) {
+      if (hot_n[0][i]) atomicAdd(&rowcnt[hot_id[0][i]], (unsigned long long)hot_n[0][i]);
+      if (hot_n[1][i]) atomicAdd(&lowcnt[hot_id[1][i]], (unsigned long long)hot_n[1][i]);
     }
   }
   for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); !DENSE && b < cap; b += stride) {
@@ -1653,7 +1693,9 @@ extern "C" int lne_sparsify(lne_ctx* ctx, const lne_graph* g, const lne_sparsify
   // sliced aggregation (every slot occupied)
   const Slot* tsrc = sliced ? uniq : table;
   const uint64_t tcap = sliced ? (uint64_t)h_cnt[2] : cap;
-  const unsigned tgrid = grid_for((int64_t)tcap, 256, (int64_t)ctx->num_sms * 16);
+  // dense: two rounds or more a block (each loads the logarithm's table first)
+  const unsigned tgrid = sliced ? grid_for((int64_t)tcap, 512 * kTruncLogPer, (int64_t)ctx->num_sms * 16)
+                                : grid_for((int64_t)tcap, 256, (int64_t)ctx->num_sms * 16);
   if (p->sample)
     k_trunclog<true, false><<<tgrid, 256, 0, st>>>(tsrc, tcap, g->vdata, factor, p->upper,
                                             (const LogTable*)ctx->log_table, rowcnt, lowcnt, diag, counters + 3, counters + 4,

@@ -44,3 +44,11 @@ def test_row_counts_around_a_scan(ctx, n):
     i = np.arange(n - 1)
     off, nbrs = graphs.csr_from_edges(n, i, i + 1)
     check(ctx, off, nbrs, walk_len=3, sample_ratio=0.5, tablesz=3_000_000)
+
+
+@pytest.mark.parametrize("n", [900, 1025, 5000])
+def test_row_counts_around_a_hub(ctx, n):
+    """Every pair's walk passes the hub; more vertices than the blocks' counting
+    tables have slots, and fewer."""
+    off, nbrs = graphs.star_graph(n)
+    check(ctx, off, nbrs, walk_len=4, sample_ratio=3.0, tablesz=3_000_000)

@@ -321,10 +321,8 @@ int lne_chebyshev_coefficients(int32_t order, double s, float* out);
  * (device n x dim), d_ga = dL/da (device n x dim, may be NULL), *h_dmu =
  * dL/dmu and *h_ds = dL/ds (host, may be NULL; they need d_a).  Uses
  * M^T = D~ M D~^-1, so dL/da = h - D~ sum_k c_k T_k(X) D~^-1 h with
- * h = (A + I) g; dL/ds = -sum_k c_k'(s) <V_k, D~ a> and dL/dmu =
- * sum_j e_j <M V_j, D~ a> with V_k = T_k(X) D~^-1 h and e_j the coefficients
- * of sum_k k c_k U_{k-1} in the T_j: sums over the vectors of dL/da's own
- * recursion, which the 16-bit forms run once more in FP32 for them.
+ * h = (A + I) g; dL/ds = -sum_k c_k'(s) <h, T_k a>; dL/dmu from the forward
+ * tangent T'_1 = -M a, T'_{k+1} = 2 X T'_k - T'_{k-1} - 2 M T_k.
  * The derivatives are of the real-valued map (mu, s not rounded to float).
  */
 int lne_propagate_adjoint(lne_ctx* ctx, const lne_graph* g, const lne_propagate_params* p, const float* d_a,

@@ -197,93 +197,38 @@ __device__ __forceinline__ float coef_dt(const float4* __restrict__ coef, int64_
   return __ldg(reinterpret_cast<const float*>(coef + r) + 2);
 }
 
-// <V_k, D~ a> sums of the adjoint's parameter gradients, taken in the
-// epilogues of the recursion: per lane in FP32 over the rows of its warp (or
-// one long row), then in FP64, each warp and each long row (which any block
-// may take) into a place of its own; k_dot_sum adds the places in order.
-struct DotOut {
-  const float* __restrict__ a = nullptr;  // the input embedding (n x ld)
-  int64_t ld = 0;
-  double* pv = nullptr;                   // <V_k, D~ a> by place
-  double* pw = nullptr;                   // <M V_k, D~ a>, or null
-};
-struct DotState {
-  static constexpr bool kSums = true;
-  float v = 0.0f, w = 0.0f;
-  __device__ __forceinline__ static double warp_sum(float x) {
-    double d = (double)x;
-    for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(kFull, d, o);
-    return d;
-  }
-  // Adds the warp's sums (the column slabs of a row follow one another).
-  __device__ __forceinline__ void put(const DotOut& o, uint32_t place) const {
-    const double dv = warp_sum(v), dw = warp_sum(w);
-    if ((threadIdx.x & 31) == 0) {
-      o.pv[place] += dv;
-      if (o.pw) o.pw[place] += dw;
-    }
-  }
-};
-
-// Adds a row's <x, D~ a> to the sums.
-template <int N>
-__device__ __forceinline__ void dot_v(const DotOut& o, const float4* __restrict__ coef, int64_t r, int e0,
-                                      const float (&x)[N], DotState& st) {
-  float a[N];
-  load_f32<N>(o.a, o.ld, r, e0, a);
-  const float dt = coef_dt(coef, r);
-#pragma unroll
-  for (int i = 0; i < N; ++i) st.v = fmaf(x[i], dt * a[i], st.v);
-}
-
 // Epilogues of the SpMM (spmm_core.cuh): load() fetches the row's operands
 // ahead of the gathers, store() applies the recursion to the finished sums.
-// With DOTS they also add the parameter gradients' sums.
 
 // tmp = M x: out = m_i x_i + o_i acc (operand x of type XT); FP32 and/or
-// 16-bit outputs.  DOTS: <x, D~ a> and <M x, D~ a>.
-template <typename XT, bool DOTS = false>
+// 16-bit outputs.
+template <typename XT>
 struct EpiApplyM {
   using HT = typename ShadowOf<XT>::type;
-  using State = typename std::conditional<DOTS, DotState, NoState>::type;
   const float4* __restrict__ coef;
   const XT* __restrict__ X;  // the operand (diagonal term)
   int64_t ld;
   float* __restrict__ out_f;
   HT* __restrict__ out_b;
-  DotOut dot;
   template <int N>
   struct Pre {
     float2 c;
     RawRow<XT, N> x;
-    float a[DOTS ? N : 1], dt;
   };
   template <int N>
   __device__ __forceinline__ Pre<N> load(int64_t r, int e0) const {
     Pre<N> q;
     q.c = coef_mo(coef, r);
     q.x.load(X, ld, r, e0);
-    if constexpr (DOTS) {
-      q.dt = coef_dt(coef, r);
-      load_f32<N>(dot.a, dot.ld, r, e0, q.a);
-    }
     return q;
   }
   template <int N>
-  __device__ __forceinline__ void store(int64_t r, int e0, const float (&a)[N], const Pre<N>& q, State& st) const {
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&a)[N], const Pre<N>& q) const {
     float y[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) y[i] = fmaf(q.c.x, q.x.at(i), q.c.y * a[i]);
     if (out_f) store_f32<N>(out_f, ld, r, e0, y);
     if (out_b) store_16<HT, N>(out_b, ld, r, e0, y);
-    if constexpr (DOTS) {
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        const float da = q.dt * q.a[i];
-        st.v = fmaf(q.x.at(i), da, st.v);
-        st.w = fmaf(y[i], da, st.w);
-      }
-    }
   }
 };
 
@@ -314,12 +259,11 @@ struct FinalOut {
 };
 
 // First order: Lx1 = 0.5 M tmp - x;  conv = c0 x + c1 Lx1 (conv may be null:
-// no sum is kept);  or the final vector when order <= 2.  x = x_scale A.
-// DOTS: <Lx1, D~ a>.
-template <typename XT, bool DOTS = false>
+// the tangent pass keeps no sum);  or the final vector when order <= 2.
+// x = x_scale A.
+template <typename XT>
 struct EpiFirst {
   using HT = typename ShadowOf<XT>::type;
-  using State = typename std::conditional<DOTS, DotState, NoState>::type;
   const float4* __restrict__ coef;
   const XT* __restrict__ T;        // tmp (operand)
   const float* __restrict__ A;     // x (FP32)
@@ -330,7 +274,6 @@ struct EpiFirst {
   int64_t ld;
   float c0, c1;
   float x_scale;
-  DotOut dot;
   template <int N>
   struct Pre {
     float2 c;
@@ -346,7 +289,7 @@ struct EpiFirst {
     return q;
   }
   template <int N>
-  __device__ __forceinline__ void store(int64_t r, int e0, const float (&acc)[N], const Pre<N>& q, State& st) const {
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&acc)[N], const Pre<N>& q) const {
     float l1[N], cv[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -355,7 +298,6 @@ struct EpiFirst {
       l1[i] = fmaf(0.5f, mt, -a);
       cv[i] = fmaf(c1, l1[i], c0 * a);
     }
-    if constexpr (DOTS) dot_v<N>(dot, coef, r, e0, l1, st);
     if (L1) store_state<XT, N>(L1, ld, r, e0, l1);
     if (L1b) store_16<HT, N>(L1b, ld, r, e0, l1);
     if (fin.base)
@@ -369,11 +311,11 @@ struct EpiFirst {
 // null);  or the final vector on the last order.  Lx0 = l0_scale L0.
 // The sum is read and written every second order: `skip` leaves conv alone
 // and the next order adds ck_prev Lx1 (the skipped order's vector) as well.
-// DOTS (the last order): <Lx2, D~ a>.
-template <typename XT, bool DOTS = false>
+// TAN (the tangent pass): Lx2 = M tmp - Lx0 - 2 Lx1 - 2 extra, where L0 ==
+// null means a zero Lx0.
+template <typename XT, bool TAN = false>
 struct EpiStep {
   using HT = typename ShadowOf<XT>::type;
-  using State = typename std::conditional<DOTS, DotState, NoState>::type;
   const float4* __restrict__ coef;
   const XT* __restrict__ T;
   const float* __restrict__ L0;
@@ -387,34 +329,40 @@ struct EpiStep {
   float ck_prev = 0.0f;
   bool skip = false;
   float l0_scale = 1.0f;
-  DotOut dot;
+  const float* __restrict__ extra = nullptr;
   template <int N>
   struct Pre {
     float2 c;
     RawRow<XT, N> t;
-    float l0[N], l1[N], cv[N];
+    float l0[N], l1[N], cv[N], ex[TAN ? N : 1];
   };
   template <int N>
   __device__ __forceinline__ Pre<N> load(int64_t r, int e0) const {
     Pre<N> q;
     q.c = coef_mo(coef, r);
     q.t.load(T, ld, r, e0);
-    load_f32<N>(L0, ld, r, e0, q.l0);
+    if (!TAN || L0) {
+      load_f32<N>(L0, ld, r, e0, q.l0);
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) q.l0[i] = 0.0f;
+    }
     load_f32<N>(L1, ld, r, e0, q.l1);
+    if constexpr (TAN) load_f32<N>(extra, ld, r, e0, q.ex);
     if (conv && !skip) load_f32<N>(conv, ld, r, e0, q.cv);
     return q;
   }
   template <int N>
-  __device__ __forceinline__ void store(int64_t r, int e0, const float (&acc)[N], const Pre<N>& q, State& st) const {
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&acc)[N], const Pre<N>& q) const {
     float l2[N], cv[N];
     const bool sum = conv && !skip;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       const float mt = fmaf(q.c.x, q.t.at(i), q.c.y * acc[i]);
       l2[i] = fmaf(-2.0f, q.l1[i], fmaf(-l0_scale, q.l0[i], mt));
+      if constexpr (TAN) l2[i] = fmaf(-2.0f, q.ex[i], l2[i]);
       cv[i] = fmaf(ck, l2[i], sum ? fmaf(ck_prev, q.l1[i], q.cv[i]) : 0.0f);
     }
-    if constexpr (DOTS) dot_v<N>(dot, coef, r, e0, l2, st);
     if (fin.base) {
       fin.template apply<N>(r, e0, ld, coef, cv);
     } else {
@@ -430,7 +378,6 @@ struct EpiStep {
 // FP16 form; 1 otherwise); vec: Y's rows are whole 16-byte vectors.
 template <typename XT>
 struct EpiAPlusI {
-  using State = NoState;
   const XT* __restrict__ X;
   int64_t ld;
   float* __restrict__ Y;
@@ -449,7 +396,7 @@ struct EpiAPlusI {
     return q;
   }
   template <int N>
-  __device__ __forceinline__ void store(int64_t r, int e0, const float (&acc)[N], const Pre<N>& q, State&) const {
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&acc)[N], const Pre<N>& q) const {
     float o[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) o[i] = out_scale * (q.x.at(i) + acc[i]);
@@ -464,12 +411,11 @@ struct EpiAPlusI {
   }
 };
 
-// Adjoint start: h = (A + I) g (H may be null), g = g_scale times the operand
-// (a power of two);  b = h / d~_i (FP32 and 16-bit copy).
+// Adjoint start: h = (A + I) g, g = g_scale times the operand (a power of
+// two);  b = h / d~_i (FP32, may be null, and 16-bit copy).
 template <typename XT>
 struct EpiAdjInit {
   using HT = typename ShadowOf<XT>::type;
-  using State = NoState;
   const float4* __restrict__ coef;
   const XT* __restrict__ G;
   int64_t ld;
@@ -490,15 +436,15 @@ struct EpiAdjInit {
     return q;
   }
   template <int N>
-  __device__ __forceinline__ void store(int64_t r, int e0, const float (&acc)[N], const Pre<N>& q, State&) const {
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&acc)[N], const Pre<N>& q) const {
     float h[N], b[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       h[i] = g_scale * (q.g.at(i) + acc[i]);
       b[i] = h[i] * q.inv_dt;
     }
-    if (H) store_f32<N>(H, ld, r, e0, h);
-    store_f32<N>(Bf, ld, r, e0, b);
+    store_f32<N>(H, ld, r, e0, h);
+    if (Bf) store_f32<N>(Bf, ld, r, e0, b);
     if (Bb) store_16<HT, N>(Bb, ld, r, e0, b);
   }
 };
@@ -572,11 +518,21 @@ __global__ void k_amax_partial(const float* __restrict__ x, int64_t total, float
   }
 }
 
-// out[slot] = sum of part[slot][0 .. count) in a fixed order (one block per slot).
-__global__ void k_dot_sum(const double* __restrict__ part, int64_t count, double* __restrict__ out) {
-  const double* p = part + (int64_t)blockIdx.x * count;
-  double d = 0.0;
-  for (int64_t t = threadIdx.x; t < count; t += blockDim.x) d += p[t];
+// y = alpha x.
+__global__ void k_scale_copy(const float* __restrict__ x, int64_t total, float alpha, float* __restrict__ y) {
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x)
+    y[t] = alpha * x[t];
+}
+
+// <h, x> partial sums: FP32 within a thread, FP64 across threads, one
+// value per block (summed in block order on the host).
+static constexpr int kDotBlocks = 1024;
+__global__ void k_dot_partial(const float* __restrict__ h, const float* __restrict__ x, int64_t total,
+                              double* __restrict__ out) {
+  float s = 0.0f;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x)
+    s = fmaf(h[t], x[t], s);
+  double d = (double)s;
   for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(kFull, d, o);
   __shared__ double ws[32];
   if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = d;
@@ -605,19 +561,6 @@ struct Bufs {
   }
 };
 
-// The parameter gradients' sums of one recursion: slot k holds the parts of
-// <V_k, D~ a>, slot K + k those of <M V_k, D~ a>.
-struct Dots {
-  const float* a = nullptr;  // n x ld
-  int64_t ld = 0;
-  double* part = nullptr;    // [2 K][places]
-  int64_t places = 0;
-  int K = 0;
-  DotOut slots(int k, bool with_m) const {
-    return DotOut{a, ld, part + (int64_t)k * places, with_m ? part + (int64_t)(K + k) * places : nullptr};
-  }
-};
-
 // Shared state of one filter evaluation.
 template <typename XT>
 struct Filter {
@@ -640,26 +583,22 @@ struct Filter {
     return spmm_run<XT, false>(ctx, g->plan, g->nbrs, nullptr, X, ld, ld, epi, launches, 0, work);
   }
 
-  int apply_m(const XT* X, float* out_f, HT* out_b, const Dots* dots, int k) {
-    if constexpr (!k16) {
-      if (dots) return spmm(X, EpiApplyM<XT, true>{coef, X, ld, out_f, out_b, dots->slots(k, true)});
-    }
-    return spmm(X, EpiApplyM<XT>{coef, X, ld, out_f, out_b, DotOut()});
+  int apply_m(const XT* X, float* out_f, HT* out_b) {
+    return spmm(X, EpiApplyM<XT>{coef, X, ld, out_f, out_b});
   }
 
   // The Chebyshev filter on x = x_scale xf (operand copy xb):
   // fin.base_scale fin.base - scale * sum_k c_k T_k(X) x written as `fin`
-  // says.  With a null fin.base only the recursion runs, for its dots (FP32
-  // operands).
+  // says.
   int run(const float* xf, const HT* xb, float x_scale, int order, const std::vector<float>& c,
-          const FinalOut<HT>& fin, const Dots* dots = nullptr) {
+          const FinalOut<HT>& fin) {
     int rc;
     float *conv = nullptr, *Tf = nullptr;
     HT* Tb = nullptr;
     float* ring[3] = {nullptr, nullptr, nullptr};
     HT* ringb[3] = {nullptr, nullptr, nullptr};
     const int nring = order > 2 ? 3 : 0;
-    if (order > 2 && fin.base && (rc = B->get(&conv, sz(), "conv"))) return rc;
+    if (order > 2 && (rc = B->get(&conv, sz(), "conv"))) return rc;
     for (int i = 0; i < nring; ++i) {
       if ((rc = B->get(&ring[i], sz(), "Chebyshev vector"))) return rc;
       if (k16 && (rc = B->get(&ringb[i], sz(), "Chebyshev vector 16-bit"))) return rc;
@@ -671,19 +610,10 @@ struct Filter {
     }
     const XT* X0 = op(xf, xb);
     const XT* Tx = k16 ? (const XT*)Tb : (const XT*)Tf;
-    if ((rc = apply_m(X0, k16 ? nullptr : Tf, k16 ? Tb : nullptr, dots, 0))) return rc;  // tmp = M x
+    if ((rc = apply_m(X0, k16 ? nullptr : Tf, k16 ? Tb : nullptr))) return rc;  // tmp = M x
     {
-      // the sums of the last vector are taken as it is formed, those of the
-      // others when M is applied to them
-      const bool last = order <= 2;
-      const FinalOut<HT> fo = last ? fin : FinalOut<HT>();
-      if constexpr (!k16) {
-        if (last && dots) {
-          EpiFirst<XT, true> epi{coef, Tx, xf, ring[0], ringb[0], conv, fo, ld, c[0], c[1], x_scale, dots->slots(1, false)};
-          return spmm(Tx, epi);
-        }
-      }
-      EpiFirst<XT> epi{coef, Tx, xf, ring[0], ringb[0], conv, fo, ld, c[0], c[1], x_scale, DotOut()};
+      const FinalOut<HT> fo = order <= 2 ? fin : FinalOut<HT>();
+      EpiFirst<XT> epi{coef, Tx, xf, ring[0], ringb[0], conv, fo, ld, c[0], c[1], x_scale};
       if ((rc = spmm(Tx, epi))) return rc;
     }
     const float* l0 = xf;
@@ -691,7 +621,7 @@ struct Filter {
     int j1 = 0;
     for (int k = 2; k < order; ++k) {
       const int j2 = (j1 + 1) % 3;
-      if ((rc = apply_m(op(ring[j1], ringb[j1]), k16 ? nullptr : Tf, k16 ? Tb : nullptr, dots, k - 1))) return rc;
+      if ((rc = apply_m(op(ring[j1], ringb[j1]), k16 ? nullptr : Tf, k16 ? Tb : nullptr))) return rc;
       const bool last = k == order - 1;
       const FinalOut<HT> fo = last ? fin : FinalOut<HT>();
       // conv is updated on odd orders (and on the last): even orders are
@@ -700,14 +630,7 @@ struct Filter {
       const float ck_prev = (k % 2 == 1) ? c[k - 1] : 0.0f;
       float* out = last ? nullptr : ring[j2];
       HT* outb = last ? nullptr : ringb[j2];
-      if constexpr (!k16) {
-        if (last && dots) {
-          EpiStep<XT, true> epi{coef, Tx,   l0,      ring[j1], out,      outb, conv, fo,
-                                ld,   c[k], ck_prev, skip,     l0_scale, dots->slots(k, false)};
-          return spmm(Tx, epi);
-        }
-      }
-      EpiStep<XT> epi{coef, Tx, l0, ring[j1], out, outb, conv, fo, ld, c[k], ck_prev, skip, l0_scale, DotOut()};
+      EpiStep<XT> epi{coef, Tx, l0, ring[j1], out, outb, conv, fo, ld, c[k], ck_prev, skip, l0_scale};
       if ((rc = spmm(Tx, epi))) return rc;
       l0 = ring[j1];
       l0_scale = 1.0f;
@@ -868,39 +791,97 @@ void chebyshev_coeffs_ds(int order, double s, std::vector<double>& dc) {
     dc[k] = ((k & 1) ? -1.0 : 1.0) * (bessel_i(k - 1, sf) + bessel_i(k + 1, sf));
 }
 
-// dL/dmu and dL/ds (P3) from the sums the adjoint's recursion leaves:
-// with f(M) = sum_k c_k T_k(X), X = M^2/2 - I, L = <h, a - f(M) a>:
-//   dL/ds  = -sum_k c_k'(s) <h, T_k a>,
-//   dL/dmu = <h, f'(M) a>  (dM/dmu = -I),
-//   f'(M)  = sum_k k c_k U_{k-1}(X) M = sum_j e_j T_j(X) M,
-// U_n being 2 (T_n + T_{n-2} + ...), T_0 counted once.  All of these are
-// polynomials in M, and M^T = D~ M D~^-1, so with V_k = T_k(X) D~^-1 h (the
-// vectors the adjoint's recursion forms anyway)
-//   <h, T_k a> = <V_k, D~ a>,  <h, T_j M a> = <M V_j, D~ a>:
-// no recursion on a is run (the tangent recursion this replaces took 36
-// products with the graph per gradient; these sums take none of their own).
-int param_grads(lne_ctx* ctx, const lne_propagate_params* p, const std::vector<float>& c, const Dots& dots,
-                Bufs& B, int* launches, double hscale, double* h_dmu, double* h_ds) {
-  const int K = dots.K;
-  double* d_sum = nullptr;
+// dL/dmu and dL/ds in FP32 (P3): the forward pass on a with the mu-tangent
+// T'_1 = -M a, T'_{k+1} = M(M T'_k) - 2 T'_k - T'_{k-1} - 2 M T_k, and the
+// dots <h, T_k a>, <h, T'_k> (h = hscale^-1 H): dL/ds = -sum_k c_k'(s)
+// <h, T_k a>, dL/dmu = -sum_k c_k <h, T'_k>.
+//
+// The same gradients as sums over the vectors V_k = T_k(X) D~^-1 h that
+// dL/da's recursion forms anyway (<V_k, D~ a>, <M V_j, D~ a>) take none of
+// these products, but are less exact: the row of a hub is an FP32 sum over its
+// neighbours, weighted by its d~.  At 6,000 vertices with a hub of 5,500
+// neighbours and 128 columns that form was off by 7.1e-7 (mu) and 6.0e-7 (s)
+// of |h a|, root mean square of 8 draws, this one by 1.3e-7 and 2.7e-7; at
+// 1.14M vertices and 128 columns that form's relative errors were up to 40
+// times this one's (1.7e-7 against 4.8e-9 in dL/dmu of one draw).
+int param_grads(lne_ctx* ctx, Filter<float>& F, const lne_propagate_params* p, const std::vector<float>& c,
+                const float* H, const float* d_a, double hscale, double* h_dmu, double* h_ds) {
+  const int64_t n = F.n, ld = F.ld;
+  const int d = (int)p->dim;
+  const int order = p->order;
+  const size_t sz = (size_t)n * ld;
+  const int64_t total = (int64_t)sz;
+  cudaStream_t st = ctx->stream;
+  Bufs& B = *F.B;
+  int& launches = *F.launches;
   int rc;
-  if ((rc = B.get(&d_sum, (size_t)2 * K, "dot sums"))) return rc;
-  k_dot_sum<<<2 * K, 256, 0, ctx->stream>>>(dots.part, dots.places, d_sum);
-  *launches += 1;
-  std::vector<double> h((size_t)2 * K);
-  LNE_CUDA_TRY(cudaMemcpyAsync(h.data(), d_sum, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, ctx->stream));
-  LNE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  std::vector<double> dc;
-  chebyshev_coeffs_ds(p->order, p->s, dc);
-  double gs = 0.0, gmu = 0.0;
-  for (int k = 0; k < K; ++k) gs -= dc[k] * h[k];
-  for (int j = 0; j + 1 < K; ++j) {
-    double e = 0.0;
-    for (int k = j + 1; k < K; k += 2) e += (double)k * (double)c[k];
-    gmu += (j == 0 ? 1.0 : 2.0) * e * h[K + j];
+  const int K = order > 2 ? order : 2;
+  double* partial = nullptr;
+  if ((rc = B.get(&partial, (size_t)2 * K * kDotBlocks, "dot partials"))) return rc;
+  LNE_CUDA_TRY(cudaMemsetAsync(partial, 0, sizeof(double) * 2 * K * kDotBlocks, st));
+  auto dot = [&](int slot, const float* x) {
+    k_dot_partial<<<kDotBlocks, 256, 0, st>>>(H, x, total, partial + (int64_t)slot * kDotBlocks);
+    launches += 1;
+  };
+  float *Tm = nullptr, *Tpm = nullptr;  // M T_k, M T'_k
+  float* T[3];
+  float* Tp[3];
+  if ((rc = B.get(&Tm, sz, "M T")) || (rc = B.get(&Tpm, sz, "M T'"))) return rc;
+  for (int i = 0; i < 3; ++i)
+    if ((rc = B.get(&T[i], sz, "T")) || (rc = B.get(&Tp[i], sz, "T'"))) return rc;
+  const unsigned pg = (unsigned)std::min<int64_t>((total + 255) / 256, (int64_t)ctx->num_sms * 32);
+  const float* A = d_a;
+  if (!rows_direct(d_a, d, ld)) {
+    float* Acopy = nullptr;
+    if ((rc = B.get(&Acopy, sz, "a"))) return rc;
+    k_pad_copy<__nv_bfloat16><<<pg, 256, 0, st>>>(d_a, n, d, 1.0f, Acopy, ld, nullptr);
+    launches += 1;
+    A = Acopy;
   }
-  if (h_ds) *h_ds = gs * hscale;
-  if (h_dmu) *h_dmu = gmu * hscale;
+  dot(0, A);  // <h, T_0>
+  // tmp = M a;  T_1 = 0.5 M tmp - a;  T'_1 = -tmp
+  const FinalOut<__nv_bfloat16> none;
+  if ((rc = F.apply_m(A, Tm, nullptr))) return rc;
+  if ((rc = F.spmm(Tm, EpiFirst<float>{F.coef, Tm, A, T[0], nullptr, nullptr, none, ld, 0.0f, 0.0f, 1.0f}))) return rc;
+  k_scale_copy<<<pg, 256, 0, st>>>(Tm, total, -1.0f, Tp[0]);
+  launches += 1;
+  dot(1, T[0]);
+  dot(K + 1, Tp[0]);
+  const float* t0 = A;         // T_{k-1}
+  const float* tp0 = nullptr;  // T'_{k-1} (T'_0 = 0)
+  int j1 = 0;
+  for (int k = 1; k + 1 < order; ++k) {
+    const int j2 = (j1 + 1) % 3;
+    // tmp = M T_k; T_{k+1} = M tmp - 2 T_k - T_{k-1}
+    if ((rc = F.apply_m(T[j1], Tm, nullptr))) return rc;
+    if ((rc = F.spmm(Tm, EpiStep<float>{F.coef, Tm, t0, T[j1], T[j2], nullptr, nullptr, none, ld, 0.0f}))) return rc;
+    // tmp' = M T'_k; T'_{k+1} = M tmp' - 2 T'_k - T'_{k-1} - 2 M T_k
+    if ((rc = F.apply_m(Tp[j1], Tpm, nullptr))) return rc;
+    if ((rc = F.spmm(Tpm, EpiStep<float, true>{F.coef, Tpm, tp0, Tp[j1], Tp[j2], nullptr, nullptr, none, ld, 0.0f, 0.0f,
+                                               false, 1.0f, Tm})))
+      return rc;
+    dot(k + 1, T[j2]);
+    dot(K + k + 1, Tp[j2]);
+    t0 = T[j1];
+    tp0 = Tp[j1];
+    j1 = j2;
+  }
+  std::vector<double> hp((size_t)2 * K * kDotBlocks);
+  LNE_CUDA_TRY(cudaMemcpyAsync(hp.data(), partial, sizeof(double) * hp.size(), cudaMemcpyDeviceToHost, st));
+  LNE_CUDA_TRY(cudaStreamSynchronize(st));
+  std::vector<double> dots(2 * K, 0.0);
+  for (int sidx = 0; sidx < 2 * K; ++sidx) {
+    for (int b = 0; b < kDotBlocks; ++b) dots[sidx] += hp[(size_t)sidx * kDotBlocks + b];
+    dots[sidx] *= hscale;
+  }
+  std::vector<double> dc;
+  chebyshev_coeffs_ds(order, p->s, dc);
+  // only the terms the forward filter uses: k < max(order, 2)
+  double gs = 0.0, gmu = 0.0;
+  for (int k = 0; k < K; ++k) gs -= dc[k] * dots[k];
+  for (int k = 1; k < K; ++k) gmu -= (double)c[k] * dots[K + k];
+  if (h_ds) *h_ds = gs;
+  if (h_dmu) *h_dmu = gmu;
   return LNE_OK;
 }
 
@@ -927,7 +908,7 @@ int adjoint_impl(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, cons
   const size_t sz = (size_t)n * ld;
   const bool params = h_dmu || h_ds;
   // the FP16 form runs on a scaled output gradient sg * g (dL/da is linear
-  // in g; the FP32 parameter-gradient pass unscales its sums by 1 / sg)
+  // in g; the FP32 parameter-gradient pass unscales its dots by 1 / sg)
   float sg = 1.0f;
   if ((rc = input_scale<XT>(ctx, d_gy, n * d, B, &launches, &sg))) return rc;
   // g is read in place where its rows are whole 16-byte vectors
@@ -948,40 +929,27 @@ int adjoint_impl(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, cons
     launches += 1;
   }
   const float* G = g_direct ? d_gy : Gcopy;  // (Gcopy holds sg * g)
-  // the parameter gradients' sums
-  Dots dots;
-  if (params) {
-    dots.K = order > 2 ? order : 2;
-    dots.places = spmm_places(ctx, g->plan);
-    if ((rc = B.get(&dots.part, (size_t)2 * dots.K * dots.places, "dot partials"))) return rc;
-    LNE_CUDA_TRY(cudaMemsetAsync(dots.part, 0, sizeof(double) * 2 * dots.K * dots.places, st));
-    dots.ld = ld;
-    dots.a = d_a;
-    if (!rows_direct(d_a, d, ld)) {
-      float* Acopy = nullptr;
-      if ((rc = B.get(&Acopy, sz, "a"))) return rc;
-      k_pad_copy<__nv_bfloat16><<<pg, 256, 0, st>>>(d_a, n, d, 1.0f, Acopy, ld, nullptr);
-      launches += 1;
-      dots.a = Acopy;
-    }
-  }
-  if (k16 && params) {
-    // The parameter gradients run in FP32 in every form: they are sums over
-    // the orders whose terms cancel, so 16-bit gathers would cost them far
-    // more relative accuracy than they cost dL/da.  The 16-bit forms run an
-    // FP32 recursion for them, before dL/da is written.
-    Filter<float> F32{ctx, g, n, ld, F.coef, &launches, &B, &work};
-    float* B32 = nullptr;
-    if ((rc = B.get(&B32, sz, "b fp32"))) return rc;
-    EpiAdjInit<float> epi{F.coef, G, ld, nullptr, B32, nullptr, g_direct ? sg : 1.0f};
-    if ((rc = F32.spmm(G, epi))) return rc;
-    if ((rc = F32.run(B32, nullptr, 1.0f, order, c, FinalOut<__nv_bfloat16>(), &dots))) return rc;
-  }
   // h = (A + I) g, b = D~^-1 h
   {
     const XT* Gx = F.op(G, Gb);
     EpiAdjInit<XT> epi{F.coef, Gx, ld, H, Bf, Bb, 1.0f};
     if ((rc = F.spmm(Gx, epi))) return rc;
+  }
+  if (params) {
+    // The parameter gradients run in FP32 in every form: they are sums over
+    // the orders whose terms cancel, so 16-bit gathers would cost them far
+    // more relative accuracy than they cost dL/da.  The 16-bit forms first
+    // form an FP32 h = (A + I) g from the FP32 (scaled) g.  They read a, so
+    // they come before dL/da is written.
+    Filter<float> F32{ctx, g, n, ld, F.coef, &launches, &B, &work};
+    const float* H32 = H;
+    if (k16) {
+      float* H2 = nullptr;
+      if ((rc = B.get(&H2, sz, "h fp32"))) return rc;
+      if ((rc = F32.spmm(G, EpiAdjInit<float>{F.coef, G, ld, H2, nullptr, nullptr, g_direct ? sg : 1.0f}))) return rc;
+      H32 = H2;
+    }
+    if ((rc = param_grads(ctx, F32, p, c, H32, d_a, 1.0 / (double)sg, h_dmu, h_ds))) return rc;
   }
   // grad a = h - D~ sum_k c_k T_k(X) b      (M^T = D~ M D~^-1)
   const bool out_direct = d_ga && rows_direct(d_ga, d, ld);
@@ -992,13 +960,10 @@ int adjoint_impl(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, cons
   fin.scale_dt = true;
   fin.out = out_direct ? d_ga : GA;
   fin.out_scale = out_direct ? 1.0f / sg : 1.0f;
-  if ((rc = F.run(Bf, Bb, 1.0f, order, c, fin, !k16 && params ? &dots : nullptr))) return rc;
+  if ((rc = F.run(Bf, Bb, 1.0f, order, c, fin))) return rc;
   if (d_ga && !out_direct) {
     k_unpad_copy<<<pg, 256, 0, st>>>(GA, ld, n, d, 1.0f / sg, d_ga);
     launches += 1;
-  }
-  if (params) {
-    if ((rc = param_grads(ctx, p, c, dots, B, &launches, 1.0 / (double)sg, h_dmu, h_ds))) return rc;
   }
   cudaEventRecord(ev.e[1], st);
   LNE_CUDA_TRY(cudaEventSynchronize(ev.e[1]));

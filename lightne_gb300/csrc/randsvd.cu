@@ -58,7 +58,6 @@ struct EpiStore {
   int d;
   bool add;
   float scale = 1.0f;
-  using State = NoState;
   template <int N>
   using Pre = NoPre;
   template <int N>
@@ -66,7 +65,7 @@ struct EpiStore {
     return NoPre();
   }
   template <int N>
-  __device__ __forceinline__ void store(int64_t r, int e0, const float (&a)[N], const NoPre&, NoState&) const {
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&a)[N], const NoPre&) const {
     float* y = Y + r * ldy + e0;
 #pragma unroll
     for (int i = 0; i < N; ++i)

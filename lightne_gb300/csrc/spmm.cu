@@ -216,7 +216,6 @@ struct EpiAxpby {
   int64_t ldy;
   int d;
   bool add;
-  using State = NoState;
   template <int N>
   using Pre = NoPre;
   template <int N>
@@ -224,7 +223,7 @@ struct EpiAxpby {
     return NoPre();
   }
   template <int N>
-  __device__ __forceinline__ void store(int64_t r, int e0, const float (&a)[N], const NoPre&, NoState&) const {
+  __device__ __forceinline__ void store(int64_t r, int e0, const float (&a)[N], const NoPre&) const {
     float* y = Y + r * ldy + e0;
 #pragma unroll
     for (int i = 0; i < N; ++i) {

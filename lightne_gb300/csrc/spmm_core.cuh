@@ -35,11 +35,8 @@ namespace lne {
 
 static constexpr unsigned kFull = 0xffffffffu;
 
-// An epilogue without operands to load ahead, and without sums over rows.
+// An epilogue without operands to load ahead.
 struct NoPre {};
-struct NoState {
-  static constexpr bool kSums = false;
-};
 
 // Row ranges of a sparse operator, from which a work list is built.
 struct CsrRows {  // explicit CSR: int64 row_ptr
@@ -341,11 +338,9 @@ __global__ void __launch_bounds__(kHeavyWarps * 32, 4) k_spmm_heavy(const SpmmAr
   }
   const bool out = on && lane < W;
   const int e0 = q * EW;
-  uint32_t place = it;
   const uint2 sp = it < s.n_big ? __ldg(s.span + it) : make_uint2(it, 1);
   if (sp.y > 1) {
     // a chunk: the warp that completes its row's last one adds them, in order
-    place = sp.x;
     if (out) {
 #pragma unroll
       for (int e = 0; e < EW; ++e) __stcg(s.partial + (int64_t)it * s.ldp + e0 + e, acc[0][e]);
@@ -378,12 +373,10 @@ __global__ void __launch_bounds__(kHeavyWarps * 32, 4) k_spmm_heavy(const SpmmAr
       }
     }
   }
-  typename Epi::State state;
   if (out) {
     const auto pre = epi.template load<EW>(r, s.e_base + e0);
-    epi.template store<EW>(r, s.e_base + e0, acc[0], pre, state);
+    epi.template store<EW>(r, s.e_base + e0, acc[0], pre);
   }
-  if constexpr (Epi::State::kSums) state.put(epi.dot, place * Tune::kParts + part);
 }
 
 // Every item to a warp, or (BAL) the rows of at most warp_max entries.
@@ -413,8 +406,6 @@ __global__ void __launch_bounds__(kSpmmThreads, 4) k_spmm(const SpmmArgs<XT> s, 
     static_assert(VPL == 1 && (G & (G - 1)) == 0, "the balanced form has one vector per lane");
     it += s.n_heavy;
   }
-  static_assert(BAL || !Epi::State::kSums, "sums over rows are taken by the balanced form");
-  typename Epi::State state;
   const uint4* items = reinterpret_cast<const uint4*>(s.items);
   const uint4 none = make_uint4(0, 0, 0, 0);
   uint4 nxt = it < s.n_items ? __ldg(items + it) : none;
@@ -572,7 +563,7 @@ __global__ void __launch_bounds__(kSpmmThreads, 4) k_spmm(const SpmmArgs<XT> s, 
           const int ch = gl + G * k;
           if (ch >= s.C) continue;
           if (!kHoist) pre[k] = epi.template load<N>(r, s.e_base + ch * E + e_lane);
-          epi.template store<N>(r, s.e_base + ch * E + e_lane, sum[k], pre[k], state);
+          epi.template store<N>(r, s.e_base + ch * E + e_lane, sum[k], pre[k]);
         }
       }
     } else {
@@ -619,14 +610,12 @@ __global__ void __launch_bounds__(kSpmmThreads, 4) k_spmm(const SpmmArgs<XT> s, 
               }
             }
           }
-          epi.template store<4>(r, s.e_base + q, t, fin, state);
+          epi.template store<4>(r, s.e_base + q, t, fin);
         }
         __syncwarp();
       }
     }
   }
-  if constexpr (Epi::State::kSums)
-    state.put(epi.dot, s.n_heavy * HeavyTune<G, VAL>::kParts + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5));
   // Launched beside k_spmm_heavy, whose blocks have all started by then:
   // this launch ends after that one, so that what follows it on the stream
   // sees the rows of both.

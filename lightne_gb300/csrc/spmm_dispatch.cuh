@@ -26,11 +26,6 @@ static inline int64_t spmm_bal_blocks(const lne_ctx* ctx, const SpmmPlan& plan) 
   const int64_t want = (plan.n_items - plan.n_heavy + kSpmmWarps - 1) / kSpmmWarps;
   return std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->num_sms * 4));
 }
-// Places of the sums an epilogue takes over the rows: one per part of a
-// heavy item, one per warp.
-static inline int64_t spmm_places(const lne_ctx* ctx, const SpmmPlan& plan) {
-  return plan.n_heavy * kSpmmPartsMax + spmm_bal_blocks(ctx, plan) * kSpmmWarps;
-}
 
 // The heavy rows, and the light rows beside them (programmatic dependent
 // launch: the second kernel starts once the first one's blocks all have, and
@@ -188,7 +183,7 @@ static int spmm_run(lne_ctx* ctx, const SpmmPlan& plan, const uint32_t* col, con
       else
         spmm_launch_bal<XT, 32, VAL>(ctx, plan, s, epi, &nl);
     } else if (nine) {
-      // E == 4 rows have no 9-lane layout, and sums over rows none either
+      // E == 4 rows have no 9-lane layout
       if constexpr (E == 8) spmm_launch<XT, 9, 2, VAL>(ctx, s, epi, &nl);
       if constexpr (E == 16) spmm_launch<XT, 9, 1, VAL>(ctx, s, epi, &nl);
     } else if (E == 16 && C == 1) {

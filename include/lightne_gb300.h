@@ -303,7 +303,8 @@ typedef struct lne_propagate_stats {
  * with X = M^2/2 - I, M = I - D~^-1 (A + I) - mu I, c_k the Bessel weights.
  * d_a (input) and d_y (output): device n x dim FP32, row-major; y must not
  * alias a.  d_a_out (optional, may be NULL) receives a - conv, the value the
- * reference leaves in its mutated argument.  Replaces
+ * reference leaves in its mutated argument; it may be a, or overlap it.
+ * Replaces
  * spectral_propagation::chebyshev_expansion up to the (A+I)a product
  * (LightNE/SpectralPropagation.h:45-221).
  */
@@ -324,6 +325,7 @@ int lne_chebyshev_coefficients(int32_t order, double s, float* out);
  * h = (A + I) g; dL/ds = -sum_k c_k'(s) <h, T_k a>; dL/dmu from the forward
  * tangent T'_1 = -M a, T'_{k+1} = 2 X T'_k - T'_{k-1} - 2 M T_k.
  * The derivatives are of the real-valued map (mu, s not rounded to float).
+ * d_ga may be a or g, or overlap them.
  */
 int lne_propagate_adjoint(lne_ctx* ctx, const lne_graph* g, const lne_propagate_params* p, const float* d_a,
                           const float* d_gy, float* d_ga, double* h_dmu, double* h_ds, lne_propagate_stats* stats);

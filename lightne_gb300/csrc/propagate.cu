@@ -745,10 +745,12 @@ int propagate_impl(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, co
   }
   const float* A = direct ? d_a : Acopy;
   const float a_scale = direct ? sc : 1.0f;
-  // a - conv: to the caller's buffer where it can be written in place (the
-  // (A + I) product gathers it in the FP32 form, so it must not be y)
-  const bool out_direct =
-      d_a_out && rows_direct(d_a_out, d, ld) && !ranges_overlap(d_a_out, d_y, sizeof(float) * (size_t)n * d);
+  // a - conv: to the caller's buffer where it can be written in place.  The
+  // (A + I) product gathers it in the FP32 form, so it must not be y; and rows
+  // are written while other rows of a are still read, so it must not be a.
+  const size_t bytes = sizeof(float) * (size_t)n * d;
+  const bool out_direct = d_a_out && rows_direct(d_a_out, d, ld) && !ranges_overlap(d_a_out, d_y, bytes) &&
+                          !ranges_overlap(d_a_out, d_a, bytes);
   float* Af = nullptr;
   if (!out_direct && (!k16 || d_a_out) && (rc = B.get(&Af, sz, "a - conv"))) return rc;
   FinalOut<HT> fin;

@@ -411,8 +411,8 @@ struct EpiAPlusI {
   }
 };
 
-// Adjoint start: h = (A + I) g, g = g_scale times the operand (a power of
-// two);  b = h / d~_i (FP32, may be null, and 16-bit copy).
+// Adjoint start: h = (A + I) g;  b = h / d~_i (FP32, may be null, and 16-bit
+// copy).
 template <typename XT>
 struct EpiAdjInit {
   using HT = typename ShadowOf<XT>::type;
@@ -422,7 +422,6 @@ struct EpiAdjInit {
   float* __restrict__ H;
   float* __restrict__ Bf;
   HT* __restrict__ Bb;
-  float g_scale;
   template <int N>
   struct Pre {
     float inv_dt;
@@ -440,7 +439,7 @@ struct EpiAdjInit {
     float h[N], b[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      h[i] = g_scale * (q.g.at(i) + acc[i]);
+      h[i] = q.g.at(i) + acc[i];
       b[i] = h[i] * q.inv_dt;
     }
     store_f32<N>(H, ld, r, e0, h);
@@ -913,8 +912,9 @@ int adjoint_impl(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, cons
   // in g; the FP32 parameter-gradient pass unscales its dots by 1 / sg)
   float sg = 1.0f;
   if ((rc = input_scale<XT>(ctx, d_gy, n * d, B, &launches, &sg))) return rc;
-  // g is read in place where its rows are whole 16-byte vectors
-  const bool g_direct = rows_direct(d_gy, d, ld);
+  // g is read in place where its rows are whole 16-byte vectors; the FP32
+  // pass of the FP16 form takes a scaled copy (sums of g itself may overflow)
+  const bool g_direct = rows_direct(d_gy, d, ld) && !(params && sg != 1.0f);
   float *Gcopy = nullptr, *H = nullptr, *Bf = nullptr;
   HT *Gb = nullptr, *Bb = nullptr;
   if ((!g_direct && (!k16 || params) && (rc = B.get(&Gcopy, sz, "g"))) || (rc = B.get(&H, sz, "h")) ||
@@ -934,7 +934,7 @@ int adjoint_impl(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, cons
   // h = (A + I) g, b = D~^-1 h
   {
     const XT* Gx = F.op(G, Gb);
-    EpiAdjInit<XT> epi{F.coef, Gx, ld, H, Bf, Bb, 1.0f};
+    EpiAdjInit<XT> epi{F.coef, Gx, ld, H, Bf, Bb};
     if ((rc = F.spmm(Gx, epi))) return rc;
   }
   if (params) {
@@ -948,7 +948,7 @@ int adjoint_impl(lne_ctx* ctx, lne_graph* g, const lne_propagate_params* p, cons
     if (k16) {
       float* H2 = nullptr;
       if ((rc = B.get(&H2, sz, "h fp32"))) return rc;
-      if ((rc = F32.spmm(G, EpiAdjInit<float>{F.coef, G, ld, H2, nullptr, nullptr, g_direct ? sg : 1.0f}))) return rc;
+      if ((rc = F32.spmm(G, EpiAdjInit<float>{F.coef, G, ld, H2, nullptr, nullptr}))) return rc;
       H32 = H2;
     }
     if ((rc = param_grads(ctx, F32, p, c, H32, d_a, 1.0 / (double)sg, h_dmu, h_ds))) return rc;

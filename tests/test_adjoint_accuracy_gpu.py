@@ -56,3 +56,19 @@ def test_parameter_gradients_with_a_hub(ctx, precision, n, hub, dim):
     print("relative errors of dL/dmu, dL/ds:", rms)
     assert (rms <= 5e-7).all(), rms
     g.free()
+
+
+@pytest.mark.parametrize("dim", [5, 8])
+def test_parameter_gradients_of_a_large_gradient(ctx, dim):
+    """An output gradient whose sum over a hub's neighbours is above FP32's
+    range: the FP16 form's scale keeps the parameter gradients finite.  Bound:
+    FP32 rounding through 20 products and 20 sums of one sign, 1e-5 of |h a|."""
+    off, nbrs = hub_graph(2000, [1900], 3)
+    g = Graph.from_numpy(ctx, off, nbrs)
+    rng = np.random.default_rng(dim)
+    a = (1e-3 * rng.standard_normal((2000, dim))).astype(np.float32)
+    gy = (1e37 * rng.uniform(0.5, 1.0, (2000, dim))).astype(np.float32)
+    mu_ref, s_ref, scale = reference(off, nbrs, a, gy, 6)
+    _, dmu, ds = propagate_adjoint(ctx, g, a, gy, dim, order=6, mu=MU, s=S, precision="fp16")
+    assert abs(dmu - mu_ref) <= 1e-5 * scale and abs(ds - s_ref) <= 1e-5 * scale, (dmu, mu_ref, ds, s_ref)
+    g.free()

@@ -1003,7 +1003,8 @@ __global__ void __launch_bounds__(256) k_jacobi_sweeps_dsmem(int r, double* __re
 // the end of a sweep.  Same pairs, same order and the same operations as
 // k_jacobi_sweeps: the columns are bit for bit the same, signs included (the
 // path is sensitive: tangents good to one unit in the last place changed
-// signs).  At r = 256, 13 sweeps: 28 ms by the cluster form, 25 with a warp
+// signs), but where the product of two squared norms leaves FP64's range,
+// which only that form mistakes for a limit.  At r = 256, 13 sweeps: 28 ms by the cluster form, 25 with a warp
 // per pair, 18.5 so.
 //
 // Launched cooperatively (the CTAs wait on one another).  Every wait gives up
@@ -1024,7 +1025,7 @@ __global__ void __launch_bounds__(128) k_jacobi_sweeps_flow(int r, double* __res
                                                             int* __restrict__ version, int* __restrict__ arrived,
                                                             int* __restrict__ abort, int max_sweeps,
                                                             int* __restrict__ sweeps_out) {
-  __shared__ double sum[3], root[2], rotn[2];
+  __shared__ double sum[3], limit, rotn[2];
   __shared__ int state;  // of the step: 0 no rotation, 1 rotation, 2 given up; at a sweep's end: 2 go on
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pk = blockIdx.x;
   const int rp = (r + 1) & ~1;  // even number of players (index r is a dummy when r is odd)
@@ -1092,11 +1093,16 @@ __global__ void __launch_bounds__(128) k_jacobi_sweeps_flow(int r, double* __res
           if (lane == 0) sum[warp] = d;
         }
         __syncthreads();
-        // the limit's roots (warps 0 and 1) beside the rotation (warp 2)
+        // the limit (warp 0) beside the rotation (warp 2)
         double c = 1.0, sn = 0.0, g = 0.0;
-        if (warp < 2) {
-          const double rt = sqrt(d);
-          if (lane == 0) root[warp] = rt;
+        if (warp == 0) {
+          const double a = sum[0], b = sum[1], ab = a * b;
+          double root = sqrt(ab);
+          if (!(ab >= 0x1p-1022 && ab < INFINITY)) {  // out of range: the same root, scaled
+            const double f = ab < 1.0 ? 0x1p512 : 0x1p-512;
+            root = sqrt((a * f) * (b * f)) * (1.0 / f);
+          }
+          if (lane == 0) limit = tol * root;
         } else if (warp == 2) {
           const double a = sum[0], b = sum[1];
           g = d;
@@ -1111,7 +1117,7 @@ __global__ void __launch_bounds__(128) k_jacobi_sweeps_flow(int r, double* __res
         }
         __syncthreads();
         g = sum[2];
-        const bool rot = fabs(g) > tol * root[0] * root[1] && g != 0.0;
+        const bool rot = fabs(g) > limit && g != 0.0;
         any = any || rot;
         if (rot) {
           c = rotn[0];

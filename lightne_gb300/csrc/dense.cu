@@ -1412,7 +1412,9 @@ __global__ void k_jacobi_norms(int r, const double* __restrict__ Wc, double* __r
 }
 
 // Block j writes column j, normalised, at its place in descending order (ties
-// by index).
+// by index).  The norms are compared as their bits without the sign, which
+// order them as the numbers do and put a NaN first, so that every column has a
+// place of its own whatever the input holds.
 __global__ void k_jacobi_finish(int r, const double* __restrict__ Wc, const double* __restrict__ norms,
                                 double* __restrict__ U, double* __restrict__ S) {
   __shared__ int place;
@@ -1420,8 +1422,10 @@ __global__ void k_jacobi_finish(int r, const double* __restrict__ Wc, const doub
   if (threadIdx.x == 0) place = 0;
   __syncthreads();
   const double nrm = norms[j];
+  auto bits = [&](int k) { return __double_as_longlong(norms[k]) & 0x7fffffffffffffffLL; };
+  const long long mine = bits(j);
   int before = 0;
-  for (int k = threadIdx.x; k < r; k += blockDim.x) before += (norms[k] > nrm) || (norms[k] == nrm && k < j);
+  for (int k = threadIdx.x; k < r; k += blockDim.x) before += bits(k) > mine || (bits(k) == mine && k < j);
   before = __reduce_add_sync(0xffffffffu, before);
   if ((threadIdx.x & 31) == 0) atomicAdd(&place, before);
   __syncthreads();

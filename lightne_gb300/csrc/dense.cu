@@ -1005,7 +1005,7 @@ __global__ void __launch_bounds__(256) k_jacobi_sweeps_dsmem(int r, double* __re
 // path is sensitive: tangents good to one unit in the last place changed
 // signs), but where the product of two squared norms leaves FP64's range,
 // which only that form mistakes for a limit.  At r = 256, 13 sweeps: 28 ms by the cluster form, 25 with a warp
-// per pair, 18.5 so.
+// per pair, 18 so.
 //
 // Launched cooperatively (the CTAs wait on one another).  Every wait gives up
 // after kFlowSpins polls, raises *abort and lets the others leave too.

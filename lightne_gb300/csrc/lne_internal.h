@@ -35,9 +35,9 @@ struct __align__(16) Vertex {
 // Work list of one sparse operator for the row-parallel SpMM (built once,
 // cached on the matrix or graph).  A row with at most kChunkNnz entries is
 // one item, a longer row is cut into items of kChunkNnz entries (chunks).
-// Items come longest first: [0, n_big) the rows above max(kBigNnz, warp_max)
-// and every chunk, [n_big, n_heavy) the rows above warp_max, then the rest
-// (at most warp_max entries).
+// Items come in three classes, each in row order: [0, n_big) the rows above
+// max(kBigNnz, warp_max) and every chunk, [n_big, n_heavy) the rows above
+// warp_max, then the rest (at most warp_max entries).
 static constexpr int kChunkNnz = 2048;
 static constexpr int kBigNnz = 512;
 static constexpr int kWarpNnzMin = 64;

@@ -137,8 +137,9 @@ struct HeavyTune {
   static constexpr int LG = 32 / W;                  // rows side by side in a warp
   static constexpr int kParts = G * 4 / W;           // warps side by side on one row
   // warps on strands of their own: an item of a graph, whose products wait
-  // for their longest rows, has the block (see k_spmm_heavy); the rows of a
-  // matrix are enough to fill the device without
+  // for their longest rows, has the block, an item of a matrix kParts warps
+  // (one of either measured, see k_spmm_heavy; the number of heavy items was
+  // not tried as the rule)
   static constexpr int NS = VAL ? 1 : kHeavyWarps / kParts;
   static constexpr int A = P / (LG * NS);            // strands per lane
   static constexpr int kWarps = kParts * NS;         // warps of one item
@@ -187,7 +188,8 @@ struct Word32<__nv_fp8_e4m3> {
 
 // kWarps warps per heavy item: warp (part, ws) has the words 32 part .. of
 // the rows, its lane group lg the strands lg + LG ws, and A - 1 more.  The
-// hardware hands out the blocks in order, so the longest items start first.
+// hardware hands out the blocks in order, so the longest class of items starts
+// first.
 // Spreading the strands of rows narrower than 512 bytes over a block's warps
 // took 19 products of a 2,001-vertex graph at 33 columns from 513 to 348 us;
 // on a matrix (12K rows of 250, 42 columns) it made a randomized SVD of

@@ -82,6 +82,7 @@ static inline int64_t spmm_work_width(int64_t d) {
   const int64_t vecs = (d + E - 1) / E;
   return (vecs < 128 ? vecs : 128) * E;
 }
+
 // Copies columns [v0, v0 + C) (16-byte vectors) of the x_rows rows of X
 // into a dense x_rows x C array.
 static __global__ void k_slab_copy(const uint4* __restrict__ X, int64_t ldv, int64_t v0, int64_t x_rows, int C,
@@ -114,9 +115,14 @@ static int spmm_run(lne_ctx* ctx, const SpmmPlan& plan, const uint32_t* col, con
   int nl = 0;
   // graphs, and matrices so small that a warp walking a 2048-entry row (some
   // 250 us) would outlast the rest: below 4 GB of gathers (about 0.4 ms).
-  // Above, the 16-byte gathers of a warp per row take fewer instructions: a
-  // 10,312-row matrix with 33M entries and 256 FP32 columns, 34 GB, takes
-  // 1.4 ms that way and 2.3 ms balanced.
+  // Above, the 16-byte gathers of a warp per row take fewer instructions.
+  // The line follows the size alone, while what decides is also how long the
+  // rows are.  Measured both ways on power-law matrices, us balanced / a warp
+  // per row: 200,000 rows of 20, FP32, 32 columns (0.5 GB) 94 / 83, 128 (2 GB)
+  // 189 / 356, 256 (4.1 GB) 380 / 734; 10,312 rows of 340, 64 columns (0.9 GB)
+  // 83 / 100, 256 (3.6 GB) 301 / 314; 60,000 rows of 280, 32 columns (2.2 GB)
+  // 167 / 163, 64 (4.4 GB) 298 / 260, 256 (17 GB) 1071 / 831; 10,312 rows of
+  // 1,100, 64 columns (2.8 GB) 237 / 167, 256 (11 GB) 930 / 503.
   const bool bal = !VAL || (plan.warp_max < kChunkNnz && (double)plan.nnz * d * sizeof(XT) < 4e9);
   SpmmWork own;
   if (!work) {
